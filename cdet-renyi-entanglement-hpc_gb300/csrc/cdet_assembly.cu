@@ -1,0 +1,423 @@
+// FP64 Green-matrix assembly for sm_103a: decode, lookup descriptor and the
+// reference's Clenshaw recurrences (g_funcs.h:395-463, 609-763), bit for bit.
+//
+// A lookup is one 2-D Chebyshev sum: nu independent row sums over v, then one
+// sum of the row values over u. One block of four warps takes up to
+// kMaxLookups lookups of one configuration. Its row sums (lookups x rows) are
+// dealt to lanes in runs of 32, so a single configuration already fills a
+// block with independent chains and no lane idles on an invalid entry of a
+// mixed-order batch; the row values go to shared memory, and one lane per
+// lookup runs the outer sum over them.
+//
+// Row sums: each lane walks one row of nv coefficients downwards. The 32 rows
+// of a warp are copied 16 columns at a time with cp.async (two buffers per
+// warp, the next chunk in flight while one is consumed), so the global reads
+// are whole 128-byte pieces of rows; read straight from global memory each
+// lane's 8-byte loads were 32 separate L1 wavefronts per step, about what the
+// FP64 work of the step takes.
+//
+// Arithmetic: a step b_k = c_k + 2x b_{k+1} - b_{k+2} is a product and two
+// additions, each rounded. The FP64 pipe bounds the kernel (two lane
+// operations per clock and SM), so the product is formed on the integer pipes
+// (cdet_softmul.cuh) and only the additions go to the FP64 pipe. A chunk in
+// which some lane's product may not be the common case is repeated from its
+// first step with the product on the FP64 pipe.
+//
+// Measured against one thread per lookup (product on the FP64 pipe, 8-byte
+// loads), whole calls: 8x8 / degree 128 / order 10, 4,096 configurations
+// 106.5 -> 56.6 ms (two FP64 additions per coefficient at the pipe's 527 G/s:
+// 51 ms); 6x6 / degree 96, 4,096 mixed orders 1..10 26.6 -> 5.2 ms (no lanes
+// on entries past a configuration's order); one order-6 configuration 2.08 ->
+// 0.14 ms (all rows at once); 128 chains of envelope 9, a step with reused
+// pairs 3.35 -> 0.86 ms (copies and evaluations in one launch).
+#include "cdet_device.cuh"
+#include "cdet_kernels.cuh"
+#include "cdet_softmul.cuh"
+
+#include <algorithm>
+
+namespace cdet {
+
+namespace {
+
+// sampled_coordinate_to_index (g_funcs.h:315-342) on value*extent; flags
+// values the reference would reject (non-finite, outside the int range).
+__device__ __forceinline__ int coordinate_index(double scaled, int extent, bool& bad) {
+    if (!(scaled > -2147483648.0 && scaled < 2147483648.0)) {
+        bad = true;
+        return 0;
+    }
+    int index = static_cast<int>(floor(scaled));
+    if (index < 0) index = 0;
+    if (index >= extent) index = extent - 1;
+    return index;
+}
+
+struct Vertex {
+    double tau, tau_unit;
+    int x, y, replica;
+};
+
+// Vertex decode of integrand_temp_typed (integrand_replica_randomly_sampled.h:422-432).
+__device__ __forceinline__ Vertex decode_vertex(const double* __restrict__ v, const Scalars& s,
+                                                int replica_count, bool& bad) {
+    Vertex out;
+    const double tu = __ldg(v + 0);
+    if (!isfinite(tu)) bad = true;
+    out.tau_unit = tu;
+    out.tau = dmul(s.beta, tu);
+    out.x = coordinate_index(dmul(static_cast<double>(s.n1), __ldg(v + 1)), s.n1, bad);
+    out.y = coordinate_index(dmul(static_cast<double>(s.n2), __ldg(v + 2)), s.n2, bad);
+    out.replica = replica_count <= 1
+                      ? 0
+                      : coordinate_index(dmul(static_cast<double>(replica_count), __ldg(v + 3)),
+                                         replica_count, bad);
+    return out;
+}
+
+__device__ __forceinline__ double clamp_unit(double value) {
+    if (value < -1.0) return -1.0;
+    if (value > 1.0) return 1.0;
+    return value;
+}
+
+constexpr int kThreads = 128;
+constexpr int kWarps = kThreads / kWarp;
+constexpr int kMaxLookups = 16;  // lookups of one block: the outer sums run on that many lanes of one warp
+constexpr int kRowBlock = 128;   // row values kept per lookup; more rows are taken block by block
+constexpr int kChunk = 16;       // columns of a staged chunk
+constexpr int kStride = 18;      // doubles between the rows of a staged chunk: 16-byte aligned, 16-byte reads free of bank conflicts
+
+// One lookup of the block.
+struct Lookup {
+    const double* coeffs;  // its block of nu x nv coefficients
+    double u, v;
+    int set, i, j;
+    int spin;    // the spin evaluated
+    int active;  // 0: nothing to evaluate (value already written, or a rejected vertex)
+};
+
+struct Shared {
+    double stage[kWarps][2][kWarp * kStride];
+    const double* row[kWarps][2][kWarp];  // the rows of the run being staged
+    Lookup lookup[kMaxLookups];
+};
+
+// fill_pair_range (integrand_replica_randomly_sampled.h:467-473) for one
+// evaluated entry: both spins when they share the evaluation.
+__device__ __forceinline__ void store_entry(const Problem& p, const Scratch& w, int64_t c, int n, int set, int i, int j,
+                                            int spin, bool both, double value) {
+    const int nmax = p.max_order;
+    const int64_t per_set = static_cast<int64_t>(nmax) * nmax;
+    const int64_t mslot = (c * 2 + set) * 2;
+    for (int sp = both ? 0 : spin; sp <= (both ? 1 : spin); ++sp) {
+        double g = value;
+        if (i == j) {
+            g = dadd(g, sp == 0 ? p.s.diag_up_shift : p.s.diag_down_shift);
+            // the double-double order-1 branch adds its own shifts to the unshifted value
+            w.diag[(mslot + sp) * nmax + i] = p.raw_diag ? value : g;
+        }
+        w.green[(mslot + sp) * per_set + i * n + j] = dmul(g, p.s.scale);
+    }
+}
+
+// The Clenshaw steps of one full staged chunk (16 columns in decreasing
+// order). kFirst: its top column starts the recurrence; kLast: its lowest
+// column ends it. kSoft: products on the integer pipes, `bad` set where one
+// of them may differ from the FP64 pipe's.
+template <bool kSoft, bool kFirst, bool kLast>
+__device__ __forceinline__ void chunk_steps(const double* st, double two_x, const SoftFactor& fx, double x, double& b1,
+                                            double& b2, bool& bad) {
+#pragma unroll
+    for (int q = kChunk / 2 - 1; q >= 0; --q) {
+        const double2 pair = *reinterpret_cast<const double2*>(st + 2 * q);
+#pragma unroll
+        for (int h = 1; h >= 0; --h) {
+            const double c = h ? pair.y : pair.x;
+            if (kFirst && q == kChunk / 2 - 1 && h == 1) {
+                // c + 2x 0 - 0
+                b1 = dsub(dadd(c, dmul(two_x, 0.0)), 0.0);
+                b2 = 0.0;
+            } else if (kLast && q == 0 && h == 0) {
+                b1 = dsub(dadd(c, dmul(b1, x)), b2);
+            } else {
+                const double t = kSoft ? soft_mul(fx, b1, bad) : dmul(two_x, b1);
+                const double bk = dsub(dadd(c, t), b2);
+                b2 = b1;
+                b1 = bk;
+            }
+        }
+    }
+}
+
+// The same for a chunk of `count` < 16 columns (the top of a row).
+__device__ __forceinline__ void partial_chunk_steps(const double* st, int count, bool last, double two_x, double x,
+                                                    double& b1, double& b2) {
+    b1 = dsub(dadd(st[count - 1], dmul(two_x, 0.0)), 0.0);
+    b2 = 0.0;
+    const int end = last ? 1 : 0;
+    for (int k = count - 2; k >= end; --k) {
+        const double bk = dsub(dadd(st[k], dmul(two_x, b1)), b2);
+        b2 = b1;
+        b1 = bk;
+    }
+    if (last) b1 = dsub(dadd(st[0], dmul(b1, x)), b2);
+}
+
+template <bool kVec16>
+__device__ __forceinline__ void stage_chunk(double* st, const double* const* row, int column, int count, int lane) {
+    const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(st));
+    if constexpr (kVec16) {  // eight lanes of 16 bytes per row
+        const int part = lane & 7;
+        if (2 * part < count) {
+#pragma unroll
+            for (int it = 0; it < kWarp / 4; ++it) {
+                const int r = it * 4 + (lane >> 3);
+                const double* src = row[r] + column + 2 * part;
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst + (r * kStride + 2 * part) * 8),
+                             "l"(src));
+            }
+        }
+    } else {  // sixteen lanes of 8 bytes per row
+        const int part = lane & 15;
+        if (part < count) {
+#pragma unroll
+            for (int it = 0; it < kWarp / 2; ++it) {
+                const int r = it * 2 + (lane >> 4);
+                const double* src = row[r] + column + part;
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + (r * kStride + part) * 8),
+                             "l"(src));
+            }
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// One block: lookups [first, first + count) of configuration blockIdx.x,
+// first = blockIdx.y * lookups_per_block. The lookups of a configuration of
+// order n, set by set and spin by spin: its n^2 entries, or, with Green-pair
+// reuse, the entries of pairs not both retained (rows i < k at columns
+// k..n-1, then rows i >= k at every column), where the blocks with
+// blockIdx.y == 0 also copy the retained ones.
+template <bool kVec16>
+__global__ void __launch_bounds__(kThreads, 4) green_assembly_fp64(const __grid_constant__ Problem p,
+                                                                  const __grid_constant__ Scratch w,
+                                                                  int lookups_per_block, int row_block) {
+    extern __shared__ __align__(16) unsigned char assembly_smem[];
+    Shared& sm = *reinterpret_cast<Shared*>(assembly_smem);
+    double* values = reinterpret_cast<double*>(assembly_smem + sizeof(Shared));  // [lookup][row_block | 1]
+    const int value_stride = row_block | 1;
+    const Scalars& s = p.s;
+    const int nmax = p.max_order;
+    const int64_t c = blockIdx.x;
+    const int tid = threadIdx.x, lane = tid & (kWarp - 1), warp = tid / kWarp;
+    const int n = p.all_subsets ? nmax : __ldg(p.orders + c);
+    if (n < 1 || n > nmax) {
+        if (blockIdx.y == 0 && tid == 0) atomicOr(p.status + c, kStatusBadInput);
+        return;
+    }
+    const double* vbase = p.vertices + c * static_cast<int64_t>(nmax) * 4;
+    const int kept = p.reuse_mask ? __popcll(__ldg(p.reuse_mask + c)) : 0;
+    const int per = n * n - kept * kept;  // evaluated entries of one set and spin
+    const int spins0 = p.same_spin[0] ? 1 : 2, spins1 = p.same_spin[1] ? 1 : 2;
+    const int total = per * (spins0 + spins1);
+
+    if (kept > 0 && blockIdx.y == 0) {
+        for (int e = tid; e < 2 * kept * kept; e += kThreads) {
+            const int set = e >= kept * kept ? 1 : 0;
+            const int r = e - set * kept * kept;
+            const int i = r / kept, j = r - (r / kept) * kept;
+            bool bad = false;  // the decode's checks, so the status bits are a fresh evaluation's
+            decode_vertex(vbase + 4 * i, s, set == 0 ? 2 : 1, bad);
+            decode_vertex(vbase + 4 * j, s, set == 0 ? 2 : 1, bad);
+            if (bad) atomicOr(p.status + c, kStatusBadInput);
+            else copy_reused_pair(p, w.green, w.diag, c, set, i, j, n);
+        }
+    }
+
+    const int first = blockIdx.y * lookups_per_block;
+    if (first >= total) return;
+    const int count = min(lookups_per_block, total - first);
+    if (tid < count) {
+        int e = first + tid;
+        const int set = e >= per * spins0 ? 1 : 0;
+        e -= set * per * spins0;
+        const int spin = e >= per ? 1 : 0;
+        e -= spin * per;
+        int i, j;
+        if (e < kept * (n - kept)) {
+            i = e / (n - kept);
+            j = kept + (e - i * (n - kept));
+        } else {
+            const int q = e - kept * (n - kept);
+            i = kept + q / n;
+            j = q - (q / n) * n;
+        }
+        Lookup l;
+        l.set = set;
+        l.spin = spin;
+        l.i = i;
+        l.j = j;
+        l.u = l.v = 1.0;  // a lookup with nothing to evaluate walks its rows harmlessly
+        l.active = 0;
+        bool bad = false;
+        const int replica_count = set == 0 ? 2 : 1;
+        const Vertex vi = decode_vertex(vbase + 4 * i, s, replica_count, bad);
+        const Vertex vj = decode_vertex(vbase + 4 * j, s, replica_count, bad);
+        // prepare_green_lookup_descriptor (g_funcs.h:609-653).
+        const bool upper = (i != j) && (vi.tau_unit > vj.tau_unit);
+        const uint64_t sitepair =
+            ((((static_cast<uint64_t>(vi.replica) * 2u + static_cast<uint64_t>(vj.replica)) * s.n1 + vi.x) * s.n2 +
+              vi.y) * s.n1 + vj.x) * s.n2 + vj.y;
+        const TableDev& t = spin == 0 ? p.up[set] : p.down[set];
+        l.coeffs = (upper ? t.upper : t.lower) + sitepair * static_cast<uint64_t>(s.nu) * static_cast<uint64_t>(s.nv);
+        const double t_outer = upper ? vi.tau : vj.tau;  // the later time of the pair
+        const double t_inner = upper ? vj.tau : vi.tau;
+        if (bad) {
+            atomicOr(p.status + c, kStatusBadInput);
+        } else if (t_outer < s.branch_eps) {
+            store_entry(p, w, c, n, set, i, j, spin, p.same_spin[set] != 0,
+                        __ldg((upper ? t.upper_corners : t.lower_corners) + sitepair));
+        } else {
+            l.u = clamp_unit(dsub(ddiv(dmul(2.0, t_outer), s.beta), 1.0));
+            l.v = clamp_unit(dsub(ddiv(dmul(2.0, t_inner), t_outer), 1.0));
+            l.active = 1;
+        }
+        sm.lookup[tid] = l;
+    }
+    __syncthreads();
+
+    const int nu = s.nu, nv = s.nv;
+    const int chunks = (nv + kChunk - 1) / kChunk;
+    const int top_count = nv - (chunks - 1) * kChunk;  // columns of a row's first (highest) chunk
+    // the outer sum of lookup tid, fed row values in decreasing order
+    OuterClenshaw outer;
+    if (tid < count) outer.init(nu - 1, sm.lookup[tid].u);
+
+    for (int hi = nu; hi > 0; hi -= row_block) {
+        const int rows = min(row_block, hi);
+        const int base_row = hi - rows;
+        const int tasks = count * rows;  // task = lookup * rows + (row - base_row)
+        const int runs = (tasks + kWarp - 1) / kWarp;
+        if (nv < 3) {
+            for (int task = tid; task < tasks; task += kThreads) {
+                const int l = task / rows, r = task - l * rows;
+                values[l * value_stride + r] = clenshaw_row(
+                    sm.lookup[l].coeffs + static_cast<int64_t>(base_row + r) * nv, nv - 1, sm.lookup[l].v);
+            }
+        } else {
+            // this warp's runs warp, warp + 4, ...: a flat sequence of (run, chunk) with one chunk staged ahead
+            const int my_runs = runs > warp ? (runs - warp + kWarps - 1) / kWarps : 0;
+            auto point_rows = [&](int m) {  // the m-th run's rows; lanes past the end repeat the last task
+                const int task = min((warp + m * kWarps) * kWarp + lane, tasks - 1);
+                const int l = task / rows, r = task - l * rows;
+                sm.row[warp][m & 1][lane] = sm.lookup[l].coeffs + static_cast<int64_t>(base_row + r) * nv;
+                __syncwarp();
+            };
+            auto stage = [&](int m, int j, int slot) {  // chunk j of run m: columns from the top
+                const int column = (chunks - 1 - j) * kChunk;
+                stage_chunk<kVec16>(sm.stage[warp][slot], sm.row[warp][m & 1], column, j == 0 ? top_count : kChunk,
+                                    lane);
+            };
+            if (my_runs > 0) {
+                point_rows(0);
+                stage(0, 0, 0);
+            }
+            int slot = 0;
+            for (int m = 0; m < my_runs; ++m) {
+                const int task = (warp + m * kWarps) * kWarp + lane;
+                const int task_c = min(task, tasks - 1);
+                const int l = task_c / rows, r = task_c - l * rows;
+                const double x = sm.lookup[l].v;
+                const double two_x = dmul(2.0, x);
+                const SoftFactor fx = soft_factor(static_cast<uint32_t>(__double2hiint(two_x)),
+                                                  static_cast<uint32_t>(__double2loint(two_x)));
+                // all-integer products while every lane's factor allows them and no chunk of this run failed
+                bool soft = __all_sync(0xffffffffu,
+                                       soft_factor_in_range(static_cast<uint32_t>(__double2hiint(two_x))));
+                double b1 = 0.0, b2 = 0.0;
+                for (int j = 0; j < chunks; ++j) {
+                    // stage the next chunk, then wait for this one
+                    if (j + 1 < chunks) {
+                        stage(m, j + 1, slot ^ 1);
+                    } else if (m + 1 < my_runs) {
+                        point_rows(m + 1);
+                        stage(m + 1, 0, slot ^ 1);
+                    } else {
+                        asm volatile("cp.async.commit_group;" ::: "memory");
+                    }
+                    asm volatile("cp.async.wait_group 1;" ::: "memory");
+                    __syncwarp();
+                    const double* st = sm.stage[warp][slot] + lane * kStride;
+                    const bool last = j == chunks - 1;
+                    if (j == 0 && top_count < kChunk) {
+                        partial_chunk_steps(st, top_count, last, two_x, x, b1, b2);
+                    } else {
+                        const double b1_in = b1, b2_in = b2;
+                        bool redo = !soft;
+                        if (soft) {
+                            bool bad = false;
+                            if (j == 0 && last) chunk_steps<true, true, true>(st, two_x, fx, x, b1, b2, bad);
+                            else if (j == 0) chunk_steps<true, true, false>(st, two_x, fx, x, b1, b2, bad);
+                            else if (last) chunk_steps<true, false, true>(st, two_x, fx, x, b1, b2, bad);
+                            else chunk_steps<true, false, false>(st, two_x, fx, x, b1, b2, bad);
+                            redo = __any_sync(0xffffffffu, bad);
+                        }
+                        if (redo) {
+                            soft = false;
+                            bool unused = false;
+                            b1 = b1_in;
+                            b2 = b2_in;
+                            if (j == 0 && last) chunk_steps<false, true, true>(st, two_x, fx, x, b1, b2, unused);
+                            else if (j == 0) chunk_steps<false, true, false>(st, two_x, fx, x, b1, b2, unused);
+                            else if (last) chunk_steps<false, false, true>(st, two_x, fx, x, b1, b2, unused);
+                            else chunk_steps<false, false, false>(st, two_x, fx, x, b1, b2, unused);
+                        }
+                    }
+                    __syncwarp();  // the buffer is free for the chunk after next
+                    slot ^= 1;
+                }
+                if (task < tasks) values[l * value_stride + r] = b1;
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+        }
+        __syncthreads();
+        if (tid < count)
+            for (int r = rows - 1; r >= 0; --r) outer.push(base_row + r, values[tid * value_stride + r]);
+        __syncthreads();
+    }
+    if (tid < count && sm.lookup[tid].active)
+        store_entry(p, w, c, n, sm.lookup[tid].set, sm.lookup[tid].i, sm.lookup[tid].j, sm.lookup[tid].spin,
+                    p.same_spin[sm.lookup[tid].set] != 0, outer.result());
+}
+
+}  // namespace
+
+cudaError_t launch_fp64_assembly(const Problem& p, const Scratch& w, int sm_count, cudaStream_t stream) {
+    if (p.batch <= 0) return cudaSuccess;
+    const int spins = (p.same_spin[0] ? 1 : 2) + (p.same_spin[1] ? 1 : 2);
+    const int64_t per_config = static_cast<int64_t>(spins) * p.max_order * p.max_order;
+    // lookups per block: 16 once the batch gives every SM its four blocks several times over (the outer
+    // sum's one busy warp per block is then 1/512th of its work at degree 128), fewer for small batches,
+    // down to one lookup per block, so that they spread over all SMs
+    const int64_t blocks_wanted = 16 * static_cast<int64_t>(sm_count > 0 ? sm_count : 152);
+    const int lookups = static_cast<int>(
+        std::max<int64_t>(1, std::min<int64_t>(kMaxLookups, p.batch * per_config / blocks_wanted)));
+    const int row_block = std::min(p.s.nu, kRowBlock);
+    const size_t smem = sizeof(Shared) + static_cast<size_t>(lookups) * (row_block | 1) * sizeof(double);
+    // 16-byte copies need 16-byte aligned rows
+    bool vec16 = p.s.nv % 2 == 0;
+    for (int set = 0; set < 2; ++set)
+        for (const TableDev* t : {&p.up[set], &p.down[set]})
+            for (const double* c : {t->upper, t->lower})
+                if (reinterpret_cast<uintptr_t>(c) % 16 != 0) vec16 = false;
+    auto kernel = vec16 ? green_assembly_fp64<true> : green_assembly_fp64<false>;
+    const cudaError_t err =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (err != cudaSuccess) return err;
+    const dim3 grid(static_cast<unsigned>(p.batch), static_cast<unsigned>((per_config + lookups - 1) / lookups));
+    kernel<<<grid, kThreads, smem, stream>>>(p, w, lookups, row_block);
+    return cudaGetLastError();
+}
+
+}  // namespace cdet

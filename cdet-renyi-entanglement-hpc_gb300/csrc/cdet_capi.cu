@@ -584,7 +584,7 @@ int run(cdet_context* ctx, const double* vertices, const int32_t* orders, int64_
         if (plan.nrb * plan.nkc > 1) ++launches;  // the sub-block combine
     } else if (!assembly_only) {
         if (tune_post) {
-            err = cdet::launch_fp64_assembly_only(p, w, stream);
+            err = cdet::launch_fp64_assembly(p, w, ctx->sm_count, stream);
             if (err != cudaSuccess) return cuda_fail(err, "kernel launch");
             rc = settle_post_form();
             if (rc != CDET_OK) return rc;
@@ -595,10 +595,9 @@ int run(cdet_context* ctx, const double* vertices, const int32_t* orders, int64_
         if (err != cudaSuccess) return cuda_fail(err, "kernel launch");
         // assembly + minors, CDet (or the queue kernel, or the double-double kernel)
         launches = (cdet::uses_queue_form(p) || p.dd_mode) ? 2 : 3;
-        if (p.reuse_mask && p.all_subsets) launches += 2;  // the reuse scan and the copies
     } else {
         launches = 1;
-        err = cdet::launch_fp64_assembly_only(p, w, stream);
+        err = cdet::launch_fp64_assembly(p, w, ctx->sm_count, stream);
         if (err != cudaSuccess) return cuda_fail(err, "kernel launch");
     }
     if (!assembly_only && cdet::sorts_orders(p)) launches += 3;  // the order sort of a mixed batch

@@ -1,25 +1,21 @@
 // FP64 CDet integrand kernels for sm_103a.
 //
-// Three launches per batch of vertex configurations:
+// After the Green matrices (cdet_assembly.cu or cdet_split.cu), two launches
+// per batch of vertex configurations:
 //
-//  1. green_assembly_fp64: one thread per Green-matrix entry (configuration,
-//     table set, i, j). It decodes the two vertices, forms the lookup
-//     descriptor and evaluates the 2-D Chebyshev sum of the spin-up (and, when
-//     the tables differ, spin-down) block by the reference's Clenshaw
-//     recurrences, rows in descending order with the outer recurrence fused.
-//  2. principal_minors_fp64: one warp per (configuration, table set). The
+//  1. principal_minors_fp64: one warp per (configuration, table set). The
 //     warp runs the shifted Schur-complement recursion of mat2pm level by
 //     level, lanes spread over (set, row, column) work items, then the prefix
 //     product and the shift removal, and writes a[mask] = pm_up * pm_down into
-//     a lane-interleaved array for step 3.
-//  3. cdet_fp64: one lane per configuration, 32 configurations per warp. Each
+//     a lane-interleaved array for step 2.
+//  2. cdet_fp64: one lane per configuration, 32 configurations per warp. Each
 //     lane runs the connected-sum recursion of its configuration serially, in
 //     the reference's mask and submask order, so the FP64 pipe always runs
 //     full warps. It then applies the prefactors and forms
 //     twisted - 2 * ordinary.
 //
 // On GB300 the FP64 pipe retires about 504 G lane-operations per second and a
-// partially active warp costs as much as a full one, so all three kernels keep
+// partially active warp costs as much as a full one, so both kernels keep
 // every lane of every FP64 instruction busy.
 #include "cdet_device.cuh"
 #include "cdet_kernels.cuh"
@@ -29,238 +25,6 @@
 namespace cdet {
 
 namespace {
-
-// sampled_coordinate_to_index (g_funcs.h:315-342) on value*extent; flags
-// values the reference would reject (non-finite, outside the int range).
-__device__ __forceinline__ int coordinate_index(double scaled, int extent, bool& bad) {
-    if (!(scaled > -2147483648.0 && scaled < 2147483648.0)) {
-        bad = true;
-        return 0;
-    }
-    int index = static_cast<int>(floor(scaled));
-    if (index < 0) index = 0;
-    if (index >= extent) index = extent - 1;
-    return index;
-}
-
-struct Vertex {
-    double tau, tau_unit;
-    int x, y, replica;
-};
-
-// Vertex decode of integrand_temp_typed (integrand_replica_randomly_sampled.h:422-432).
-__device__ __forceinline__ Vertex decode_vertex(const double* __restrict__ v, const Scalars& s,
-                                                int replica_count, bool& bad) {
-    Vertex out;
-    const double tu = __ldg(v + 0);
-    if (!isfinite(tu)) bad = true;
-    out.tau_unit = tu;
-    out.tau = dmul(s.beta, tu);
-    out.x = coordinate_index(dmul(static_cast<double>(s.n1), __ldg(v + 1)), s.n1, bad);
-    out.y = coordinate_index(dmul(static_cast<double>(s.n2), __ldg(v + 2)), s.n2, bad);
-    out.replica = replica_count <= 1
-                      ? 0
-                      : coordinate_index(dmul(static_cast<double>(replica_count), __ldg(v + 3)),
-                                         replica_count, bad);
-    return out;
-}
-
-__device__ __forceinline__ double clamp_unit(double value) {
-    if (value < -1.0) return -1.0;
-    if (value > 1.0) return 1.0;
-    return value;
-}
-
-// ------------------------------------------------------ 1. assembly -------
-// Entry (i, j) of table set `set` of configuration c (order n): decode,
-// descriptor, Clenshaw sums, shifts and scale. With copy_retained, a pair of
-// vertices retained from the previous evaluation is copied instead.
-__device__ __forceinline__ void assemble_entry(const Problem& p, const Scratch& w, int64_t c, int set, int i, int j,
-                                               int n, bool copy_retained) {
-    const int nmax = p.max_order;
-    const int64_t per_set = static_cast<int64_t>(nmax) * nmax;
-    const Scalars& s = p.s;
-    const int replica_count = set == 0 ? 2 : 1;
-    bool bad = false;
-    const double* vbase = p.vertices + c * static_cast<int64_t>(nmax) * 4;
-    const Vertex vi = decode_vertex(vbase + 4 * i, s, replica_count, bad);
-    const Vertex vj = decode_vertex(vbase + 4 * j, s, replica_count, bad);
-    if (bad) {
-        atomicOr(p.status + c, kStatusBadInput);
-        return;
-    }
-    if (copy_retained && copy_reused_pair(p, w.green, w.diag, c, set, i, j, n)) return;
-
-    // prepare_green_lookup_descriptor (g_funcs.h:609-653).
-    const bool upper = (i != j) && (vi.tau_unit > vj.tau_unit);
-    const uint64_t sitepair =
-        ((((static_cast<uint64_t>(vi.replica) * 2u + static_cast<uint64_t>(vj.replica)) * s.n1 +
-           vi.x) * s.n2 + vi.y) * s.n1 + vj.x) * s.n2 + vj.y;
-    const double t_outer = upper ? vi.tau : vj.tau;  // the later time of the pair
-    const double t_inner = upper ? vj.tau : vi.tau;
-    const TableDev& tu = p.up[set];
-    const TableDev& td = p.down[set];
-    const bool one_spin = p.same_spin[set] != 0;
-    double up, down;
-    if (t_outer < s.branch_eps) {
-        up = __ldg((upper ? tu.upper_corners : tu.lower_corners) + sitepair);
-        down = one_spin ? up : __ldg((upper ? td.upper_corners : td.lower_corners) + sitepair);
-    } else {
-        const double u = clamp_unit(dsub(ddiv(dmul(2.0, t_outer), s.beta), 1.0));
-        const double v = clamp_unit(dsub(ddiv(dmul(2.0, t_inner), t_outer), 1.0));
-        const uint64_t base = sitepair * static_cast<uint64_t>(s.nu) * static_cast<uint64_t>(s.nv);
-        const double* bu = (upper ? tu.upper : tu.lower) + base;
-        OuterClenshaw ou;
-        ou.init(s.nu - 1, u);
-        if (one_spin) {
-            for (int a = s.nu - 1; a >= 0; --a)
-                ou.push(a, clenshaw_row(bu + static_cast<int64_t>(a) * s.nv, s.nv - 1, v));
-            up = down = ou.result();
-        } else {
-            const double* bd = (upper ? td.upper : td.lower) + base;
-            OuterClenshaw od;
-            od.init(s.nu - 1, u);
-            for (int a = s.nu - 1; a >= 0; --a) {
-                double ru, rd;
-                clenshaw_row_pair(bu + static_cast<int64_t>(a) * s.nv,
-                                  bd + static_cast<int64_t>(a) * s.nv, s.nv - 1, v, ru, rd);
-                ou.push(a, ru);
-                od.push(a, rd);
-            }
-            up = ou.result();
-            down = od.result();
-        }
-    }
-    // fill_pair_range (integrand_replica_randomly_sampled.h:467-473).
-    const int64_t mslot = (c * 2 + set) * 2;
-    if (i == j) {
-        const double up_raw = up, down_raw = down;
-        up = dadd(up, s.diag_up_shift);
-        down = dadd(down, s.diag_down_shift);
-        // the double-double order-1 branch adds its own shifts to the unshifted value
-        w.diag[mslot * nmax + i] = p.raw_diag ? up_raw : up;
-        w.diag[(mslot + 1) * nmax + i] = p.raw_diag ? down_raw : down;
-    }
-    w.green[mslot * per_set + i * n + j] = dmul(up, s.scale);
-    w.green[(mslot + 1) * per_set + i * n + j] = dmul(down, s.scale);
-}
-
-// One thread per (configuration, set, i, j) entry.
-__global__ void __launch_bounds__(128) green_assembly_fp64(const __grid_constant__ Problem p,
-                                                          const __grid_constant__ Scratch w) {
-    const int nmax = p.max_order;
-    const int64_t per_set = static_cast<int64_t>(nmax) * nmax;
-    const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (idx >= p.batch * 2 * per_set) return;
-    const int64_t c = idx / (2 * per_set);
-    const int64_t rem = idx - c * 2 * per_set;
-    const int set = static_cast<int>(rem / per_set);
-    const int pair = static_cast<int>(rem - set * per_set);
-    const int i = pair / nmax;
-    const int j = pair - i * nmax;
-    const int n = p.all_subsets ? nmax : __ldg(p.orders + c);
-    if (n < 1 || n > nmax) {
-        if (rem == 0) atomicOr(p.status + c, kStatusBadInput);
-        return;
-    }
-    if (i >= n || j >= n) return;
-    assemble_entry(p, w, c, set, i, j, n, p.reuse_mask != nullptr);
-}
-
-// Green-pair reuse in the FP64 assembly (all-subsets batches): the copies and
-// the evaluations go to separate launches, so no warp waits on another lane's
-// Clenshaw sums while its own lanes only copy. reuse_offsets: per
-// configuration the first of its fresh entries, 2 (n^2 - k^2) of them with k
-// retained vertices, exclusive over configurations, and the total.
-constexpr uint32_t kReuseTotalIndex = 56;  // the total's uint32 slot in Scratch::order_count
-
-__global__ void __launch_bounds__(1024) reuse_scan(const __grid_constant__ Problem p, int32_t* offsets,
-                                                   uint32_t* total) {
-    __shared__ uint32_t part[1024];
-    const int n = p.max_order;
-    const int64_t per = (p.batch + 1023) / 1024;
-    const int64_t begin = threadIdx.x * per, end = min(p.batch, begin + per);
-    uint32_t sum = 0;
-    for (int64_t c = begin; c < end; ++c) {
-        const int k = __popcll(__ldg(p.reuse_mask + c));
-        sum += 2u * static_cast<uint32_t>(n * n - k * k);
-    }
-    part[threadIdx.x] = sum;
-    __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {  // inclusive scan of the thread sums
-        const uint32_t add = threadIdx.x >= static_cast<unsigned>(off) ? part[threadIdx.x - off] : 0u;
-        __syncthreads();
-        part[threadIdx.x] += add;
-        __syncthreads();
-    }
-    uint32_t run = part[threadIdx.x] - sum;
-    for (int64_t c = begin; c < end; ++c) {
-        offsets[c] = static_cast<int32_t>(run);
-        const int k = __popcll(__ldg(p.reuse_mask + c));
-        run += 2u * static_cast<uint32_t>(n * n - k * k);
-    }
-    if (threadIdx.x == 1023) *total = part[1023];
-}
-
-// The copies: one thread per entry of the retained block (i, j < k).
-__global__ void __launch_bounds__(128) green_copy_retained(const __grid_constant__ Problem p,
-                                                          const __grid_constant__ Scratch w) {
-    const int n = p.max_order;
-    const int64_t per_set = static_cast<int64_t>(n) * n;
-    const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (idx >= p.batch * 2 * per_set) return;
-    const int64_t c = idx / (2 * per_set);
-    const int64_t rem = idx - c * 2 * per_set;
-    const int set = static_cast<int>(rem / per_set);
-    const int pair = static_cast<int>(rem - set * per_set);
-    const int i = pair / n, j = pair - (pair / n) * n;
-    const int k = __popcll(__ldg(p.reuse_mask + c));
-    if (i >= k || j >= k) return;
-    bool bad = false;  // the decode's checks, so the status bits are a fresh evaluation's
-    const double* vbase = p.vertices + c * n * 4;
-    decode_vertex(vbase + 4 * i, p.s, set == 0 ? 2 : 1, bad);
-    decode_vertex(vbase + 4 * j, p.s, set == 0 ? 2 : 1, bad);
-    if (bad) {
-        atomicOr(p.status + c, kStatusBadInput);
-        return;
-    }
-    copy_reused_pair(p, w.green, w.diag, c, set, i, j, n);
-}
-
-// The evaluations: one thread per fresh entry, compacted over the batch.
-// Fresh entries of a set, in order: rows i < k at columns k..n-1, then rows
-// i >= k at every column.
-__global__ void __launch_bounds__(128) green_assembly_fp64_fresh(const __grid_constant__ Problem p,
-                                                                const __grid_constant__ Scratch w,
-                                                                const int32_t* __restrict__ offsets,
-                                                                const uint32_t* __restrict__ total) {
-    const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (idx >= static_cast<int64_t>(__ldg(total))) return;
-    // the configuration: the last offset <= idx
-    int64_t lo = 0, hi = p.batch - 1;
-    while (lo < hi) {
-        const int64_t mid = (lo + hi + 1) >> 1;
-        if (static_cast<int64_t>(__ldg(offsets + mid)) <= idx) lo = mid;
-        else hi = mid - 1;
-    }
-    const int64_t c = lo;
-    const int n = p.max_order;
-    const int k = __popcll(__ldg(p.reuse_mask + c));
-    const int per = n * n - k * k;  // fresh entries per set (> 0 here: this configuration owns idx)
-    const int r = static_cast<int>(idx - __ldg(offsets + c));
-    const int set = r >= per ? 1 : 0;
-    const int rr = r - set * per;
-    int i, j;
-    if (rr < k * (n - k)) {
-        i = rr / (n - k);
-        j = k + (rr - i * (n - k));
-    } else {
-        const int q = rr - k * (n - k);
-        i = k + q / n;
-        j = q - (q / n) * n;
-    }
-    assemble_entry(p, w, c, set, i, j, n, false);
-}
 
 // ------------------------------------------------- 2. principal minors ----
 // Partial-pivot LU minor of the principal submatrix selected by mask
@@ -1693,13 +1457,6 @@ bool fp64_single_order_uses_dp_lanes(int max_order) {
     return !(max_order > kWarpCdetMaxOrder && max_order <= kBlockCdetMaxOrder);
 }
 
-cudaError_t launch_fp64_assembly_only(const Problem& p, const Scratch& w, cudaStream_t stream) {
-    if (p.batch <= 0) return cudaSuccess;
-    const int64_t entries = p.batch * 2 * static_cast<int64_t>(p.max_order) * p.max_order;
-    green_assembly_fp64<<<static_cast<unsigned>((entries + 127) / 128), 128, 0, stream>>>(p, w);
-    return cudaGetLastError();
-}
-
 // ------------------------------------------- order-sorted slots ----------
 // A counting sort of a mixed-order batch by decreasing order (invalid orders
 // last): config_at[slot] and slot_of[config]. Slots within one order follow
@@ -1957,18 +1714,7 @@ cudaError_t launch_fp64_integrand(const Problem& p_in, const Scratch& w, int sm_
     if (assembly) {
         mark(0);
         mark(1);
-        const int64_t entries = p_in.batch * 2 * static_cast<int64_t>(p_in.max_order) * p_in.max_order;
-        const unsigned grid = static_cast<unsigned>((entries + 127) / 128);
-        if (p_in.reuse_mask && p_in.all_subsets) {
-            // Green-pair reuse: scan of the fresh entries, copies, compacted evaluations
-            // (the configurations' slot array is free in an all-subsets evaluation)
-            reuse_scan<<<1, 1024, 0, stream>>>(p_in, w.slot_of, w.order_count + kReuseTotalIndex);
-            green_copy_retained<<<grid, 128, 0, stream>>>(p_in, w);
-            green_assembly_fp64_fresh<<<grid, 128, 0, stream>>>(p_in, w, w.slot_of, w.order_count + kReuseTotalIndex);
-        } else {
-            green_assembly_fp64<<<grid, 128, 0, stream>>>(p_in, w);
-        }
-        const cudaError_t err = cudaGetLastError();
+        const cudaError_t err = launch_fp64_assembly(p_in, w, sm_count, stream);
         if (err != cudaSuccess) return err;
         mark(2);
     }

@@ -299,7 +299,9 @@ cudaError_t launch_split_assembly(const Problem& p, const Scratch& w, const Spli
                                   size_t scratch_bytes, int sm_count, int32_t** error_flag_out,
                                   cudaStream_t stream, const KernelEvents* events);
 
-cudaError_t launch_fp64_assembly_only(const Problem& p, const Scratch& scratch, cudaStream_t stream);
+// The Green matrices of every configuration (with Green-pair reuse the
+// retained pairs copied), by the reference's FP64 Clenshaw recurrences.
+cudaError_t launch_fp64_assembly(const Problem& p, const Scratch& scratch, int sm_count, cudaStream_t stream);
 size_t minors_workspace_doubles(int max_order);
 // Whether the minors kernel keeps its per-warp workspace in global memory
 // (orders whose workspace does not fit four warps' worth of shared memory).
