@@ -21,8 +21,7 @@
 // arena per spin: 40.5 KB per warp at order 10 with one spin per set, five
 // warps per SM), the masks of a popcount level dealt to its lanes, each mask's
 // submask sum on one lane in the reference's order.
-#include "cdet_device.cuh"
-#include "cdet_kernels.cuh"
+#include "cdet_dd.cuh"
 
 #include <algorithm>
 
@@ -30,126 +29,13 @@ namespace cdet {
 
 namespace {
 
-// ------------------------------------------------ DoubleDouble (the rest) ---
-// operator/ (utility/types.h:114-120): q1 = x.hi / y.hi, the remainder
-// x - q1 y, q2 = (r.hi + r.lo) / y.hi, q1 + q2 renormalised.
-__device__ __forceinline__ DD dd_div(DD x, DD y) {
-    const double q1 = ddiv(x.hi, y.hi);
-    const DD r = dd_sub(x, dd_mul(DD{q1, 0.0}, y));
-    const double q2 = ddiv(dadd(r.hi, r.lo), y.hi);
-    DD q = dd_add(DD{q1, 0.0}, DD{q2, 0.0});
-    const double s = dadd(q.hi, q.lo);
-    q.lo = dsub(q.lo, dsub(s, q.hi));
-    q.hi = s;
-    return q;
-}
-// dd_abs (utility/types.h:221-223)
-__device__ __forceinline__ DD dd_abs(DD x) { return x.hi < 0.0 ? DD{-x.hi, -x.lo} : x; }
-// the comparison operators (utility/types.h:146-168): lexicographic on (hi, lo)
-__device__ __forceinline__ bool dd_lt(DD a, DD b) { return a.hi < b.hi || (a.hi == b.hi && a.lo < b.lo); }
-__device__ __forceinline__ bool dd_gt(DD a, DD b) { return dd_lt(b, a); }
-__device__ __forceinline__ bool dd_eq(DD a, DD b) { return a.hi == b.hi && a.lo == b.lo; }
-__device__ __forceinline__ bool dd_zero(DD a) { return a.hi == 0.0 && a.lo == 0.0; }
-// subtract_product for DoubleDouble (fast_principle_minors.h:30-37): base - left * right
-__device__ __forceinline__ DD dd_sub_prod(DD left, DD right, DD base) { return dd_sub(base, dd_mul(left, right)); }
-
-// The lighter steps used on the split assembly's Green matrices, where the
-// reference's values are not the contract: products as FMAs without the
-// lo x lo term, sums as one two-sum of the highs plus the lows and one
-// renormalisation (relative error a few 2^-104 of the operands).
-__device__ __forceinline__ DD dd_mul_light(DD x, DD y) {
-    const double p = dmul(x.hi, y.hi);
-    double e = dfma(x.hi, y.hi, -p);
-    e = dfma(x.hi, y.lo, e);
-    e = dfma(x.lo, y.hi, e);
-    DD r;
-    r.hi = quick_two_sum(p, e, r.lo);
-    return r;
-}
-__device__ __forceinline__ DD dd_add_light(DD x, DD y) {
-    double e;
-    const double s = two_sum(x.hi, y.hi, e);
-    e = dadd(e, dadd(x.lo, y.lo));
-    DD r;
-    r.hi = quick_two_sum(s, e, r.lo);
-    return r;
-}
-// base - left * right with the product as FMAs
-__device__ __forceinline__ DD dd_sub_prod_light(DD left, DD right, DD base) {
-    const double p = dmul(left.hi, right.hi);
-    double pe = dfma(left.hi, right.hi, -p);
-    pe = dfma(left.hi, right.lo, pe);
-    pe = dfma(left.lo, right.hi, pe);
-    double e;
-    const double s = two_sum(base.hi, -p, e);
-    e = dadd(e, dsub(base.lo, pe));
-    DD r;
-    r.hi = quick_two_sum(s, e, r.lo);
-    return r;
-}
-template <bool Exact>
-__device__ __forceinline__ DD mul_t(DD x, DD y) { return Exact ? dd_mul(x, y) : dd_mul_light(x, y); }
-template <bool Exact>
-__device__ __forceinline__ DD add_t(DD x, DD y) { return Exact ? dd_add(x, y) : dd_add_light(x, y); }
-template <bool Exact>
-__device__ __forceinline__ DD sub_prod_t(DD l, DD r, DD b) {
-    return Exact ? dd_sub_prod(l, r, b) : dd_sub_prod_light(l, r, b);
-}
-
 __device__ __forceinline__ DD shfl_dd(DD v, int src_lane_xor) {
     return DD{__shfl_xor_sync(0xffffffffu, v.hi, src_lane_xor), __shfl_xor_sync(0xffffffffu, v.lo, src_lane_xor)};
-}
-
-// determinant_principal_minor_from_buffer<DoubleDouble> (fast_principle_minors.h:39-105)
-// for one mask on one lane; m is this lane's n x n DoubleDouble scratch.
-__device__ DD minor_by_lu_dd(const DD* a, int n, uint32_t mask, DD* m) {
-    int idx[kMaxOrder];
-    int k = 0;
-    for (int i = 0; i < n; ++i)
-        if (mask & (1u << i)) idx[k++] = i;
-    if (k == 0) return DD{1.0, 0.0};
-    for (int r = 0; r < k; ++r)
-        for (int c = 0; c < k; ++c) m[r * k + c] = a[idx[r] * n + idx[c]];
-    DD det{1.0, 0.0};
-    int sign = 1;
-    for (int col = 0; col < k; ++col) {
-        int pivot_row = col;
-        DD pivot_abs = dd_abs(m[col * k + col]);
-        for (int row = col + 1; row < k; ++row) {
-            const DD cand = dd_abs(m[row * k + col]);
-            if (dd_gt(cand, pivot_abs)) {
-                pivot_abs = cand;
-                pivot_row = row;
-            }
-        }
-        if (dd_zero(pivot_abs)) return DD{0.0, 0.0};
-        if (pivot_row != col) {
-            for (int c = col; c < k; ++c) {
-                const DD t = m[col * k + c];
-                m[col * k + c] = m[pivot_row * k + c];
-                m[pivot_row * k + c] = t;
-            }
-            sign = -sign;
-        }
-        const DD pivot = m[col * k + col];
-        det = dd_mul(det, pivot);
-        for (int row = col + 1; row < k; ++row) {
-            const DD factor = dd_div(m[row * k + col], pivot);
-            if (dd_zero(factor)) continue;
-            m[row * k + col] = DD{0.0, 0.0};
-            for (int c = col + 1; c < k; ++c) m[row * k + c] = dd_sub_prod(factor, m[col * k + c], m[row * k + c]);
-        }
-    }
-    return sign < 0 ? DD{-det.hi, -det.lo} : det;
 }
 
 // mat2pm_from_buffer<DoubleDouble> (fast_principle_minors.h:120-246) for one
 // matrix on one warp: shifted[mask] (mask >= 1) ends as the principal minor of
 // the rows and columns in mask. Returns true when the LU fallback ran.
-// Exact: the reference's operations; otherwise the lighter steps for the
-// Schur updates, the minor sums and products and the shift removal (the
-// pivots, their inverses and the fallback decision stay exact).
-template <bool Exact>
 __device__ bool mat2pm_dd_warp(const DD* A, int n, DD tol, DD thresh, const WsLayout& lay, DD* ws, DD* shifted,
                                DD* lu_lane, int lane) {
     const int msize = n * n;
@@ -208,7 +94,7 @@ __device__ bool mat2pm_dd_warp(const DD* A, int n, DD tol, DD thresh, const WsLa
             const int set = item / new_size;
             const int row = item - set * new_size;
             DD* entry = old_list + set * old_msize + (row + 1) * old_size;
-            *entry = mul_t<Exact>(*entry, old_list[set * old_msize]);
+            *entry = dd_mul(*entry, old_list[set * old_msize]);
         }
         __syncwarp();
         if (level == n - 2) {
@@ -216,8 +102,8 @@ __device__ bool mat2pm_dd_warp(const DD* A, int n, DD tol, DD thresh, const WsLa
             for (int set = lane; set < sets; set += kWarp) {
                 const DD* m = old_list + set * 4;
                 const DD base = m[3];
-                shifted[minor_index + set] = add_t<Exact>(p, base);
-                shifted[minor_index + sets + set] = add_t<Exact>(p, sub_prod_t<Exact>(m[1], m[2], base));
+                shifted[minor_index + set] = dd_add(p, base);
+                shifted[minor_index + sets + set] = dd_add(p, dd_sub_prod(m[1], m[2], base));
             }
             __syncwarp();
             minor_index += 2 * sets;
@@ -235,11 +121,11 @@ __device__ bool mat2pm_dd_warp(const DD* A, int n, DD tol, DD thresh, const WsLa
             const DD base = old_list[src + (row + 1) * old_size + col + 1];
             new_list[item] = base;
             new_list[items + item] =
-                sub_prod_t<Exact>(old_list[src + 1 + col], old_list[src + (row + 1) * old_size], base);
+                dd_sub_prod(old_list[src + 1 + col], old_list[src + (row + 1) * old_size], base);
         }
         __syncwarp();
         for (int m = lane; m < 2 * sets; m += kWarp)
-            shifted[minor_index + m] = add_t<Exact>(p, new_list[m * new_msize]);
+            shifted[minor_index + m] = dd_add(p, new_list[m * new_msize]);
         minor_index += 2 * sets;
         old_list = new_list;
         __syncwarp();
@@ -253,7 +139,7 @@ __device__ bool mat2pm_dd_warp(const DD* A, int n, DD tol, DD thresh, const WsLa
     for (uint32_t step = 1; step < subsets; step <<= 1) {  // the prefix product over levels
 #pragma unroll 4
         for (uint32_t set = step + 1 + lane; set < 2 * step; set += kWarp)
-            shifted[set] = mul_t<Exact>(shifted[set], shifted[set - step]);
+            shifted[set] = dd_mul(shifted[set], shifted[set - step]);
         __syncwarp();
     }
     for (uint32_t step = subsets; step > 1; step >>= 1) {  // the shift removal, bit by bit from the top
@@ -262,7 +148,7 @@ __device__ bool mat2pm_dd_warp(const DD* A, int n, DD tol, DD thresh, const WsLa
 #pragma unroll 4
         for (uint32_t q = lane; q < subsets / 2; q += kWarp) {
             const uint32_t ss = ((q >> hb) << (hb + 1)) + half + (q & (half - 1u));
-            shifted[ss] = sub_prod_t<Exact>(p, shifted[ss - half], shifted[ss]);
+            shifted[ss] = dd_sub_prod(p, shifted[ss - half], shifted[ss]);
         }
         __syncwarp();
     }
@@ -304,19 +190,7 @@ __device__ DD cdet_dd_warp(const DD* a, DD* dp_s, int n, DD threshold, int lane)
 __device__ DD dd_set_value(const Problem& p, const Scratch& w, int64_t c, int set, int n, const WsLayout& lay,
                            DD* ws, DD* lu_lane, int lane, int32_t& status) {
     const int nmax = p.max_order;
-    const int r = set == 0 ? 2 : 1;
-    if (n == 1) {
-        // order1_density_integrand_from_sampled_vertex (:173-213) with
-        // IntegrandRealT = DoubleDouble: the unshifted diagonal widened, the
-        // DoubleDouble shifts added; no finiteness check on this branch
-        const double* diag = w.diag + c * 2 * 2 * nmax;
-        const DD su = dd_add(DD{diag[(set * 2) * nmax], 0.0}, DD{p.dd_shift[0].hi, p.dd_shift[0].lo});
-        const DD sd = dd_add(DD{diag[(set * 2 + 1) * nmax], 0.0}, DD{p.dd_shift[1].hi, p.dd_shift[1].lo});
-        const DD counter = dd_mul(DD{p.dd_shift[0].hi, p.dd_shift[0].lo}, DD{p.dd_shift[1].hi, p.dd_shift[1].lo});
-        const DD ru = dd_mul(dd_mul(DD{static_cast<double>(-r), 0.0}, DD{p.dd_u.hi, p.dd_u.lo}),
-                             DD{p.dd_beta.hi, p.dd_beta.lo});
-        return dd_mul(ru, dd_sub(dd_mul(su, sd), counter));
-    }
+    if (n == 1) return dd_order1_value(p, w, c, set);
     const double* green = w.green + (c * 2 + set) * 2 * static_cast<int64_t>(nmax) * nmax;
     DD* A = ws + lay.a;
     const DD tol{p.dd_tol.hi, p.dd_tol.lo}, thresh{p.dd_fpm_shift.hi, p.dd_fpm_shift.lo};
@@ -324,12 +198,12 @@ __device__ DD dd_set_value(const Problem& p, const Scratch& w, int64_t c, int se
     for (int k = lane; k < n * n; k += kWarp) A[k] = DD{green[k], 0.0};
     __syncwarp();
     DD* su = ws + lay.shifted_up;
-    fb |= mat2pm_dd_warp<true>(A, n, tol, thresh, lay, ws, su, lu_lane, lane);
+    fb |= mat2pm_dd_warp(A, n, tol, thresh, lay, ws, su, lu_lane, lane);
     const bool one_spin = p.same_spin[set] != 0;
     if (!one_spin) {
         for (int k = lane; k < n * n; k += kWarp) A[k] = DD{green[static_cast<int64_t>(nmax) * nmax + k], 0.0};
         __syncwarp();
-        fb |= mat2pm_dd_warp<true>(A, n, tol, thresh, lay, ws, ws + lay.shifted_down, lu_lane, lane);
+        fb |= mat2pm_dd_warp(A, n, tol, thresh, lay, ws, ws + lay.shifted_down, lu_lane, lane);
     }
     const DD* sd = one_spin ? su : ws + lay.shifted_down;
     // a[mask] = up[mask - 1] * down[mask - 1] (:254-257), in place of the up minors
@@ -395,7 +269,6 @@ __device__ __forceinline__ DD* lane_dp(const Scratch& w, int64_t slot, int set, 
            ((slot >> 5) * 2 + set) * (subsets / 2) * kWarp + (slot & 31);
 }
 
-template <bool Exact>
 __global__ void __launch_bounds__(kDDMaxWarps * 32) principal_minors_dd(const __grid_constant__ Problem p,
                                                           const __grid_constant__ Scratch w) {
     extern __shared__ double dd_smem[];
@@ -421,17 +294,17 @@ __global__ void __launch_bounds__(kDDMaxWarps * 32) principal_minors_dd(const __
         for (int k = lane; k < n * n; k += kWarp) A[k] = DD{green[k], 0.0};
         __syncwarp();
         DD* su = ws + lay.shifted_up;
-        fb |= mat2pm_dd_warp<Exact>(A, n, tol, thresh, lay, ws, su, lu_lane, lane);
+        fb |= mat2pm_dd_warp(A, n, tol, thresh, lay, ws, su, lu_lane, lane);
         const bool one_spin = p.same_spin[set] != 0;
         if (!one_spin) {
             for (int k = lane; k < n * n; k += kWarp) A[k] = DD{green[static_cast<int64_t>(nmax) * nmax + k], 0.0};
             __syncwarp();
-            fb |= mat2pm_dd_warp<Exact>(A, n, tol, thresh, lay, ws, ws + lay.shifted_down, lu_lane, lane);
+            fb |= mat2pm_dd_warp(A, n, tol, thresh, lay, ws, ws + lay.shifted_down, lu_lane, lane);
         }
         const DD* sd = one_spin ? su : ws + lay.shifted_down;
         DD* a = lane_a(w, __ldg(w.slot_of + c), set, nmax);
         for (uint32_t m = lane; m < (1u << n); m += kWarp)
-            a[static_cast<int64_t>(m) * kWarp] = m == 0 ? DD{0.0, 0.0} : mul_t<Exact>(su[m], sd[m]);
+            a[static_cast<int64_t>(m) * kWarp] = m == 0 ? DD{0.0, 0.0} : dd_mul(su[m], sd[m]);
         if (fb && lane == 0) atomicOr(p.status + c, kStatusFpmFallback);
         __syncwarp();
     }
@@ -440,14 +313,6 @@ __global__ void __launch_bounds__(kDDMaxWarps * 32) principal_minors_dd(const __
 // compute_dp_ztransform<DoubleDouble> for the slot's configuration on one
 // lane, masks holding vertex 0 in popcount order, each one's submasks in the
 // reference's descending order; then the prefactors and the combine.
-// Exact: the reference's DoubleDouble operations (51 FP64 operations per
-// pair update). Otherwise (the split assembly's Green matrices, where the
-// reference's values are not the contract): the product as FMAs without the
-// lo x lo term, the subtraction as one two-sum of the highs plus the lows and
-// one renormalisation, and the round-off filter's magnitude sum in FP64 on
-// the products' high parts (16 operations; the accumulated error stays near
-// 1e-32 of the terms' magnitude sum).
-template <bool Exact>
 __global__ void __launch_bounds__(32) cdet_dd_lane(const __grid_constant__ Problem p,
                                                    const __grid_constant__ Scratch w) {
     const int64_t slot = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -463,15 +328,8 @@ __global__ void __launch_bounds__(32) cdet_dd_lane(const __grid_constant__ Probl
     int32_t status = 0;
     DD value[2];
     for (int set = 0; set < 2; ++set) {
-        const int r = set == 0 ? 2 : 1;
         if (n == 1) {
-            const double* diag = w.diag + c * 2 * 2 * nmax;
-            const DD shu{p.dd_shift[0].hi, p.dd_shift[0].lo}, shd{p.dd_shift[1].hi, p.dd_shift[1].lo};
-            const DD su = dd_add(DD{diag[(set * 2) * nmax], 0.0}, shu);
-            const DD sd = dd_add(DD{diag[(set * 2 + 1) * nmax], 0.0}, shd);
-            const DD ru = dd_mul(dd_mul(DD{static_cast<double>(-r), 0.0}, DD{p.dd_u.hi, p.dd_u.lo}),
-                                 DD{p.dd_beta.hi, p.dd_beta.lo});
-            value[set] = dd_mul(ru, dd_sub(dd_mul(su, sd), dd_mul(shu, shd)));
+            value[set] = dd_order1_value(p, w, c, set);
             continue;
         }
         const DD* a = lane_a(w, slot, set, nmax);
@@ -481,34 +339,15 @@ __global__ void __launch_bounds__(32) cdet_dd_lane(const __grid_constant__ Probl
         for (int bits = 2; bits <= n; ++bits) {
             for (uint32_t rest = (1u << (bits - 1)) - 1u; rest < rest_limit; rest = next_same_popcount(rest)) {
                 DD acc = a[static_cast<int64_t>((rest << 1) | 1u) * kWarp];
-                if constexpr (Exact) {
-                    DD rhs = dd_abs(acc);
-                    for (uint32_t sm = (rest - 1u) & rest;; sm = (sm - 1u) & rest) {
-                        const DD term = dd_mul(dp[static_cast<int64_t>(sm) * kWarp],
-                                               a[static_cast<int64_t>((rest ^ sm) << 1) * kWarp]);
-                        acc = dd_sub(acc, term);
-                        rhs = dd_add(rhs, dd_abs(term));
-                        if (sm == 0) break;
-                    }
-                    if (filter && dd_lt(dd_abs(acc), dd_mul(threshold, rhs))) acc = zero;
-                } else {
-                    double rhs = fabs(acc.hi);
-                    for (uint32_t sm = (rest - 1u) & rest;; sm = (sm - 1u) & rest) {
-                        const DD x = dp[static_cast<int64_t>(sm) * kWarp];
-                        const DD y = a[static_cast<int64_t>((rest ^ sm) << 1) * kWarp];
-                        const double ph = dmul(x.hi, y.hi);
-                        double pe = dfma(x.hi, y.hi, -ph);
-                        pe = dfma(x.hi, y.lo, pe);
-                        pe = dfma(x.lo, y.hi, pe);
-                        double e;
-                        const double s = two_sum(acc.hi, -ph, e);
-                        e = dadd(e, dsub(acc.lo, pe));
-                        acc.hi = quick_two_sum(s, e, acc.lo);
-                        rhs = dadd(rhs, fabs(ph));
-                        if (sm == 0) break;
-                    }
-                    if (filter && fabs(acc.hi) < dmul(threshold.hi, rhs)) acc = zero;
+                DD rhs = dd_abs(acc);
+                for (uint32_t sm = (rest - 1u) & rest;; sm = (sm - 1u) & rest) {
+                    const DD term = dd_mul(dp[static_cast<int64_t>(sm) * kWarp],
+                                           a[static_cast<int64_t>((rest ^ sm) << 1) * kWarp]);
+                    acc = dd_sub(acc, term);
+                    rhs = dd_add(rhs, dd_abs(term));
+                    if (sm == 0) break;
                 }
+                if (filter && dd_lt(dd_abs(acc), dd_mul(threshold, rhs))) acc = zero;
                 dp[static_cast<int64_t>(rest) * kWarp] = acc;
                 if (bits == n) break;  // one mask at the top level
             }
@@ -529,6 +368,8 @@ static int64_t dd_lane_min_batch(int sm_count) { return static_cast<int64_t>(sm_
 
 cudaError_t launch_integrand_dd(const Problem& p, const Scratch& w, int sm_count, cudaStream_t stream) {
     if (p.batch <= 0) return cudaSuccess;
+    // on the split assembly the reference's DoubleDouble steps are not the contract: 113-bit integer arithmetic
+    if (p.fused_cdet) return launch_integrand_wide(p, w, sm_count, stream);
     const bool two_spins = !(p.same_spin[0] && p.same_spin[1]);
     const bool lanes = p.integrand_form == kIntegrandStaged ||
                        (p.integrand_form == kIntegrandAuto && p.batch >= dd_lane_min_batch(sm_count));
@@ -540,19 +381,14 @@ cudaError_t launch_integrand_dd(const Problem& p, const Scratch& w, int sm_count
         int64_t blocks = std::min<int64_t>(static_cast<int64_t>(sms) * per_sm, (p.batch * 2 + wpb - 1) / wpb);
         blocks = std::min<int64_t>(blocks, std::max<int64_t>(1, static_cast<int64_t>(w.ws_warps) / (2 * wpb)));
         const size_t smem = ws_bytes * wpb;
-        auto minors = p.fused_cdet ? principal_minors_dd<false> : principal_minors_dd<true>;
-        cudaError_t err = cudaFuncSetAttribute(minors, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t err = cudaFuncSetAttribute(principal_minors_dd, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                static_cast<int>(smem));
         if (err != cudaSuccess) return err;
-        minors<<<static_cast<unsigned>(blocks), wpb * kWarp, smem, stream>>>(p, w);
+        principal_minors_dd<<<static_cast<unsigned>(blocks), wpb * kWarp, smem, stream>>>(p, w);
         err = cudaGetLastError();
         if (err != cudaSuccess) return err;
-        // the reference's arithmetic on the FP64 assembly; the lighter one on the split assembly
         // one warp per block, so that a small batch still spreads over every SM
-        if (p.fused_cdet)
-            cdet_dd_lane<false><<<static_cast<unsigned>((p.batch + kWarp - 1) / kWarp), kWarp, 0, stream>>>(p, w);
-        else
-            cdet_dd_lane<true><<<static_cast<unsigned>((p.batch + kWarp - 1) / kWarp), kWarp, 0, stream>>>(p, w);
+        cdet_dd_lane<<<static_cast<unsigned>((p.batch + kWarp - 1) / kWarp), kWarp, 0, stream>>>(p, w);
         return cudaGetLastError();
     }
     const size_t ws_bytes = compact_minors_layout(p.max_order, two_spins, true).total * sizeof(DD);

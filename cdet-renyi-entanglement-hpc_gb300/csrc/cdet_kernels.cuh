@@ -389,6 +389,8 @@ bool uses_queue_form(const Problem& p);
 constexpr int kDDMaxOrder = 10;
 constexpr int kDDMaxWarps = 8;  // warps per block of the double-double minors and warp-form kernels
 cudaError_t launch_integrand_dd(const Problem& p, const Scratch& scratch, int sm_count, cudaStream_t stream);
+// The same integrand behind the split assembly, in 113-bit integer arithmetic.
+cudaError_t launch_integrand_wide(const Problem& p, const Scratch& scratch, int sm_count, cudaStream_t stream);
 // The post-assembly stages alone (sort, minors, CDet, or the queue kernel),
 // on Green matrices already in scratch: what the autotuner times.
 cudaError_t launch_post_assembly(const Problem& p, const Scratch& scratch, int sm_count, cudaStream_t stream);

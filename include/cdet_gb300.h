@@ -483,19 +483,19 @@ enum cdet_integrand_real {
  * DoubleDouble arithmetic on the Green matrices of the context's assembly:
  * with CDET_ASSEMBLY_FP64 (VECTOR_REAL=double) cdet_integrand_device / _host
  * return the reference's double-double values bit for bit; with
- * CDET_ASSEMBLY_SPLIT_BF16 the same arithmetic runs on the tensor-core
+ * CDET_ASSEMBLY_SPLIT_BF16 the same recursion runs on the tensor-core
  * Green matrices (no counterpart in the reference: its values differ from
  * the reference mode's by what the Green entries' last bits move, not by the
  * FP64 recursion's round-off). dd may be null for CDET_INTEGRAND_REAL_DOUBLE.
  * Single-configuration integrands of order <= 10 only: an all-subsets call or
- * a higher order fails with CDET_ERR_INVALID. Its work layout follows
- * cdet_set_integrand_form: CDET_INTEGRAND_STAGED = minors by warps, then the
- * recursion one lane per configuration; CDET_INTEGRAND_QUEUE = one warp per
- * configuration; AUTO = the lane layout from one warp of configurations per
- * SM. On the FP64 assembly both layouts give the reference's values; on the
- * split assembly the lane layout's minors and recursion take lighter
- * double-double steps (FMA products, one renormalisation per sum, the
- * filter's magnitude sum in FP64), so there they differ in the last bits. */
+ * a higher order fails with CDET_ERR_INVALID. On the FP64 assembly the work
+ * layout follows cdet_set_integrand_form: CDET_INTEGRAND_STAGED = minors by
+ * warps, then the recursion one lane per configuration;
+ * CDET_INTEGRAND_QUEUE = one warp per configuration; AUTO = the lane layout
+ * from one warp of configurations per SM; all give the reference's values. On
+ * the split assembly every form is the same kernel, whose minors and recursion
+ * run in 113-bit arithmetic on the integer pipes (at least the DoubleDouble
+ * steps' accuracy, not their last bits). */
 int cdet_set_integrand_real(cdet_context* ctx, int real_type, const cdet_dd_scalars* dd);
 
 /* Builds the bf16 slices of every uploaded table for the split assembly
