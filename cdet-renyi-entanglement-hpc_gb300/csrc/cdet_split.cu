@@ -211,18 +211,38 @@ __device__ __forceinline__ double int128_to_double(int64_t hi, uint64_t lo, int 
     return __longlong_as_double(static_cast<long long>(bits));
 }
 
+// x = hi 2^32 + lo with both halves signed (|x| <= 2^62): the four partial
+// products of two such numbers are plain signed 32 x 32 multiply-adds, with no
+// sign corrections.
+struct SignedHalves {
+    int32_t hi, lo;
+};
+__host__ __device__ __forceinline__ SignedHalves signed_halves(int64_t x) {
+    const int32_t lo = static_cast<int32_t>(x);
+    return SignedHalves{static_cast<int32_t>(x >> 32) + (lo < 0 ? 1 : 0), lo};
+}
+
+// floor((a b + round) / 2^Shift) modulo 2^64, 32 < Shift < 64. |a|, |b| <=
+// 2^62, so no partial sum leaves 64 bits. Four multiply-adds and about eight
+// other instructions; the same product as 64-bit low and high halves takes
+// about 28.
+template <int Shift>
+__host__ __device__ __forceinline__ int64_t mul_shift(SignedHalves a, SignedHalves b, int64_t round) {
+    const int64_t low = static_cast<int64_t>(a.lo) * b.lo + round;
+    int64_t mid = static_cast<int64_t>(a.hi) * b.lo + (low >> 32);
+    mid = static_cast<int64_t>(a.lo) * b.hi + mid;
+    const uint64_t high = static_cast<uint64_t>(static_cast<int64_t>(a.hi) * b.hi);
+    return static_cast<int64_t>((high << (64 - Shift)) + static_cast<uint64_t>(mid >> (Shift - 32)));
+}
+
 // One step of the Chebyshev recurrence T_{k+1} = 2 u T_k - T_{k-1} in Q62
 // fixed point (u, T in [-1, 1] scaled by 2^62). The 128-bit product is
 // rounded to Q62; the wrap-around 64-bit arithmetic is exact because the
 // result lies in [-1, 1]. The rounding error per step is 2^-63 and grows at
 // most like k^2 (about 2^-50 at degree 128), 2^11 below the FP64 recurrence.
 __device__ __forceinline__ int64_t cheb_step_q62(int64_t ufix, int64_t t, int64_t tprev) {
-    const uint64_t lo = static_cast<uint64_t>(ufix) * static_cast<uint64_t>(t);
-    uint64_t hi = static_cast<uint64_t>(__mul64hi(ufix, t));
-    const uint64_t lo2 = lo + (uint64_t{1} << 60);
-    hi += lo2 < lo ? 1u : 0u;
-    const uint64_t twice = (hi << 3) | (lo2 >> 61);  // round(2 u t) in Q62, modulo 2^64
-    return static_cast<int64_t>(twice - static_cast<uint64_t>(tprev));
+    const int64_t twice = mul_shift<61>(signed_halves(ufix), signed_halves(t), int64_t{1} << 60);
+    return static_cast<int64_t>(static_cast<uint64_t>(twice) - static_cast<uint64_t>(tprev));
 }
 
 // Two fp16 digits (the same slice of two consecutive k) from the biased
@@ -1328,11 +1348,9 @@ __global__ void __launch_bounds__(kAssemblyThreads, 1) split_assembly(const __gr
 #pragma unroll
                     for (int q = 0; q < 8; ++q) {
                         const int64_t tf = ch[q & 3].next(w8);
-                        const uint64_t plo = static_cast<uint64_t>(wfix[q]) * static_cast<uint64_t>(tf);
-                        int64_t phi = __mul64hi(wfix[q], tf);
-                        const uint64_t plo2 = plo + (uint64_t{1} << 61);
-                        phi += plo2 < plo ? 1 : 0;
-                        const int64_t prod = static_cast<int64_t>((static_cast<uint64_t>(phi) << 2) | (plo2 >> 62));
+                        // |wfix| < 2^62, |tf| <= 2^62
+                        const int64_t prod =
+                            mul_shift<62>(signed_halves(wfix[q]), signed_halves(tf), int64_t{1} << 61);
                         const uint64_t nlo = slo + static_cast<uint64_t>(prod);
                         shi += (prod < 0 ? -1 : 0) + (nlo < slo ? 1 : 0);
                         slo = nlo;
