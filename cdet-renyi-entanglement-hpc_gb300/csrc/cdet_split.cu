@@ -138,17 +138,22 @@ __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32
         : "memory");
 }
 
+// The MMA warp runs its loop converged, so that addresses and descriptors are
+// warp-uniform; `issue` (nonzero on one lane, always the same) picks the
+// thread that issues the instruction.
 __device__ __forceinline__ void mma_f16(uint32_t tmem, uint64_t adesc, uint64_t bdesc,
-                                         uint32_t idesc, uint32_t accumulate) {
+                                         uint32_t idesc, uint32_t accumulate, uint32_t issue) {
     asm volatile(
-        "{.reg .pred p; setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;}\n" ::"r"(tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
+        "{.reg .pred p, q; setp.ne.b32 p, %4, 0; setp.ne.b32 q, %5, 0;\n"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;}\n" ::"r"(tmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(issue));
 }
 
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-        smem_addr(bar)));
+__device__ __forceinline__ void mma_commit(uint64_t* bar, uint32_t issue) {
+    asm volatile(
+        "{.reg .pred q; setp.ne.b32 q, %1, 0;\n"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];}" ::"r"(smem_addr(bar)),
+        "r"(issue));
 }
 
 // ------------------------------------------------------ fixed-point helpers --
@@ -755,7 +760,6 @@ struct SplitShared {
     alignas(1024) uint16_t basis_ring[kBStages][kBStepBytes / 2];   // 3 x 28 KiB
     alignas(16) int64_t sums[kTileN][2];                             // second group's (lo, hi) per lookup
     TileMeta meta[kMetaBufs];
-    uint32_t c_lead[kCStages];  // first coefficient slice streamed into each stage (written before its copy)
     uint64_t c_full[kCStages], c_empty[kCStages];
     uint64_t b_full[kBStages], b_empty[kBStages];
     uint64_t meta_full[kMetaBufs], meta_empty[kMetaBufs];
@@ -959,31 +963,32 @@ __device__ __forceinline__ void tmem_load_4x2(uint32_t addr, uint32_t (&v)[8]) {
 }
 
 // The 29 digit-pair MMAs of a K step: coefficient slice t (8: the pre-scaled
-// eighth digit) against basis slice t', interleaved so that two MMAs into
-// the same accumulator are at least 3 apart; within a level the pairs are in
-// increasing t (the eighth digit last), so each accumulator sums its
-// products in the same order and its first MMA (t = 1, in a tile's first K
-// step, which is always complete) initialises it.
+// eighth digit) against basis slice t', by increasing t, so that a K step with
+// lead L is the tail of the list from slice L on: every lead runs the same
+// straight-line code from its own entry (eight copies of the list, one per
+// lead, cost the issuing warp an instruction fetch from beyond its cache in
+// every K step). Each accumulator level still takes its products in
+// increasing t, the eighth digit last, and its first MMA (t = 1, in a tile's
+// first K step, which is always complete) initialises it. Within a slice t'
+// runs so that two MMAs into one accumulator are at least 3 apart where the
+// slice has that many.
 constexpr int kIssue = 29;
-__device__ constexpr int8_t kIssueT[kIssue] = {1, 1, 1, 1, 1, 2, 2, 1, 2, 3, 2, 2, 3, 4, 3,
-                                               1, 5, 4, 3, 4, 3, 6, 2, 5, 7, 5, 4, 6, 8};
-__device__ constexpr int8_t kIssueTp[kIssue] = {3, 5, 7, 6, 4, 6, 4, 2, 5, 5, 2, 3, 4, 4, 3,
-                                                1, 3, 3, 2, 2, 1, 2, 1, 2, 1, 1, 1, 1, 1};
+__device__ constexpr int8_t kIssueT[kIssue] = {1, 1, 1, 1, 1, 1, 1, 2, 2, 2, 2, 2, 2, 3, 3,
+                                               3, 3, 3, 4, 4, 4, 4, 5, 5, 5, 6, 6, 7, 8};
+__device__ constexpr int8_t kIssueTp[kIssue] = {1, 2, 3, 4, 5, 6, 7, 1, 2, 3, 4, 5, 6, 1, 2,
+                                                3, 4, 5, 1, 2, 3, 4, 1, 2, 3, 1, 2, 1, 1};
 
-// One K step's MMAs with coefficient slices from Lead on, as straight-line
-// code: every operand is in a register before the first MMA, so the single
-// issuing thread puts them into the tensor pipe back to back (computing an
-// operand or branching between two MMAs costs the thread tens of clocks of
-// latency, which the tensor pipe would spend idle).
-template <int Lead, bool First>
-__device__ __forceinline__ void issue_kstep(const uint32_t (&d)[kLevels], const uint32_t (&idesc)[kLevels],
-                                            const uint64_t (&ad)[kSlices], const uint64_t (&bd)[kSlicesA]) {
+// The MMAs of coefficient slice T.
+template <int T>
+__device__ __forceinline__ void issue_slice(const uint32_t (&d)[kLevels], const uint32_t (&idesc)[kLevels], uint64_t a0,
+                                            uint64_t b0, uint32_t accumulate, uint32_t issue) {
 #pragma unroll
     for (int i = 0; i < kIssue; ++i) {
-        const int t = kIssueT[i], tp = kIssueTp[i];
-        if (t < Lead) continue;
-        const int lv = t == 8 ? kLevels - 1 : t + tp - 2;
-        mma_f16(d[lv], ad[tp - 1], bd[t - 1], idesc[lv], (First && t == 1) ? 0u : 1u);
+        if (kIssueT[i] != T) continue;
+        const int tp = kIssueTp[i];
+        const int lv = T == 8 ? kLevels - 1 : T + tp - 2;
+        mma_f16(d[lv], a0 + (tp - 1) * (kSliceBytes / 16), b0 + (T - 1) * (kSliceBytes / 16), idesc[lv],
+                T == 1 ? accumulate : 1u, issue);
     }
 }
 
@@ -1441,7 +1446,6 @@ __global__ void __launch_bounds__(kAssemblyThreads, 1) split_assembly(const __gr
                         // stage completes by a copy)
                         const int lead = step_lead(src.leads, ks);
                         const uint16_t* from = src.a + static_cast<int64_t>(ks) * (kAStageBytes / 2);
-                        sh.c_lead[st] = static_cast<uint32_t>(lead);
                         const int cols = max(g.cols, 16);
                         if (g.row0 == 0 && cols == kRows) {  // whole slices: one copy
                             const uint32_t offset = static_cast<uint32_t>(lead - 1) * (kRows * kKStep);
@@ -1472,96 +1476,89 @@ __global__ void __launch_bounds__(kAssemblyThreads, 1) split_assembly(const __gr
         }
     } else if (warp == kWarpMma) {
         // ---------------------------------------------------- MMA issue --
-        if (lane == 0) {
-            uint32_t c_cnt = 0, b_cnt = 0, pass_cnt = 0;
-            unsigned long long mmas = 0;
-            bool ok = true, issued = false;
-            for (uint32_t tile = tile_begin; ok && tile < tile_end && !failed(sh); ++tile) {
-                const TileSource src = tile_source<Chunked>(plan, tiles[tile].block);
-                const uint64_t rows = __ldg(reinterpret_cast<const unsigned long long*>(src.rows));
-                const int npass = pass_geom(rows, 0).npass;
-                for (int pass = 0; ok && pass < npass; ++pass, ++pass_cnt) {
-                    const PassGeom g = pass_geom(rows, pass);
-                    // the previous pass's accumulators have been drained
-                    if (pass_cnt > 0 && !mbar_wait(&sh.acc_empty, (pass_cnt - 1) & 1)) {
+        // the whole warp, converged; lane 0 issues
+        const uint32_t issue = lane == 0 ? 1u : 0u;
+        const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
+        uint32_t cnt = 0, pass_cnt = 0;  // K steps (the rings' position), passes
+        unsigned long long mmas = 0;
+        bool ok = true;
+        for (uint32_t tile = tile_begin; ok && tile < tile_end && !__any_sync(0xffffffffu, failed(sh)); ++tile) {
+            const TileSource src = tile_source<Chunked>(plan, tiles[tile].block);
+            const uint64_t rows = __ldg(reinterpret_cast<const unsigned long long*>(src.rows));
+            // lane ks holds K step ks's lead (1 in a tile's first): pairs with
+            // a coefficient slice before it are zero, not issued
+            const int my_lead = lane < src.ksteps ? step_lead(src.leads, lane) : kSlicesA;
+            const int ksteps = __shfl_sync(0xffffffffu, src.ksteps, 0);
+            const int npass = __shfl_sync(0xffffffffu, pass_geom(rows, 0).npass, 0);
+            for (int pass = 0; ok && pass < npass; ++pass, ++pass_cnt) {
+                const PassGeom g = pass_geom(rows, pass);
+                // per-level accumulator addresses and instruction descriptors
+                // of the pass; a level without columns writes 16 columns of
+                // the sink at the top of tensor memory, which nothing reads
+                uint32_t dcol[kLevels], idesc[kLevels];
+#pragma unroll
+                for (int lv = 0; lv < kLevels; ++lv) {
+                    const int n = __shfl_sync(0xffffffffu, g.n[lv], 0), col = __shfl_sync(0xffffffffu, g.col[lv], 0);
+                    dcol[lv] = tmem_u + static_cast<uint32_t>(n > 0 ? col : kTmemSink);
+                    idesc[lv] = mma_idesc(kTileN, n > 0 ? n : 16);
+                }
+                const int row0 = __shfl_sync(0xffffffffu, g.row0, 0);
+                // the previous pass's accumulators have been drained
+                const bool drained = pass_cnt == 0 || mbar_wait(&sh.acc_empty, (pass_cnt - 1) & 1);
+                if (!__all_sync(0xffffffffu, drained)) {  // (the lanes leave together)
+                    ok = false;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;");
+                for (int ks = 0; ks < ksteps; ++ks, ++cnt) {
+                    const int sc = static_cast<int>(cnt % kCStages);
+                    const int sb = static_cast<int>(cnt % kBStages);
+                    const int lead = __shfl_sync(0xffffffffu, my_lead, ks);
+                    // the stages' first slices; a slice further on is the same
+                    // descriptor plus its byte offset / 16 (the 14-bit address
+                    // field cannot carry: shared memory < 256 KiB)
+                    const uint64_t a0 = smem_desc(smem_addr(sh.basis_ring[sb]), 128, 256);
+                    const uint64_t b0 = smem_desc(smem_addr(sh.coeff_ring[sc] + row0 * kKStep), 128, 256);
+                    const uint32_t accumulate = ks > 0 ? 1u : 0u;
+                    const bool ready = mbar_wait(&sh.c_full[sc], (cnt / kCStages) & 1) &&
+                                       mbar_wait(&sh.b_full[sb], (cnt / kBStages) & 1);
+                    if (!__all_sync(0xffffffffu, ready)) {
                         ok = false;
                         break;
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;");
-                    // per-level accumulator addresses and instruction descriptors
-                    // of the pass; a level without columns writes 16 columns of
-                    // the sink at the top of tensor memory, which nothing reads
-                    uint32_t dcol[kLevels], idesc[kLevels];
-#pragma unroll
-                    for (int lv = 0; lv < kLevels; ++lv) {
-                        dcol[lv] = tmem + static_cast<uint32_t>(g.n[lv] > 0 ? g.col[lv] : kTmemSink);
-                        idesc[lv] = mma_idesc(kTileN, g.n[lv] > 0 ? g.n[lv] : 16);
+                    switch (lead) {
+                        case 1: issue_slice<1>(dcol, idesc, a0, b0, accumulate, issue); [[fallthrough]];
+                        case 2: issue_slice<2>(dcol, idesc, a0, b0, accumulate, issue); [[fallthrough]];
+                        case 3: issue_slice<3>(dcol, idesc, a0, b0, accumulate, issue); [[fallthrough]];
+                        case 4: issue_slice<4>(dcol, idesc, a0, b0, accumulate, issue); [[fallthrough]];
+                        case 5: issue_slice<5>(dcol, idesc, a0, b0, accumulate, issue); [[fallthrough]];
+                        case 6: issue_slice<6>(dcol, idesc, a0, b0, accumulate, issue); [[fallthrough]];
+                        case 7: issue_slice<7>(dcol, idesc, a0, b0, accumulate, issue); [[fallthrough]];
+                        default: issue_slice<8>(dcol, idesc, a0, b0, accumulate, issue);
                     }
-                    // accumulator columns a K step's MMAs write, by its lead (the
-                    // counter of issued tensor work: 2 x 128 x 16 flops per column)
-                    uint32_t cols_at_lead[kSlicesA + 1] = {};
+                    mma_commit(&sh.c_empty[sc], issue);
+                    mma_commit(&sh.b_empty[sb], issue);
+                }
+                if (!ok) break;
+                mma_commit(&sh.acc_full, issue);
+                // the counter of issued tensor work (accumulator columns, each
+                // 2 x 128 x 16 flops), off the issue path: lane ks adds up K step ks
+                if (lane < ksteps) {
 #pragma unroll
-                    for (int i = 0; i < kIssue; ++i) {
-                        const int t = kIssueT[i], tp = kIssueTp[i];
-                        const int lv = t == 8 ? kLevels - 1 : t + tp - 2;
-#pragma unroll
-                        for (int lead = 1; lead <= kSlicesA; ++lead)
-                            if (t >= lead) cols_at_lead[lead] += g.n[lv] > 0 ? g.n[lv] : 16;
+                    for (int lv = 0; lv < kLevels; ++lv) {  // pairs (t, lv + 2 - t) with lead <= t; the eighth digit's
+                        const int pairs = max(0, lv + 2 - my_lead) + (lv == kLevels - 1 ? 1 : 0);
+                        mmas += static_cast<uint32_t>(pairs * (g.n[lv] > 0 ? g.n[lv] : 16));
                     }
-                    for (int ks = 0; ks < src.ksteps; ++ks, ++c_cnt, ++b_cnt) {
-                        const int sc = static_cast<int>(c_cnt % kCStages);
-                        const int sb = static_cast<int>(b_cnt % kBStages);
-                        if (!mbar_wait(&sh.c_full[sc], (c_cnt / kCStages) & 1) ||
-                            !mbar_wait(&sh.b_full[sb], (b_cnt / kBStages) & 1)) {
-                            ok = false;
-                            break;
-                        }
-                        asm volatile("tcgen05.fence::after_thread_sync;");
-                        // the stage's lead (1 in a tile's first K step): pairs
-                        // with a coefficient slice before it are zero, not issued
-                        const int lead = static_cast<int>(*static_cast<volatile uint32_t*>(&sh.c_lead[sc]));
-                        // descriptors of every slice of the two stages (rows row0..
-                        // of the coefficients), all in registers before the MMAs;
-                        // a slice further on is the same descriptor plus its byte
-                        // offset / 16 (the 14-bit address field cannot carry:
-                        // shared memory < 256 KiB)
-                        uint64_t ad[kSlices], bd[kSlicesA];
-                        const uint64_t a0 = smem_desc(smem_addr(sh.basis_ring[sb]), 128, 256);
-                        const uint64_t b0 = smem_desc(smem_addr(sh.coeff_ring[sc] + g.row0 * kKStep), 128, 256);
-#pragma unroll
-                        for (int k = 0; k < kSlices; ++k) ad[k] = a0 + k * (kSliceBytes / 16);
-#pragma unroll
-                        for (int k = 0; k < kSlicesA; ++k) bd[k] = b0 + k * (kSliceBytes / 16);
-                        if (ks == 0) {
-                            issue_kstep<1, true>(dcol, idesc, ad, bd);
-                        } else {
-                            switch (lead) {
-                                case 1: issue_kstep<1, false>(dcol, idesc, ad, bd); break;
-                                case 2: issue_kstep<2, false>(dcol, idesc, ad, bd); break;
-                                case 3: issue_kstep<3, false>(dcol, idesc, ad, bd); break;
-                                case 4: issue_kstep<4, false>(dcol, idesc, ad, bd); break;
-                                case 5: issue_kstep<5, false>(dcol, idesc, ad, bd); break;
-                                case 6: issue_kstep<6, false>(dcol, idesc, ad, bd); break;
-                                case 7: issue_kstep<7, false>(dcol, idesc, ad, bd); break;
-                                default: issue_kstep<8, false>(dcol, idesc, ad, bd); break;
-                            }
-                        }
-                        mmas += cols_at_lead[ks == 0 ? 1 : lead];
-                        issued = true;
-                        mma_commit(&sh.c_empty[sc]);
-                        mma_commit(&sh.b_empty[sb]);
-                    }
-                    if (!ok) break;
-                    mma_commit(&sh.acc_full);
                 }
             }
-            if (!ok) sh.error = 1;
-            if (counters) atomicAdd(counters, mmas);
-            // every MMA issued has completed before the columns are freed
-            if (issued) {
-                mma_commit(&sh.drain);
-                if (!mbar_wait(&sh.drain, 0)) sh.error = 1;
-            }
+        }
+        if (!ok) sh.error = 1;
+        if (counters) atomicAdd(counters, mmas);
+        // every MMA issued has completed before the columns are freed
+        if (cnt > 0) {
+            mma_commit(&sh.drain, issue);
+            if (!mbar_wait(&sh.drain, 0)) sh.error = 1;
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
