@@ -115,21 +115,18 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 // kSuspendNs), so a waiting warp takes no issue slots from the warps that
 // share its scheduler.
 constexpr uint32_t kSuspendNs = 200000;
-__device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
-    uint32_t done = 0;
-    asm volatile(
-        "{.reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p;}"
-        : "=r"(done)
-        : "r"(smem_addr(bar)), "r"(parity), "r"(kSuspendNs)
-        : "memory");
-    return done != 0;
-}
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-    if (mbar_try(bar, parity)) return true;  // (the clock is read only where the wait is not over at once)
+    uint32_t done = 0;
     const long long start = clock64();
-    while (!mbar_try(bar, parity))
+    while (true) {
+        asm volatile(
+            "{.reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p;}"
+            : "=r"(done)
+            : "r"(smem_addr(bar)), "r"(parity), "r"(kSuspendNs)
+            : "memory");
+        if (done) return true;
         if (clock64() - start > kWaitCycles) return false;
-    return true;
+    }
 }
 
 __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32_t bytes,
@@ -730,10 +727,8 @@ __global__ void __launch_bounds__(256) split_scatter(const SplitRecordArrays rec
 // 2^-16 resolution those digits need); rows that no level below 7 reaches
 // (|W| < 2^24 units of 2^-55) take their T_a(u) from Q30 chains, a 32 x 32
 // product and a 64-bit sum.
-// stages of the ring: a K step's coefficient slices (a bulk copy) and basis
-// slices (the producers) fill one stage and its MMAs free it, so one barrier
-// each way serves both operands
-constexpr int kStages = 3;
+constexpr int kCStages = 3;   // coefficient ring
+constexpr int kBStages = 3;   // basis ring
 constexpr int kMetaBufs = 2;
 constexpr int kProducerWarps = 4;
 constexpr int kEpilogueGroups = 2;
@@ -761,11 +756,12 @@ struct TileMeta {
 };
 
 struct SplitShared {
-    alignas(1024) uint16_t coeff_ring[kStages][kAStageBytes / 2];  // 3 x 32 KiB
-    alignas(1024) uint16_t basis_ring[kStages][kBStepBytes / 2];   // 3 x 28 KiB
+    alignas(1024) uint16_t coeff_ring[kCStages][kAStageBytes / 2];  // 3 x 32 KiB
+    alignas(1024) uint16_t basis_ring[kBStages][kBStepBytes / 2];   // 3 x 28 KiB
     alignas(16) int64_t sums[kTileN][2];                             // second group's (lo, hi) per lookup
     TileMeta meta[kMetaBufs];
-    uint64_t full[kStages], empty[kStages];
+    uint64_t c_full[kCStages], c_empty[kCStages];
+    uint64_t b_full[kBStages], b_empty[kBStages];
     uint64_t meta_full[kMetaBufs], meta_empty[kMetaBufs];
     uint64_t acc_full, acc_empty;
     uint64_t drain;  // last commit of the MMA thread, waited on before dealloc
@@ -841,40 +837,12 @@ __device__ __forceinline__ int step_lead(const uint8_t* leads, int ks) {
     return ks == 0 ? 1 : min(static_cast<int>(__ldg(leads + ks)), kSlicesA);
 }
 
-// The K steps of a tile: their leads (four bits each) and which of them start
-// a ring stage (a bit each). A K step brings 9 - lead coefficient slices and
-// max(1, 8 - lead) basis slices; consecutive K steps share a stage while both
-// operands fit (8 and 7 slices), so that the many late K steps of a few MMAs
-// cost one barrier and one commit for two or three of them.
-struct TileSteps {
-    uint32_t leads, starts;
-    int tail;  // first K step from which every lead is kTailLead or more
-    __device__ __forceinline__ int lead(int ks) const { return static_cast<int>((leads >> (4 * ks)) & 15u); }
-    // K step ks is the last of its stage
-    __device__ __forceinline__ bool ends(int ks, int ksteps) const {
-        return ks + 1 == ksteps || ((starts >> (ks + 1)) & 1u) != 0;
-    }
-};
-__host__ __device__ __forceinline__ constexpr int coeff_slices(int lead) { return kSlicesA + 1 - lead; }
-__host__ __device__ __forceinline__ constexpr int basis_slices(int lead) { return lead < kSlicesA ? kSlicesA - lead : 1; }
-__device__ __forceinline__ TileSteps tile_steps(const uint8_t* leads, int ksteps) {
-    TileSteps s{0u, 0u, 0};
-#pragma unroll
-    for (int ks = 0; ks < kSubKSteps; ++ks)
-        s.leads |= static_cast<uint32_t>(ks < ksteps ? step_lead(leads, ks) : kSlicesA) << (4 * ks);
-    int c = 0, b = 0;
-#pragma unroll
-    for (int ks = 0; ks < kSubKSteps; ++ks) {
-        const int nc = coeff_slices(s.lead(ks)), nb = basis_slices(s.lead(ks));
-        if (ks == 0 || c + nc > kSlicesA || b + nb > kSlices) {
-            s.starts |= 1u << ks;
-            c = b = 0;
-        }
-        c += nc;
-        b += nb;
-        if (ks < ksteps && s.lead(ks) < kTailLead) s.tail = ks + 1;
-    }
-    return s;
+// The first K step from which every lead is kTailLead or more (ksteps when
+// none): from there the basis digits 1 and 2 are all the MMAs read.
+__device__ __forceinline__ int tail_kstep(const uint8_t* leads, int ksteps) {
+    int first = ksteps;
+    for (int ks = ksteps - 1; ks >= 1 && step_lead(leads, ks) >= kTailLead; --ks) first = ks;
+    return first;
 }
 
 // Tensor-memory layout of one pass of a tile: level lv (tau = lv + 2) takes
@@ -1138,9 +1106,13 @@ __global__ void __launch_bounds__(kAssemblyThreads, 1) split_assembly(const __gr
     const uint32_t tile_end = max(tile_begin, ranges[blockIdx.x + 1]);
 
     if (tid == 0) {
-        for (int i = 0; i < kStages; ++i) {
-            mbar_init(&sh.full[i], kProducerWarps * 32 + 1);  // the producers, and the copy's bytes
-            mbar_init(&sh.empty[i], 1);
+        for (int i = 0; i < kCStages; ++i) {
+            mbar_init(&sh.c_full[i], 1);
+            mbar_init(&sh.c_empty[i], 1);
+        }
+        for (int i = 0; i < kBStages; ++i) {
+            mbar_init(&sh.b_full[i], kProducerWarps * 32);
+            mbar_init(&sh.b_empty[i], 1);
         }
         for (int i = 0; i < kMetaBufs; ++i) {
             mbar_init(&sh.meta_full[i], kProducerWarps * 32);
@@ -1190,8 +1162,7 @@ __global__ void __launch_bounds__(kAssemblyThreads, 1) split_assembly(const __gr
             }
             mbar_arrive(&sh.meta_full[mb]);
             const int npass = pass_geom(rows, 0).npass;
-            const TileSteps steps = tile_steps(src.leads, src.ksteps);
-            const int ks_tail = steps.tail;
+            const int ks_tail = tail_kstep(src.leads, src.ksteps);
             const int64_t vfix = fixed_from_double(v, 62);
             const int b0 = src.kc * kSubK;
             bool ok = true;
@@ -1212,21 +1183,16 @@ __global__ void __launch_bounds__(kAssemblyThreads, 1) split_assembly(const __gr
 #pragma unroll
                     for (int j = 0; j < 8; ++j) ch[j].next(w8);
                 // one K step's digits (biased Q56 values of b = b0 + 16 ks + m:
-                // k = 0..7 hold the even m, k = 8..15 the odd m) into its stage
-                int slot = 0;  // the stage's next free slice
+                // k = 0..7 hold the even m, k = 8..15 the odd m) into a stage
                 auto emit = [&](int ks, const uint64_t (&ye)[8], const uint64_t (&yo)[8]) -> bool {
-                    const int st = static_cast<int>(b_cnt % kStages);
-                    if ((steps.starts >> ks) & 1u) {
-                        slot = 0;
-                        if (b_cnt >= kStages && !mbar_wait(&sh.empty[st], ((b_cnt / kStages) - 1) & 1)) {
-                            sh.error = 1;
-                            return false;
-                        }
+                    const int sb = static_cast<int>(b_cnt % kBStages);
+                    if (b_cnt >= kBStages && !mbar_wait(&sh.b_empty[sb], ((b_cnt / kBStages) - 1) & 1)) {
+                        sh.error = 1;
+                        return false;
                     }
                     // only the basis slices the K step's MMAs read: t' <= 8 - lead
-                    const int tmax = basis_slices(steps.lead(ks));
-                    uint16_t* base = sh.basis_ring[st] + slot * kTileN * kKStep + core_offset(l, 0);
-                    slot += tmax;
+                    const int tmax = max(1, kSlicesA - step_lead(src.leads, ks));
+                    uint16_t* base = sh.basis_ring[sb] + core_offset(l, 0);
 #pragma unroll
                     for (int t = 1; t <= kSlices; ++t) {
                         if (t > tmax) break;
@@ -1240,11 +1206,9 @@ __global__ void __launch_bounds__(kAssemblyThreads, 1) split_assembly(const __gr
                                      "r"(digit_pair(yo[4], yo[5], t)), "r"(digit_pair(yo[6], yo[7], t))
                                      : "memory");
                     }
-                    if (steps.ends(ks, src.ksteps)) {
-                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                        mbar_arrive(&sh.full[st]);
-                        ++b_cnt;
-                    }
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    mbar_arrive(&sh.b_full[sb]);
+                    ++b_cnt;
                     return true;
                 };
                 int ks = 0;
@@ -1468,47 +1432,46 @@ __global__ void __launch_bounds__(kAssemblyThreads, 1) split_assembly(const __gr
                 const TileSource src = tile_source<Chunked>(plan, tiles[tile].block);
                 const uint64_t rows = __ldg(reinterpret_cast<const unsigned long long*>(src.rows));
                 const int npass = pass_geom(rows, 0).npass;
-                const TileSteps steps = tile_steps(src.leads, src.ksteps);
                 for (int pass = 0; ok && pass < npass; ++pass) {
                     const PassGeom g = pass_geom(rows, pass);
-                    const int cols = max(g.cols, 16);  // the pass's rows: at least one 16-row group
-                    const uint32_t slice_bytes = static_cast<uint32_t>(cols) * kKStep * 2;
-                    for (int ks = 0; ks < src.ksteps; ++c_cnt) {
-                        const int st = static_cast<int>(c_cnt % kStages);
-                        if (c_cnt >= kStages && !mbar_wait(&sh.empty[st], ((c_cnt / kStages) - 1) & 1)) {
+                    for (int ks = 0; ks < src.ksteps; ++ks, ++c_cnt) {
+                        const int st = static_cast<int>(c_cnt % kCStages);
+                        if (c_cnt >= kCStages && !mbar_wait(&sh.c_empty[st], ((c_cnt / kCStages) - 1) & 1)) {
                             sh.error = 1;
                             ok = false;
                             break;
                         }
-                        // the stage's K steps, each one's slices lead..8 (the ones
-                        // before the lead are zero), one after the other
-                        int last = ks, slices = coeff_slices(steps.lead(ks));
-                        while (!steps.ends(last, src.ksteps)) slices += coeff_slices(steps.lead(++last));
-                        mbar_expect_tx(&sh.full[st], slice_bytes * static_cast<uint32_t>(slices));
-                        streamed += slice_bytes * static_cast<uint32_t>(slices);
-                        uint16_t* to = sh.coeff_ring[st] + g.row0 * kKStep;
-                        for (; ks <= last; ++ks) {
-                            const int lead = steps.lead(ks), n = coeff_slices(lead);
-                            const uint16_t* from = src.a + static_cast<int64_t>(ks) * (kAStageBytes / 2) +
-                                                   (lead - 1) * (kRows * kKStep) + g.row0 * kKStep;
-                            if (cols == kRows) {  // whole slices: one copy
-                                bulk_copy_g2s(to, from, kSliceBytes * static_cast<uint32_t>(n), &sh.full[st]);
-                            } else {  // each slice's rows row0 .. row0 + cols
-                                for (int t = 0; t < n; ++t)
-                                    bulk_copy_g2s(to + t * kRows * kKStep, from + t * kRows * kKStep, slice_bytes,
-                                                  &sh.full[st]);
+                        // slices lead..8 (the ones before the lead are zero), the
+                        // pass's rows (at least one 16-row group, so that every
+                        // stage completes by a copy)
+                        const int lead = step_lead(src.leads, ks);
+                        const uint16_t* from = src.a + static_cast<int64_t>(ks) * (kAStageBytes / 2);
+                        const int cols = max(g.cols, 16);
+                        if (g.row0 == 0 && cols == kRows) {  // whole slices: one copy
+                            const uint32_t offset = static_cast<uint32_t>(lead - 1) * (kRows * kKStep);
+                            const uint32_t bytes = kAStageBytes - offset * 2;
+                            mbar_expect_tx(&sh.c_full[st], bytes);
+                            bulk_copy_g2s(sh.coeff_ring[st] + offset, from + offset, bytes, &sh.c_full[st]);
+                            streamed += bytes;
+                        } else {  // each slice's rows row0 .. row0 + cols
+                            const uint32_t bytes = static_cast<uint32_t>(cols) * kKStep * 2;
+                            mbar_expect_tx(&sh.c_full[st], bytes * static_cast<uint32_t>(kSlicesA + 1 - lead));
+                            for (int t = lead; t <= kSlicesA; ++t) {
+                                const uint32_t offset = static_cast<uint32_t>(t - 1) * (kRows * kKStep) +
+                                                        static_cast<uint32_t>(g.row0) * kKStep;
+                                bulk_copy_g2s(sh.coeff_ring[st] + offset, from + offset, bytes, &sh.c_full[st]);
+                                streamed += bytes;
                             }
-                            to += n * kRows * kKStep;
                         }
                     }
                 }
             }
             if (counters) atomicAdd(counters + 1, streamed);
             // copies still in flight (only after an error) land before the CTA exits
-            for (uint32_t st = 0; st < static_cast<uint32_t>(kStages); ++st) {
+            for (uint32_t st = 0; st < static_cast<uint32_t>(kCStages); ++st) {
                 if (c_cnt <= st) continue;
-                const uint32_t last = c_cnt - 1 - (c_cnt - 1 - st) % kStages;
-                if (!mbar_wait(&sh.full[st], (last / kStages) & 1)) sh.error = 1;
+                const uint32_t last = c_cnt - 1 - (c_cnt - 1 - st) % kCStages;
+                if (!mbar_wait(&sh.c_full[st], (last / kCStages) & 1)) sh.error = 1;
             }
         }
     } else if (warp == kWarpMma) {
@@ -1522,10 +1485,9 @@ __global__ void __launch_bounds__(kAssemblyThreads, 1) split_assembly(const __gr
         for (uint32_t tile = tile_begin; ok && tile < tile_end && !__any_sync(0xffffffffu, failed(sh)); ++tile) {
             const TileSource src = tile_source<Chunked>(plan, tiles[tile].block);
             const uint64_t rows = __ldg(reinterpret_cast<const unsigned long long*>(src.rows));
-            // pairs with a coefficient slice before a K step's lead are zero, not issued
-            TileSteps steps = tile_steps(src.leads, src.ksteps);
-            steps.leads = __shfl_sync(0xffffffffu, steps.leads, 0);
-            steps.starts = __shfl_sync(0xffffffffu, steps.starts, 0);
+            // lane ks holds K step ks's lead (1 in a tile's first): pairs with
+            // a coefficient slice before it are zero, not issued
+            const int my_lead = lane < src.ksteps ? step_lead(src.leads, lane) : kSlicesA;
             const int ksteps = __shfl_sync(0xffffffffu, src.ksteps, 0);
             const int npass = __shfl_sync(0xffffffffu, pass_geom(rows, 0).npass, 0);
             for (int pass = 0; ok && pass < npass; ++pass, ++pass_cnt) {
@@ -1548,25 +1510,23 @@ __global__ void __launch_bounds__(kAssemblyThreads, 1) split_assembly(const __gr
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;");
-                uint64_t a0 = 0, b0 = 0;
-                for (int ks = 0; ks < ksteps; ++ks) {
-                    const int st = static_cast<int>(cnt % kStages);
-                    const int lead = steps.lead(ks);
-                    if ((steps.starts >> ks) & 1u) {
-                        const bool ready = mbar_wait(&sh.full[st], (cnt / kStages) & 1);
-                        if (!__all_sync(0xffffffffu, ready)) {
-                            ok = false;
-                            break;
-                        }
-                        asm volatile("tcgen05.fence::after_thread_sync;");
-                        a0 = smem_desc(smem_addr(sh.basis_ring[st]), 128, 256);
-                        b0 = smem_desc(smem_addr(sh.coeff_ring[st] + row0 * kKStep), 128, 256);
-                    }
-                    // b0 as if the stage began with slice 1: slice t is that
-                    // descriptor plus t - 1 slices' bytes / 16 (the sum stays in
-                    // the 14-bit address field: shared memory < 256 KiB)
-                    b0 -= static_cast<uint64_t>(lead - 1) * (kSliceBytes / 16);
+                for (int ks = 0; ks < ksteps; ++ks, ++cnt) {
+                    const int sc = static_cast<int>(cnt % kCStages);
+                    const int sb = static_cast<int>(cnt % kBStages);
+                    const int lead = __shfl_sync(0xffffffffu, my_lead, ks);
+                    // the stages' first slices; a slice further on is the same
+                    // descriptor plus its byte offset / 16 (the 14-bit address
+                    // field cannot carry: shared memory < 256 KiB)
+                    const uint64_t a0 = smem_desc(smem_addr(sh.basis_ring[sb]), 128, 256);
+                    const uint64_t b0 = smem_desc(smem_addr(sh.coeff_ring[sc] + row0 * kKStep), 128, 256);
                     const uint32_t accumulate = ks > 0 ? 1u : 0u;
+                    const bool ready = mbar_wait(&sh.c_full[sc], (cnt / kCStages) & 1) &&
+                                       mbar_wait(&sh.b_full[sb], (cnt / kBStages) & 1);
+                    if (!__all_sync(0xffffffffu, ready)) {
+                        ok = false;
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;");
                     switch (lead) {
                         case 1: issue_slice<1>(dcol, idesc, a0, b0, accumulate, issue); [[fallthrough]];
                         case 2: issue_slice<2>(dcol, idesc, a0, b0, accumulate, issue); [[fallthrough]];
@@ -1577,19 +1537,14 @@ __global__ void __launch_bounds__(kAssemblyThreads, 1) split_assembly(const __gr
                         case 7: issue_slice<7>(dcol, idesc, a0, b0, accumulate, issue); [[fallthrough]];
                         default: issue_slice<8>(dcol, idesc, a0, b0, accumulate, issue);
                     }
-                    a0 += static_cast<uint64_t>(basis_slices(lead)) * (kSliceBytes / 16);
-                    b0 += static_cast<uint64_t>(kSlicesA) * (kSliceBytes / 16);
-                    if (steps.ends(ks, ksteps)) {
-                        mma_commit(&sh.empty[st], issue);
-                        ++cnt;
-                    }
+                    mma_commit(&sh.c_empty[sc], issue);
+                    mma_commit(&sh.b_empty[sb], issue);
                 }
                 if (!ok) break;
                 mma_commit(&sh.acc_full, issue);
                 // the counter of issued tensor work (accumulator columns, each
                 // 2 x 128 x 16 flops), off the issue path: lane ks adds up K step ks
                 if (lane < ksteps) {
-                    const int my_lead = steps.lead(lane);
 #pragma unroll
                     for (int lv = 0; lv < kLevels; ++lv) {  // pairs (t, lv + 2 - t) with lead <= t; the eighth digit's
                         const int pairs = max(0, lv + 2 - my_lead) + (lv == kLevels - 1 ? 1 : 0);
