@@ -670,8 +670,16 @@ __global__ void __launch_bounds__(1024) split_scan(const SplitPlan plan, const u
     }
 }
 
-struct SplitTile {
-    uint32_t block, start, count, pad;
+// A tile: its sort key, its lookups in the sorted list, and what every role of
+// the assembly needs of its sub-block, so that a role learns all of it from
+// one 32-byte record that it loads a tile ahead.
+struct alignas(16) SplitTile {
+    uint32_t block, start, count;
+    int32_t exponent;  // the block's binary exponent
+    uint32_t leads;    // four bits per K step: its lead as the assembly uses it (step_lead)
+    uint32_t pad;
+    uint64_t rows;     // the sub-block's level rows
+    __device__ __forceinline__ int lead(int ks) const { return static_cast<int>((leads >> (4 * ks)) & 15u); }
 };
 
 // Scatter records into block order and emit the tile list.
@@ -837,12 +845,36 @@ __device__ __forceinline__ int step_lead(const uint8_t* leads, int ks) {
     return ks == 0 ? 1 : min(static_cast<int>(__ldg(leads + ks)), kSlicesA);
 }
 
+// The leads of a sub-block's K steps, four bits each.
+__device__ __forceinline__ uint32_t pack_leads(const uint8_t* leads, int ksteps) {
+    uint32_t packed = 0;
+    for (int ks = 0; ks < kSubKSteps; ++ks)
+        packed |= static_cast<uint32_t>(ks < ksteps ? step_lead(leads, ks) : kSlicesA) << (4 * ks);
+    return packed;
+}
+
 // The first K step from which every lead is kTailLead or more (ksteps when
 // none): from there the basis digits 1 and 2 are all the MMAs read.
-__device__ __forceinline__ int tail_kstep(const uint8_t* leads, int ksteps) {
+__device__ __forceinline__ int tail_kstep(const SplitTile& tile, int ksteps) {
     int first = ksteps;
-    for (int ks = ksteps - 1; ks >= 1 && step_lead(leads, ks) >= kTailLead; --ks) first = ks;
+    for (int ks = ksteps - 1; ks >= 1 && tile.lead(ks) >= kTailLead; --ks) first = ks;
     return first;
+}
+
+// Tile `index` of the list, or an empty one past the end of a CTA's range.
+__device__ __forceinline__ SplitTile load_tile(const SplitTile* __restrict__ tiles, uint32_t index, uint32_t end) {
+    SplitTile t{};
+    if (index < end) {
+        const uint4* q = reinterpret_cast<const uint4*>(tiles + index);
+        const uint4 a = __ldg(q), b = __ldg(q + 1);
+        t.block = a.x;
+        t.start = a.y;
+        t.count = a.z;
+        t.exponent = static_cast<int32_t>(a.w);
+        t.leads = b.x;
+        t.rows = (static_cast<uint64_t>(b.w) << 32) | b.z;
+    }
+    return t;
 }
 
 // Tensor-memory layout of one pass of a tile: level lv (tau = lv + 2) takes
@@ -1069,7 +1101,15 @@ __global__ void __launch_bounds__(256) split_tiles(const SplitPlan plan, const u
     const uint32_t cnt = counts[b];
     if (cnt == 0) return;
     uint32_t t = tile_offsets[b];
-    for (uint32_t s = 0; s < cnt; s += kTileN, ++t) tiles[t] = SplitTile{b, offsets[b] + s, min(kTileN * 1u, cnt - s), 0};
+    {
+        const TileSource src = plan.nrb * plan.nkc > 1 ? tile_source<true>(plan, b) : tile_source<false>(plan, b);
+        SplitTile tile{b, offsets[b], 0, __ldg(src.exponent), pack_leads(src.leads, src.ksteps), 0,
+                       __ldg(reinterpret_cast<const unsigned long long*>(src.rows))};
+        for (uint32_t s = 0; s < cnt; s += kTileN, ++t, tile.start += kTileN) {
+            tile.count = min(kTileN * 1u, cnt - s);
+            tiles[t] = tile;
+        }
+    }
     const uint32_t m = (cnt + kTileN - 1) / kTileN;
     const unsigned long long wq = key_cost(plan, b) + mean;
     const unsigned long long p0 = cost_prefix[b] + mean * tile_offsets[b], p1 = p0 + m * wq;
@@ -1139,30 +1179,34 @@ __global__ void __launch_bounds__(kAssemblyThreads, 1) split_assembly(const __gr
         // ---------------------------------------------- basis producers --
         const int l = tid;  // the lookup of this thread
         uint32_t b_cnt = 0, tile_cnt = 0;
+        // the tile record two ahead and the lookup one ahead are loaded before
+        // the tile's work, so that no tile begins by waiting for memory
+        auto load_lookup = [&](const SplitTile& t) {
+            return static_cast<uint32_t>(l) < t.count ? sorted[t.start + l] : SortedLookup{0.0, 0.0, ~uint64_t{0}, 0};
+        };
+        SplitTile tl = load_tile(tiles, tile_begin, tile_end), tl_next = load_tile(tiles, tile_begin + 1, tile_end);
+        SortedLookup look = load_lookup(tl);
         for (uint32_t tile = tile_begin; tile < tile_end && !failed(sh); ++tile, ++tile_cnt) {
-            const SplitTile tl = tiles[tile];
+            const SplitTile tl_after = load_tile(tiles, tile + 2, tile_end);
+            const SortedLookup look_next = load_lookup(tl_next);
             const int mb = static_cast<int>(tile_cnt % kMetaBufs);
             if (tile_cnt >= kMetaBufs && !mbar_wait(&sh.meta_empty[mb], ((tile_cnt / kMetaBufs) - 1) & 1)) {
                 sh.error = 1;
                 break;
             }
             const TileSource src = tile_source<Chunked>(plan, tl.block);
-            const uint64_t rows = __ldg(reinterpret_cast<const unsigned long long*>(src.rows));
-            const bool live = static_cast<uint32_t>(l) < tl.count;
-            SortedLookup look{0.0, 0.0, ~uint64_t{0}, 0};
-            if (live) look = sorted[tl.start + l];
             const double v = look.v;
             sh.meta[mb].u[l] = look.u;
             sh.meta[mb].info[l] = look.info;
             if (l == 0) {
                 sh.meta[mb].count = tl.count;
-                sh.meta[mb].exponent = __ldg(src.exponent);
+                sh.meta[mb].exponent = tl.exponent;
                 sh.meta[mb].sub = src.sub;
-                sh.meta[mb].rows = rows;
+                sh.meta[mb].rows = tl.rows;
             }
             mbar_arrive(&sh.meta_full[mb]);
-            const int npass = pass_geom(rows, 0).npass;
-            const int ks_tail = tail_kstep(src.leads, src.ksteps);
+            const int npass = pass_geom(tl.rows, 0).npass;
+            const int ks_tail = tail_kstep(tl, src.ksteps);
             const int64_t vfix = fixed_from_double(v, 62);
             const int b0 = src.kc * kSubK;
             bool ok = true;
@@ -1191,7 +1235,7 @@ __global__ void __launch_bounds__(kAssemblyThreads, 1) split_assembly(const __gr
                         return false;
                     }
                     // only the basis slices the K step's MMAs read: t' <= 8 - lead
-                    const int tmax = max(1, kSlicesA - step_lead(src.leads, ks));
+                    const int tmax = max(1, kSlicesA - tl.lead(ks));
                     uint16_t* base = sh.basis_ring[sb] + core_offset(l, 0);
 #pragma unroll
                     for (int t = 1; t <= kSlices; ++t) {
@@ -1261,6 +1305,9 @@ __global__ void __launch_bounds__(kAssemblyThreads, 1) split_assembly(const __gr
                 }
             }
             if (!ok) break;
+            tl = tl_next;
+            tl_next = tl_after;
+            look = look_next;
         }
     } else if (warp < kProducerWarps + kEpilogueWarps) {
         // ------------------------------------------------------ epilogue --
@@ -1331,7 +1378,7 @@ __global__ void __launch_bounds__(kAssemblyThreads, 1) split_assembly(const __gr
                         for (int q = 0; q < 8; ++q) {
                             const float f7 = has7 ? __uint_as_float(v7[q]) * 0.5f : 0.0f;
                             wfix[q] = __float2int_rn(fmaf(__uint_as_float(v8[q]), 0.001953125f, f7));
-                            wfix[q] += static_cast<int64_t>(__float2int_rn(__uint_as_float(v6[q]))) << 7;
+                            wfix[q] += static_cast<int64_t>(__float2int_rn(__uint_as_float(v6[q]))) * 128;
                         }
                     }
                     if (g.n[kLevels - 4] > c0) {  // levels 2..5
@@ -1343,10 +1390,17 @@ __global__ void __launch_bounds__(kAssemblyThreads, 1) split_assembly(const __gr
 #pragma unroll
                         for (int lv = 0; lv < kLevels - 3; ++lv) {
                             if (g.n[lv] <= c0) continue;
-                            const int shift = 39 - 8 * lv;  // 2^(55 - 8 tau), tau = lv + 2
+                            // times 2^(55 - 8 tau), tau = lv + 2: one multiply-add with a
+                            // factor up to 2^30 (level 3's other power of two in its FP32
+                            // value, exactly), level 2 in the upper word
+                            const int shift = 39 - 8 * lv;
 #pragma unroll
-                            for (int q = 0; q < 8; ++q)
-                                wfix[q] += static_cast<int64_t>(__float2int_rn(__uint_as_float(v[lv][q]))) << shift;
+                            for (int q = 0; q < 8; ++q) {
+                                const float level = __uint_as_float(v[lv][q]);
+                                if (lv == 0) wfix[q] += static_cast<int64_t>(__float2int_rn(level) * 128) * (int64_t{1} << 32);
+                                else if (lv == 1) wfix[q] += static_cast<int64_t>(__float2int_rn(level * 2.0f)) * (1 << 30);
+                                else wfix[q] += static_cast<int64_t>(__float2int_rn(level)) * (1 << shift);
+                            }
                         }
                     }
                     // sum_a T_a(u) W_a: products rounded to 2^-55, summed exactly
@@ -1356,9 +1410,9 @@ __global__ void __launch_bounds__(kAssemblyThreads, 1) split_assembly(const __gr
                         // |wfix| < 2^62, |tf| <= 2^62
                         const int64_t prod =
                             mul_shift<62>(signed_halves(wfix[q]), signed_halves(tf), int64_t{1} << 61);
-                        const uint64_t nlo = slo + static_cast<uint64_t>(prod);
-                        shi += (prod < 0 ? -1 : 0) + (nlo < slo ? 1 : 0);
-                        slo = nlo;
+                        asm("add.cc.u64 %0, %0, %2;\n addc.u64 %1, %1, %3;"
+                            : "+l"(slo), "+l"(shi)
+                            : "l"(prod), "l"(prod >> 63));
                     }
                 }
                 if (c_head < g.cols) {
@@ -1428,9 +1482,11 @@ __global__ void __launch_bounds__(kAssemblyThreads, 1) split_assembly(const __gr
             uint32_t c_cnt = 0;
             unsigned long long streamed = 0;
             bool ok = true;
+            SplitTile tl = load_tile(tiles, tile_begin, tile_end);
             for (uint32_t tile = tile_begin; ok && tile < tile_end && !failed(sh); ++tile) {
-                const TileSource src = tile_source<Chunked>(plan, tiles[tile].block);
-                const uint64_t rows = __ldg(reinterpret_cast<const unsigned long long*>(src.rows));
+                const SplitTile tl_next = load_tile(tiles, tile + 1, tile_end);
+                const TileSource src = tile_source<Chunked>(plan, tl.block);
+                const uint64_t rows = tl.rows;
                 const int npass = pass_geom(rows, 0).npass;
                 for (int pass = 0; ok && pass < npass; ++pass) {
                     const PassGeom g = pass_geom(rows, pass);
@@ -1444,7 +1500,7 @@ __global__ void __launch_bounds__(kAssemblyThreads, 1) split_assembly(const __gr
                         // slices lead..8 (the ones before the lead are zero), the
                         // pass's rows (at least one 16-row group, so that every
                         // stage completes by a copy)
-                        const int lead = step_lead(src.leads, ks);
+                        const int lead = tl.lead(ks);
                         const uint16_t* from = src.a + static_cast<int64_t>(ks) * (kAStageBytes / 2);
                         const int cols = max(g.cols, 16);
                         if (g.row0 == 0 && cols == kRows) {  // whole slices: one copy
@@ -1465,6 +1521,7 @@ __global__ void __launch_bounds__(kAssemblyThreads, 1) split_assembly(const __gr
                         }
                     }
                 }
+                tl = tl_next;
             }
             if (counters) atomicAdd(counters + 1, streamed);
             // copies still in flight (only after an error) land before the CTA exits
@@ -1482,12 +1539,14 @@ __global__ void __launch_bounds__(kAssemblyThreads, 1) split_assembly(const __gr
         uint32_t cnt = 0, pass_cnt = 0;  // K steps (the rings' position), passes
         unsigned long long mmas = 0;
         bool ok = true;
+        SplitTile tl = load_tile(tiles, tile_begin, tile_end);
         for (uint32_t tile = tile_begin; ok && tile < tile_end && !__any_sync(0xffffffffu, failed(sh)); ++tile) {
-            const TileSource src = tile_source<Chunked>(plan, tiles[tile].block);
-            const uint64_t rows = __ldg(reinterpret_cast<const unsigned long long*>(src.rows));
-            // lane ks holds K step ks's lead (1 in a tile's first): pairs with
-            // a coefficient slice before it are zero, not issued
-            const int my_lead = lane < src.ksteps ? step_lead(src.leads, lane) : kSlicesA;
+            const SplitTile tl_next = load_tile(tiles, tile + 1, tile_end);
+            const TileSource src = tile_source<Chunked>(plan, tl.block);
+            const uint64_t rows = tl.rows;
+            // pairs with a coefficient slice before a K step's lead (1 in a
+            // tile's first K step) are zero, not issued
+            const int my_lead = lane < src.ksteps ? tl.lead(lane) : kSlicesA;
             const int ksteps = __shfl_sync(0xffffffffu, src.ksteps, 0);
             const int npass = __shfl_sync(0xffffffffu, pass_geom(rows, 0).npass, 0);
             for (int pass = 0; ok && pass < npass; ++pass, ++pass_cnt) {
@@ -1552,6 +1611,7 @@ __global__ void __launch_bounds__(kAssemblyThreads, 1) split_assembly(const __gr
                     }
                 }
             }
+            tl = tl_next;
         }
         if (!ok) sh.error = 1;
         if (counters) atomicAdd(counters, mmas);
