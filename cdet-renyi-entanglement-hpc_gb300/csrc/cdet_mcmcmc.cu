@@ -1,5 +1,4 @@
-// Device-resident MCMCMC chains: one thread per chain runs run_mcmcmc_step
-// (mcmcmc_sampler.h:524-577) on the all-subset integrand values of its
+// Device-resident MCMCMC chains: run_mcmcmc_step (mcmcmc_sampler.h:524-577) on the all-subset integrand values of its
 // envelope, so a batch of chains advances one step per launch pair
 // (integrand, step) with no host round trip. The seed kernel is the uniform
 // one (mcmcmc_seed.h:41-61) or the factorized histogram (:71-229), whose
@@ -25,6 +24,44 @@ namespace {
 constexpr int kMtN = 312;
 constexpr int kMtM = 156;
 
+// One word of the state transition, from words i, i + 1 and i + 156.
+__device__ __forceinline__ uint64_t mt_twist(uint64_t word, uint64_t next, uint64_t far) {
+    const uint64_t x = (word & 0xFFFFFFFF80000000ull) | (next & 0x7FFFFFFFull);
+    return far ^ (x >> 1) ^ ((x & 1ull) ? 0xB5026F5AA96619E9ull : 0ull);
+}
+__device__ __forceinline__ uint64_t mt_temper(uint64_t y) {
+    y ^= (y >> 29) & 0x5555555555555555ull;
+    y ^= (y << 17) & 0x71D67FFFEDA60000ull;
+    y ^= (y << 37) & 0xFFF7EEE000000000ull;
+    return y ^ (y >> 43);
+}
+
+// std::generate_canonical<double, 53> of one word as libstdc++ computes it.
+// The division by 2^64 is exact, and so is the product with 2^-64.
+__device__ __forceinline__ double mt_canonical(uint64_t word) {
+    const double r = dmul(__ull2double_rn(word), 0x1p-64);
+    return r >= 1.0 ? __longlong_as_double(0x3FEFFFFFFFFFFFFFll) : r;
+}
+
+// std::uniform_int_distribution<int>(0, n - 1)
+template <class Generator>
+__device__ __forceinline__ int mt_uniform_int(Generator& g, int n) {
+    const uint64_t range = static_cast<uint64_t>(n);
+    uint64_t x = g.next();
+    uint64_t low = x * range;
+    uint64_t high = __umul64hi(x, range);
+    if (low < range) {
+        const uint64_t threshold = (0ull - range) % range;
+        while (low < threshold) {
+            x = g.next();
+            low = x * range;
+            high = __umul64hi(x, range);
+        }
+    }
+    return static_cast<int>(high);
+}
+
+// A chain's generator on one thread.
 struct Mt64 {
     uint64_t* words;  // word i of this chain at words[i * stride]
     int64_t stride;
@@ -34,42 +71,76 @@ struct Mt64 {
 
     __device__ uint64_t next() const {
         if (*index >= kMtN) {
-            const uint64_t upper = 0xFFFFFFFF80000000ull, lower = 0x7FFFFFFFull, matrix = 0xB5026F5AA96619E9ull;
-            for (int i = 0; i < kMtN; ++i) {
-                const uint64_t x = (at(i) & upper) | (at(i + 1 < kMtN ? i + 1 : 0) & lower);
-                at(i) = at(i + kMtM < kMtN ? i + kMtM : i + kMtM - kMtN) ^ (x >> 1) ^ ((x & 1ull) ? matrix : 0ull);
-            }
+            for (int i = 0; i < kMtN; ++i)
+                at(i) = mt_twist(at(i), at(i + 1 < kMtN ? i + 1 : 0),
+                                 at(i + kMtM < kMtN ? i + kMtM : i + kMtM - kMtN));
             *index = 0;
         }
-        uint64_t y = at((*index)++);
-        y ^= (y >> 29) & 0x5555555555555555ull;
-        y ^= (y << 17) & 0x71D67FFFEDA60000ull;
-        y ^= (y << 37) & 0xFFF7EEE000000000ull;
-        y ^= y >> 43;
-        return y;
+        return mt_temper(at((*index)++));
     }
+    __device__ double canonical() const { return mt_canonical(next()); }
+};
 
-    // std::generate_canonical<double, 53> as libstdc++ computes it
-    __device__ double canonical() const {
-        const double r = ddiv(__ull2double_rn(next()), 18446744073709551616.0);
-        return r >= 1.0 ? __longlong_as_double(0x3FEFFFFFFFFFFFFFll) : r;
-    }
+// A chain's generator on one warp, every lane calling together: lane k holds
+// word base + k of the state, tempered, so that a draw is a shuffle, and the
+// state transition runs on all lanes (32 words at a time; a word's new value
+// needs only its neighbour's old one, which the next 32 have not replaced
+// yet). The same words in the same order as Mt64's.
+struct WarpMt64 {
+    uint64_t* words;
+    int64_t stride;
+    int lane;
+    int32_t index;
+    int32_t base;
+    uint64_t buffer;
 
-    // std::uniform_int_distribution<int>(0, n - 1)
-    __device__ int uniform_int(int n) const {
-        const uint64_t range = static_cast<uint64_t>(n);
-        uint64_t x = next();
-        uint64_t low = x * range;
-        uint64_t high = __umul64hi(x, range);
-        if (low < range) {
-            const uint64_t threshold = (0ull - range) % range;
-            while (low < threshold) {
-                x = next();
-                low = x * range;
-                high = __umul64hi(x, range);
+    __device__ WarpMt64(uint64_t* w, int64_t s, int32_t i, int l)
+        : words(w), stride(s), lane(l), index(i), base(-kWarp), buffer(0) {}
+    __device__ __forceinline__ uint64_t& at(int i) const { return words[static_cast<int64_t>(i) * stride]; }
+
+    __device__ void transition() {
+        for (int part = 0; part < 2; ++part) {  // words 0..155, then 156..311 from the new 0..155
+            for (int i0 = part * kMtM; i0 < (part + 1) * kMtM; i0 += kWarp) {
+                const int i = i0 + lane;
+                const bool in = i < (part + 1) * kMtM;
+                uint64_t v = 0;
+                if (in) v = mt_twist(at(i), at(i + 1 < kMtN ? i + 1 : 0), at(part == 0 ? i + kMtM : i - kMtM));
+                __syncwarp();
+                if (in) at(i) = v;
+                __syncwarp();
             }
         }
-        return static_cast<int>(high);
+    }
+    // The buffer holds words index .. index + count - 1 (count <= 32, index + count <= 312).
+    __device__ __forceinline__ void fill(int count) {
+        if (index >= base && index + count <= base + kWarp) return;
+        base = index;
+        buffer = base + lane < kMtN ? mt_temper(at(base + lane)) : 0;
+    }
+    __device__ uint64_t next() {
+        if (index >= kMtN) {
+            transition();
+            index = 0;
+            base = -kWarp;
+        }
+        fill(1);
+        return __shfl_sync(0xffffffffu, buffer, index++ - base);
+    }
+    __device__ double canonical() { return mt_canonical(next()); }
+    // Four canonical draws in order, the k-th on every lane l with l & 3 == k.
+    __device__ double canonical4() {
+        uint64_t word = 0;
+        if (index + 4 <= kMtN) {
+            fill(4);
+            word = __shfl_sync(0xffffffffu, buffer, index - base + (lane & 3));
+            index += 4;
+        } else {
+            for (int k = 0; k < 4; ++k) {
+                const uint64_t w = next();
+                if ((lane & 3) == k) word = w;
+            }
+        }
+        return mt_canonical(word);
     }
 };
 
@@ -84,7 +155,8 @@ __device__ __forceinline__ int unit_index(double value, int extent) {
 // sample_from_row (mcmcmc_seed.h:205-218): std::lower_bound (the binary search
 // for the first entry not below the draw) in one CDF row; past the end, the
 // last column
-__device__ int sample_row(const double* __restrict__ cdf, int columns, int row, const Mt64& g) {
+template <class Generator>
+__device__ int sample_row(const double* __restrict__ cdf, int columns, int row, Generator& g) {
     const double threshold = g.canonical();
     const double* b = cdf + static_cast<int64_t>(row) * columns;
     int first = 0, len = columns;
@@ -115,7 +187,8 @@ __device__ double hist_density(const McmcmcStepArgs& a, const double* child, con
 
 // sample_child_from_parent (mcmcmc_seed.h:106-128): three row draws, then the
 // four in-cell offsets in vertex order
-__device__ void hist_child(const McmcmcStepArgs& a, const Mt64& g, const double* parent, double* child) {
+template <class Generator>
+__device__ void hist_child(const McmcmcStepArgs& a, Generator& g, const double* parent, double (&child)[4]) {
     const int child_tau = sample_row(a.tau_cdf, a.tau_bins, unit_index(parent[0], a.tau_bins), g);
     const int parent_site = unit_index(parent[1], a.n1) * a.n2 + unit_index(parent[2], a.n2);
     const int child_site = sample_row(a.space_cdf, a.n1 * a.n2, parent_site, g);
@@ -194,7 +267,7 @@ __global__ void mcmcmc_init(int64_t chains, int envelope, const uint64_t* __rest
                             int32_t* mt_index, double* vertices) {
     const int64_t c = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (c >= chains) return;
-    const Mt64 g{mt + c, chains, mt_index + c};
+    Mt64 g{mt + c, chains, mt_index + c};
     uint64_t x = seeds[c];
     g.at(0) = x;
     for (int i = 1; i < kMtN; ++i) {
@@ -214,7 +287,7 @@ __device__ void finish_step(const McmcmcStepArgs& a, int64_t c, int64_t row, con
     const uint64_t subsets = uint64_t{1} << env;
     const double* values = a.values + c * static_cast<int64_t>(subsets);
     const double* lam = a.lambdas + c * (env + 1);
-    const Mt64 g{a.mt + c, a.chains, a.mt_index + c};
+    Mt64 g{a.mt + c, a.chains, a.mt_index + c};
     const double* v = a.vertices + c * env * 4;
     const uint64_t full = subsets - 1;
     // flux = lambda * value * conditional probability of the complement
@@ -273,9 +346,11 @@ __device__ void finish_step(const McmcmcStepArgs& a, int64_t c, int64_t row, con
             ++size;
         }
     while (size < env) {
-        const int parent = g.uniform_int(size);
+        const int parent = mt_uniform_int(g, size);
         if constexpr (Hist) {
-            hist_child(a, g, nv + 4 * parent, nv + 4 * size);
+            double child[4];
+            hist_child(a, g, nv + 4 * parent, child);
+            for (int k = 0; k < 4; ++k) nv[4 * size + k] = child[k];
         } else {
             (void)parent;
             for (int k = 0; k < 4; ++k) nv[4 * size + k] = g.canonical();
@@ -306,122 +381,185 @@ __global__ void __launch_bounds__(128) mcmcmc_step(const __grid_constant__ Mcmcm
     finish_step<Hist>(a, c, row, Hist ? a.cprob + c * (int64_t{1} << a.envelope) : nullptr);
 }
 
-// The serial part of the step with one warp per chain (small batches): the
-// fluxes elementwise on all lanes, the local normalisation and the weighted
-// draw on lane 0 (both are running sums in mask order), each order's signal
-// sum on its own lane (its masks in increasing order, as the reference adds
-// them), then the next vertices on lane 0. Same values as finish_step.
-template <bool Hist>
-__device__ void finish_step_warp(const McmcmcStepArgs& a, int64_t c, int64_t row, const double* cprob, double* flux,
-                                 int lane) {
-    const int env = a.envelope;
-    const uint32_t subsets = 1u << env, full = subsets - 1;
-    const double* values = a.values + c * static_cast<int64_t>(subsets);
-    const double* lam = a.lambdas + c * (env + 1);
-    for (uint32_t mask = lane; mask < subsets; mask += 32) {
-        const int o = __popc(mask);
-        flux[mask] = (mask == 0 || o < a.order_min || o > a.order_max)
-                         ? 0.0
-                         : dmul(dmul(lam[o], values[mask]), Hist ? cprob[full ^ mask] : 1.0);
-    }
-    __syncwarp();
-    double norm = 0.0;
-    if (lane == 0)
-        for (uint32_t mask = 1; mask < subsets; ++mask) {
-            const int o = __popc(mask);
-            if (o < a.order_min || o > a.order_max) continue;
-            norm = dadd(norm, dmul(fabs(flux[mask]), a.inv_binom[o]));
-        }
-    norm = __shfl_sync(0xffffffffu, norm, 0);
-    if (!(norm > 0.0) || !isfinite(norm)) {
-        if (lane == 0) a.error[c] = 2;  // "MCMCMC local normalization is zero or non-finite"
-        return;
-    }
-    if (a.signal_out && lane <= env) {
-        double sig = 0.0;
-        if (lane >= 1 && lane >= a.order_min && lane <= a.order_max) {
-            const uint32_t masks = kBinomial.c[env][lane];
-            uint32_t m = (1u << lane) - 1u;
-            for (uint32_t r = 0; r < masks; ++r, m = next_same_popcount(m))
-                sig = dadd(sig, dmul(ddiv(flux[m], norm), a.inv_binom[lane]));
-        }
-        a.signal_out[(row * a.chains + c) * (env + 1) + lane] = sig;
-    }
-    if (lane != 0) return;
-    const Mt64 g{a.mt + c, a.chains, a.mt_index + c};
-    const double threshold = dadd(dmul(g.canonical(), dsub(norm, 0.0)), 0.0);
-    double cumulative = 0.0;
-    uint64_t chosen = 0, last_positive = 0;
-    bool found = false;
-    for (uint32_t mask = 1; mask < subsets && !found; ++mask) {
-        const int o = __popc(mask);
-        if (o < a.order_min || o > a.order_max) continue;
-        const double w = dmul(fabs(flux[mask]), a.inv_binom[o]);
-        if (!(w > 0.0)) continue;
-        if (isfinite(w)) last_positive = mask;
-        cumulative = dadd(cumulative, w);
-        if (cumulative > threshold) {
-            chosen = mask;
-            found = true;
-        }
-    }
-    if (!found) chosen = last_positive;
-    const double* v = a.vertices + c * env * 4;
-    double* nv = a.next_vertices + c * env * 4;
-    int size = 0;
-    for (int i = 0; i < env; ++i)
-        if (chosen & (uint64_t{1} << i)) {
-            for (int k = 0; k < 4; ++k) nv[4 * size + k] = v[4 * i + k];
-            ++size;
-        }
-    while (size < env) {
-        const int parent = g.uniform_int(size);
-        if constexpr (Hist) {
-            hist_child(a, g, nv + 4 * parent, nv + 4 * size);
-        } else {
-            (void)parent;
-            for (int k = 0; k < 4; ++k) nv[4 * size + k] = g.canonical();
-        }
-        ++size;
-    }
-    if (a.chosen_out) a.chosen_out[row * a.chains + c] = chosen;
-    if (a.retained_out) a.retained_out[c] = chosen;
-    if (a.norm_out) a.norm_out[row * a.chains + c] = norm;
-    if (a.warmup) ++a.counts[c * (env + 1) + __popcll(chosen)];
+// The step with one warp per chain (up to kStepWarpMaxChains chains), one to
+// eight chains per block. Everything elementwise runs on the chain's lanes:
+// the fluxes and selection weights, the signal terms, the search for the drawn
+// mask, the generator. What the reference adds up in mask order stays a serial
+// sum, but shares its FP64 instructions: the local normalisations of the
+// block's chains run on neighbouring lanes of one warp, and so do their
+// per-order signal sums. The weighted draw needs no second sum: its running
+// weight is the normalisation's (masks of weight zero change neither), so the
+// prefixes are kept and the first one above the threshold is found in
+// parallel. Same values as finish_step.
+//
+// Bound: the 2^envelope dependent FP64 additions of the normalisation.
+// Measured at envelope 9 against lane 0 doing all serial work with its own
+// divisions and global generator state: 128 chains 215 -> 50 us, 2,048 chains 588 -> 74 us (one
+// thread per chain before).
+constexpr int kStepWarpMaxEnvelope = 12;
+constexpr int64_t kStepWarpMaxChains = 16384;
+constexpr int kStepMaxChainsPerBlock = 8;
+
+// Doubles of shared memory per chain: fluxes and weight prefixes (each padded
+// by one, so that neighbouring chains' entries fall into other banks), for the
+// histogram seed kernel the conditional probabilities, densities and row sums.
+__host__ __device__ inline size_t step_doubles(int env, bool hist) {
+    const size_t subsets = size_t{1} << env;
+    return 2 * (subsets + 1) + (hist ? subsets + static_cast<size_t>(env) * (env + 1) : 0);
 }
 
-// The whole step for a small batch: one warp (and block) per chain, its
-// fluxes, and for the histogram seed kernel its densities and conditional
-// probabilities, in shared memory.
-constexpr int kStepWarpMaxEnvelope = 12;
-constexpr int64_t kStepWarpMaxChains = 2048;
 template <bool Hist>
-__global__ void __launch_bounds__(32) mcmcmc_step_warp(const __grid_constant__ McmcmcStepArgs a) {
+__global__ void __launch_bounds__(kStepMaxChainsPerBlock * kWarp) mcmcmc_step_warp(const __grid_constant__ McmcmcStepArgs a) {
     extern __shared__ double step_smem[];
-    const int lane = threadIdx.x;
-    const int64_t c = blockIdx.x;
+    __shared__ double s_norm[kStepMaxChainsPerBlock];
+    __shared__ int s_state[kStepMaxChainsPerBlock];  // 1: the chain makes a step; 2: its normalisation is good
+    const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp, per_block = blockDim.x / kWarp;
+    const int64_t c = static_cast<int64_t>(blockIdx.x) * per_block + warp;
     const int env = a.envelope;
-    const uint32_t subsets = 1u << env;
-    double* flux = step_smem;
-    double* prob = flux + subsets;
-    double* sd = prob + subsets;
-    double* cd0 = sd + env * env;
+    const uint32_t subsets = 1u << env, full = subsets - 1;
+    const size_t per_chain = step_doubles(env, Hist);
+    double* flux = step_smem + static_cast<size_t>(warp) * per_chain;
+    double* prefix = flux + subsets + 1;
+    double* prob = prefix + subsets + 1;
     const int64_t row = a.ring_row ? *a.ring_row : 0;
-    if (lane == 0 && a.chosen_out) a.chosen_out[row * a.chains + c] = 0;  // 0: no step (a failed chain)
-    if (lane == 0 && a.retained_out) a.retained_out[c] = 0;
-    if (a.error[c]) return;  // the same value on every lane
-    if (a.integrand_status[c] & kStatusNonFinite) {
-        if (lane == 0) a.error[c] = 1;  // "Error (all-subset integrand): Value is not finite"
-        return;
+    bool active = c < a.chains;
+    if (active) {
+        if (lane == 0 && a.chosen_out) a.chosen_out[row * a.chains + c] = 0;  // 0: no step (a failed chain)
+        if (lane == 0 && a.retained_out) a.retained_out[c] = 0;
+        if (a.error[c]) {  // the same value on every lane
+            active = false;
+        } else if (a.integrand_status[c] & kStatusNonFinite) {
+            __syncwarp();
+            if (lane == 0) a.error[c] = 1;  // "Error (all-subset integrand): Value is not finite"
+            active = false;
+        }
     }
     if constexpr (Hist) {
-        if (!conditional_probabilities_warp(a, a.vertices + c * env * 4, env, prob, sd, cd0, lane)) {
-            if (lane == 0) a.error[c] = 3;  // "MCMCMC seed density is negative or non-finite"
-            return;
+        if (active) {
+            if (!conditional_probabilities_warp(a, a.vertices + c * env * 4, env, prob, prob + subsets,
+                                                prob + subsets + env * env, lane)) {
+                if (lane == 0) a.error[c] = 3;  // "MCMCMC seed density is negative or non-finite"
+                active = false;
+            }
+            __syncwarp();
         }
-        __syncwarp();
     }
-    finish_step_warp<Hist>(a, c, row, prob, flux, lane);
+    if (active) {
+        // fluxes and selection weights (:411-430, :540-560); masks outside the orders weigh nothing
+        const double* values = a.values + c * static_cast<int64_t>(subsets);
+        const double* lam = a.lambdas + c * (env + 1);
+        for (uint32_t mask = lane; mask < subsets; mask += kWarp) {
+            const int o = __popc(mask);
+            double f = 0.0, weight = 0.0;
+            if (mask != 0 && o >= a.order_min && o <= a.order_max) {
+                f = dmul(dmul(lam[o], values[mask]), Hist ? prob[full ^ mask] : 1.0);
+                weight = dmul(fabs(f), a.inv_binom[o]);
+            }
+            flux[mask] = f;
+            prefix[mask] = weight;
+        }
+    }
+    if (lane == 0) s_state[warp] = active ? 1 : 0;
+    __syncthreads();
+    // the local normalisations: lane k adds up chain k's weights in mask order
+    if (warp == 0 && lane < per_block && s_state[lane]) {
+        double* w = step_smem + static_cast<size_t>(lane) * per_chain + subsets + 1;
+        double norm = 0.0;
+        for (uint32_t m0 = 0; m0 < subsets; m0 += 8) {  // (mask 0 weighs nothing; subsets >= 8 or the tail below)
+            double x[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) x[k] = m0 + k < subsets ? w[m0 + k] : 0.0;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                norm = dadd(norm, x[k]);
+                x[k] = norm;
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (m0 + k < subsets) w[m0 + k] = x[k];
+        }
+        s_norm[lane] = norm;
+        if (norm > 0.0 && isfinite(norm)) s_state[lane] = 2;
+        else a.error[static_cast<int64_t>(blockIdx.x) * per_block + lane] = 2;  // "MCMCMC local normalization is zero or non-finite"
+    }
+    __syncthreads();
+    if (s_state[warp] == 2) {
+        const double norm = s_norm[warp];
+        WarpMt64 g(a.mt + c, a.chains, a.mt_index[c], lane);
+        // sample_weighted_candidate_mask (:225-250): the first mask whose running weight exceeds the
+        // threshold; failing that, the last one of positive finite weight
+        const double threshold = dadd(dmul(g.canonical(), dsub(norm, 0.0)), 0.0);
+        uint32_t chosen = 0, last_positive = 0;
+        bool found = false;
+        for (uint32_t m0 = 0; m0 < subsets && !found; m0 += kWarp) {
+            const uint32_t mask = m0 + lane;
+            const uint32_t hit = __ballot_sync(0xffffffffu, mask > 0 && mask < subsets && prefix[mask] > threshold);
+            if (hit) {
+                chosen = m0 + __ffs(hit) - 1;
+                found = true;
+            }
+        }
+        if (!found) {
+            for (uint32_t m0 = 0; m0 < subsets; m0 += kWarp) {
+                const uint32_t mask = m0 + lane;
+                const int o = __popc(mask);
+                bool positive = false;
+                if (mask > 0 && mask < subsets && o >= a.order_min && o <= a.order_max) {
+                    const double weight = dmul(fabs(flux[mask]), a.inv_binom[o]);
+                    positive = weight > 0.0 && isfinite(weight);
+                }
+                const uint32_t hit = __ballot_sync(0xffffffffu, positive);
+                if (hit) last_positive = m0 + 31 - __clz(static_cast<int>(hit));
+            }
+            chosen = last_positive;
+        }
+        // the signal's terms: time = flux / local_normalization, weighted by 1/binomial (:566-571)
+        if (a.signal_out)
+            for (uint32_t mask = lane; mask < subsets; mask += kWarp)
+                flux[mask] = dmul(ddiv(flux[mask], norm), a.inv_binom[__popc(mask)]);
+        // create_next_vertices_from_seed_into (:380-400): the retained vertices in
+        // order, then children of uniformly chosen parents among the vertices so
+        // far (the uniform kernel, mcmcmc_seed.h:51-55, ignores the parent)
+        const double* v = a.vertices + c * env * 4;
+        double* nv = a.next_vertices + c * env * 4;
+        int size = __popc(chosen);
+        for (int e = lane; e < 4 * size; e += kWarp) nv[e] = v[4 * nth_set_bit(chosen, e >> 2) + (e & 3)];
+        for (; size < env; ++size) {
+            const int parent = mt_uniform_int(g, size);
+            if constexpr (Hist) {
+                __syncwarp();  // the parent's coordinates, written by other lanes
+                double child[4];
+                hist_child(a, g, nv + 4 * parent, child);
+                if (lane < 4) nv[4 * size + lane] = lane == 0 ? child[0] : (lane == 1 ? child[1] : (lane == 2 ? child[2] : child[3]));
+            } else {
+                (void)parent;
+                const double x = g.canonical4();
+                if (lane < 4) nv[4 * size + lane] = x;
+            }
+        }
+        if (lane == 0) {
+            a.mt_index[c] = g.index;
+            if (a.chosen_out) a.chosen_out[row * a.chains + c] = chosen;
+            if (a.retained_out) a.retained_out[c] = chosen;
+            if (a.norm_out) a.norm_out[row * a.chains + c] = norm;
+            if (a.warmup) ++a.counts[c * (env + 1) + __popc(chosen)];
+        }
+    }
+    if (!a.signal_out) return;  // every thread
+    __syncthreads();
+    // each order's terms in mask order, (chain, order) pairs dealt to the block's threads
+    for (int item = threadIdx.x; item < per_block * (env + 1); item += blockDim.x) {
+        const int k = item / (env + 1), order = item - k * (env + 1);
+        if (s_state[k] != 2) continue;
+        const double* terms = step_smem + static_cast<size_t>(k) * per_chain;
+        double sig = 0.0;
+        if (order >= 1 && order >= a.order_min && order <= a.order_max) {
+            const uint32_t masks = kBinomial.c[env][order];
+            uint32_t m = (1u << order) - 1u;
+            for (uint32_t r = 0; r < masks; ++r, m = next_same_popcount(m)) sig = dadd(sig, terms[m]);
+        }
+        a.signal_out[(row * a.chains + static_cast<int64_t>(blockIdx.x) * per_block + k) * (env + 1) + order] = sig;
+    }
 }
 
 // The histogram seed kernel's conditional generation probabilities, one warp
@@ -467,18 +605,17 @@ cudaError_t launch_mcmcmc_step(const McmcmcStepArgs& args, cudaStream_t stream, 
     if (args.chains <= 0) return cudaSuccess;
     const bool hist = args.tau_bins > 0;
     if (args.chains < kStepWarpMaxChains && args.envelope <= kStepWarpMaxEnvelope) {
-        const size_t subsets = size_t{1} << args.envelope;
-        const size_t smem =
-            (subsets + (hist ? subsets + static_cast<size_t>(args.envelope) * (args.envelope + 1) : 0)) *
-            sizeof(double);
-        const void* fn = hist ? reinterpret_cast<const void*>(mcmcmc_step_warp<true>)
-                              : reinterpret_cast<const void*>(mcmcmc_step_warp<false>);
-        cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        // as many chains per block as leave every SM a block, while shared memory holds them
+        const size_t per_chain = step_doubles(args.envelope, hist) * sizeof(double);
+        int per_block = 1;
+        while (per_block * 2 <= kStepMaxChainsPerBlock && args.chains >= 2 * 152 * static_cast<int64_t>(per_block) &&
+               per_chain * per_block * 2 <= 96 * 1024)
+            per_block *= 2;
+        const size_t smem = per_chain * per_block;
+        auto kernel = hist ? mcmcmc_step_warp<true> : mcmcmc_step_warp<false>;
+        cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (err != cudaSuccess) return err;
-        if (hist)
-            mcmcmc_step_warp<true><<<static_cast<unsigned>(args.chains), 32, smem, stream>>>(args);
-        else
-            mcmcmc_step_warp<false><<<static_cast<unsigned>(args.chains), 32, smem, stream>>>(args);
+        kernel<<<static_cast<unsigned>((args.chains + per_block - 1) / per_block), per_block * kWarp, smem, stream>>>(args);
         *kernels = 1;
         return cudaGetLastError();
     }
