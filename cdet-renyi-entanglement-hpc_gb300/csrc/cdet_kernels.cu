@@ -565,6 +565,50 @@ __device__ __forceinline__ void pair_update(double dps, double am, double& acc, 
     }
 }
 
+// The round-off filter without its magnitude sum. The filter zeroes acc where
+// |acc| < threshold * rhs, rhs = |a[mask]| + sum |term| in FP64; that sum is as
+// many operations of the FP64 pipe as the terms' own. Its value is only needed
+// near the threshold: from the factors' exponent fields alone (integer work)
+// rhs lies between the largest normal term's lower bound 2^(fx + fy - 2046) and
+// 2^(k-1) times the largest upper bound 2^(fx + fy + 1 - 2046 + 2) (the one more
+// covers a subnormal factor, whose field is 0 and not 1) or |a[mask]|'s, and an
+// |acc| outside the thresholds of both is decided.
+// Sums of non-negative numbers rounded to nearest are monotone, so the
+// decision is the one the FP64 sum would give. Otherwise the caller forms rhs.
+struct FilterBounds {
+    uint32_t any = 0;     // largest sum of the factors' exponent fields (<< 20)
+    uint32_t normal = 0;  // the same where neither is zero or subnormal
+    __device__ __forceinline__ void add(double x, double y) {
+        const uint32_t fx = static_cast<uint32_t>(__double2hiint(x)) & 0x7FF00000u;
+        const uint32_t fy = static_cast<uint32_t>(__double2hiint(y)) & 0x7FF00000u;
+        any = max(any, fx + fy);
+        normal = max(normal, min(fx, fy) == 0u ? 0u : fx + fy);
+    }
+    // 1: acc stays, 0: acc is filtered, -1: the sum is needed. k: at most 2^(k-1) terms, a[mask] included.
+    __device__ __forceinline__ int decide(double acc, double a_mask, double threshold, int k) const {
+        const int fa = (__double2hiint(a_mask) >> 20) & 0x7FF;
+        const int upper = max(static_cast<int>(any >> 20) + 3 - 2046, max(fa, 1) + 1 - 1023) + k;  // rhs < 2^upper
+        if (upper > 1000 || upper < -900) return -1;
+        if (fabs(acc) >= dmul(threshold, __longlong_as_double(static_cast<long long>(upper + 1023) << 52))) return 1;
+        const int lower = static_cast<int>(normal >> 20) - 2046;  // rhs >= 2^lower
+        if (normal != 0 && lower > -900 && lower < 1000 &&
+            fabs(acc) < dmul(threshold, __longlong_as_double(static_cast<long long>(lower + 1023) << 52)))
+            return 0;
+        return -1;
+    }
+};
+
+// acc -= dp[s] a[m \ s] alone.
+template <bool Fused>
+__device__ __forceinline__ void accumulate_term(double dps, double am, double& acc) {
+    acc = Fused ? __fma_rn(-dps, am, acc) : dsub(acc, dmul(dps, am));
+}
+// rhs += |dp[s] a[m \ s]| as pair_update forms it.
+template <bool Fused>
+__device__ __forceinline__ void accumulate_magnitude(double dps, double am, double& rhs) {
+    rhs = Fused ? __fma_rn(fabs(dps), fabs(am), rhs) : dadd(rhs, fabs(dmul(dps, am)));
+}
+
 // compute_dp_ztransform (integrand_replica_randomly_sampled.h:226-290) for
 // this lane's configuration: only masks holding vertex 0 are reduced.
 template <bool Fused>
@@ -697,86 +741,120 @@ __global__ void __launch_bounds__(128) cdet_fp64(const __grid_constant__ Problem
 
 
 // ------------------------------------- 3a'. all-subsets CDet, warp form ----
-// compute_dp_ztransform_all_subsets for small batches (a few MCMCMC chains):
-// one warp per configuration, both sets at once, a and dp of each set in
-// shared memory. The masks of one popcount level are independent; the lanes
-// share the level's masks of both sets, dealt out by colex rank so that no
-// lane holds more than its share, and each mask's submask sum runs on one
-// lane in the reference's descending order with the same operations as
-// cdet_all, so the values are those of cdet_fp64 bit for bit. The lane form
-// keeps the FP64 pipe full on large batches; this form gives a small batch 32
-// lanes per configuration.
+// compute_dp_ztransform_all_subsets for small batches (MCMCMC chains): a block
+// of four warps per one to four configurations, both sets at once, a and dp in
+// shared memory. The masks of one popcount level are independent; the block's
+// threads share the level's masks of all its configurations and sets (the top
+// levels, of one to a few masks each, then still fill lanes), and each mask's
+// submask sum runs on one lane in the reference's descending order with the
+// same operations as cdet_all, so the values are those of cdet_fp64 bit for
+// bit. The lane form keeps the FP64 pipe full on large batches; this form gives
+// a small batch 32 to 128 lanes per configuration.
+//
+// Bound: the FP64 pipe, one or two operations per term (the round-off filter's
+// magnitude sum is formed only where FilterBounds cannot decide); for a few
+// configurations the top masks' serial sums. Measured at envelope 9 against
+// one warp per configuration with the magnitude sums: 128 configurations 169 -> 112 us
+// (FP64 form), 2,048 configurations 478 -> 259 us (split form).
+constexpr int kAllThreads = 128;
+
 template <bool Fused>
-__global__ void __launch_bounds__(128) cdet_all_warp(const __grid_constant__ Problem p,
-                                                    const __grid_constant__ Scratch w) {
+__global__ void __launch_bounds__(kAllThreads) cdet_all_warp(const __grid_constant__ Problem p,
+                                                            const __grid_constant__ Scratch w, int per_block) {
     extern __shared__ double all_smem[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t c = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + warp;
-    if (c >= p.batch) return;  // whole warps
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int64_t c0 = static_cast<int64_t>(blockIdx.x) * per_block;
+    const int configs = static_cast<int>(min(static_cast<int64_t>(per_block), p.batch - c0));
     const int n = p.max_order;
     const uint32_t count = 1u << n;
-    double* base = all_smem + static_cast<size_t>(warp) * 4 * count;  // [set][a, dp][count]
+    // per configuration [set][a, dp][count]; then the masks by popcount and colex rank
+    uint16_t* by_rank = reinterpret_cast<uint16_t*>(all_smem + static_cast<size_t>(per_block) * 4 * count);
     const Scalars& s = p.s;
     const double threshold = dmul(s.z_eps0, s.z_safety);
     const bool filter = threshold > 0.0;
-    const int64_t g = c >> 5;
-    const int cl = static_cast<int>(c & 31);
-    for (int set = 0; set < 2; ++set) {
-        const double* a = w.a_int + (g * 2 + set) * static_cast<int64_t>(count) * kWarp + cl;
-        double* a_s = base + set * 2 * count;
-        for (uint32_t m = lane; m < count; m += 32) a_s[m] = a[static_cast<int64_t>(m) * kWarp];
+    for (int k = warp; k < configs * 2; k += kAllThreads / 32) {
+        const int64_t c = c0 + (k >> 1);
+        const int set = k & 1;
+        const double* a = w.a_int + ((c >> 5) * 2 + set) * static_cast<int64_t>(count) * kWarp + (c & 31);
+        double* a_s = all_smem + static_cast<size_t>(k) * 2 * count;
+        for (uint32_t m = lane; m < count; m += 32) {
+            const double x = a[static_cast<int64_t>(m) * kWarp];
+            a_s[m] = x;
+            if (__popc(m) == 1) a_s[count + m] = x;  // dp of a singleton
+        }
     }
-    __syncwarp();
-    for (int item = lane; item < 2 * n; item += 32) {
-        const int set = item >= n ? 1 : 0, i = item - set * n;
-        double* a_s = base + set * 2 * count;
-        a_s[count + (1u << i)] = a_s[1u << i];  // dp of a singleton
+    for (uint32_t m = 1 + tid; m < count; m += kAllThreads) {
+        uint32_t at = 0, rank = 0;
+        for (int k = 1; k < __popc(m); ++k) at += kBinomial.c[n][k];
+        int i = 1;
+        for (uint32_t rest = m; rest; rest &= rest - 1u, ++i) rank += kBinomial.c[__ffs(static_cast<int>(rest)) - 1][i];
+        by_rank[at + rank] = static_cast<uint16_t>(m);
     }
-    __syncwarp();
+    __syncthreads();
+    uint32_t level = n;  // the first level-2 mask in by_rank
     for (int bits = 2; bits <= n; ++bits) {
         const uint32_t per = kBinomial.c[n][bits];
-        for (uint32_t item = lane; item < 2 * per; item += 32) {
-            const int set = item >= per ? 1 : 0;
-            const uint32_t mask = colex_subset(item - set * per, bits, n);
-            const double* a_s = base + set * 2 * count;
-            double* dp = base + set * 2 * count + count;
+        for (uint32_t item = tid; item < 2 * per * static_cast<uint32_t>(configs); item += kAllThreads) {
+            const uint32_t k = item / per;  // configuration and set
+            const uint32_t mask = by_rank[level + item - k * per];
+            const double* a_s = all_smem + static_cast<size_t>(k) * 2 * count;
+            double* dp = all_smem + static_cast<size_t>(k) * 2 * count + count;
             const uint32_t anchor = mask & (~mask + 1u);
             const uint32_t rest = mask ^ anchor;
-            double acc = a_s[mask];
-            double rhs = fabs(acc);
+            const double am = a_s[mask];
+            double acc = am;
+            FilterBounds bounds;
+#pragma unroll 4
             for (uint32_t sm = (rest - 1u) & rest;; sm = (sm - 1u) & rest) {
-                const uint32_t sub = sm | anchor;
-                pair_update<Fused>(dp[sub], a_s[mask ^ sub], acc, rhs);
+                const double x = dp[sm | anchor], y = a_s[rest ^ sm];
+                accumulate_term<Fused>(x, y, acc);
+                bounds.add(x, y);
                 if (sm == 0) break;
             }
-            if (filter && fabs(acc) < dmul(threshold, rhs)) acc = 0.0;
+            if (filter) {
+                int keep = bounds.decide(acc, am, threshold, bits);
+                if (keep < 0) {
+                    double rhs = fabs(am);
+                    for (uint32_t sm = (rest - 1u) & rest;; sm = (sm - 1u) & rest) {
+                        accumulate_magnitude<Fused>(dp[sm | anchor], a_s[rest ^ sm], rhs);
+                        if (sm == 0) break;
+                    }
+                    keep = fabs(acc) < dmul(threshold, rhs) ? 0 : 1;
+                }
+                if (keep == 0) acc = 0.0;
+            }
             dp[mask] = acc;
         }
-        __syncwarp();  // the next level reads this one
+        level += per;
+        __syncthreads();  // the next level reads this one
     }
     // integrand_all_subset_values_typed_into (:826-877) per set, then
     // twisted - 2 * ordinary (cdet_integrand_evaluator.h:346-350)
-    const double* diag = w.diag + c * 2 * 2 * n;
-    double* out = p.values + c * static_cast<int64_t>(count);
-    bool bad = false;
-    for (uint32_t mask = lane; mask < count; mask += 32) {
-        const int k = __popc(mask);
-        double v[2];
-        for (int set = 0; set < 2; ++set) {
-            const int r = set == 0 ? 2 : 1;
-            if (k == 0) {
-                v[set] = 0.0;
-            } else if (k == 1) {
-                const int i = __ffs(mask) - 1;
-                v[set] = order1_value(s, diag[(set * 2) * n + i], diag[(set * 2 + 1) * n + i], r);
-            } else {
-                v[set] = dmul(p.pref_ld[set][k], base[set * 2 * count + count + mask]);
+    for (int j = warp; j < configs; j += kAllThreads / 32) {
+        const int64_t c = c0 + j;
+        const double* base = all_smem + static_cast<size_t>(j) * 4 * count;
+        const double* diag = w.diag + c * 2 * 2 * n;
+        double* out = p.values + c * static_cast<int64_t>(count);
+        bool bad = false;
+        for (uint32_t mask = lane; mask < count; mask += 32) {
+            const int k = __popc(mask);
+            double v[2];
+            for (int set = 0; set < 2; ++set) {
+                const int r = set == 0 ? 2 : 1;
+                if (k == 0) {
+                    v[set] = 0.0;
+                } else if (k == 1) {
+                    const int i = __ffs(mask) - 1;
+                    v[set] = order1_value(s, diag[(set * 2) * n + i], diag[(set * 2 + 1) * n + i], r);
+                } else {
+                    v[set] = dmul(p.pref_ld[set][k], base[set * 2 * count + count + mask]);
+                }
+                if (!isfinite(v[set])) bad = true;
             }
-            if (!isfinite(v[set])) bad = true;
+            out[mask] = dsub(v[0], dmul(2.0, v[1]));
         }
-        out[mask] = dsub(v[0], dmul(2.0, v[1]));
+        if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(p.status + c, kStatusNonFinite);
     }
-    if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(p.status + c, kStatusNonFinite);
 }
 
 // ------------------------------------------------- 3b. CDet, warp form ----
@@ -1295,13 +1373,28 @@ __device__ double fp64_single_warp(const double* a, double* dp_s, int n, double 
         const int masks = kBinom[nbits][kk];
         for (int idx = lane; idx < masks; idx += kWarp) {
             const uint32_t rest = colex_unrank(static_cast<uint32_t>(idx), kk, nbits);
-            double acc = a[(rest << 1) | 1u];
-            double rhs = fabs(acc);
+            const double am = a[(rest << 1) | 1u];
+            double acc = am;
+            FilterBounds bounds;
+#pragma unroll 4
             for (uint32_t sm = (rest - 1u) & rest;; sm = (sm - 1u) & rest) {
-                pair_update<false>(dp_s[sm], a[(rest ^ sm) << 1], acc, rhs);
+                const double x = dp_s[sm], y = a[(rest ^ sm) << 1];
+                accumulate_term<false>(x, y, acc);
+                bounds.add(x, y);
                 if (sm == 0) break;
             }
-            if (filter && fabs(acc) < dmul(threshold, rhs)) acc = 0.0;
+            if (filter) {
+                int keep = bounds.decide(acc, am, threshold, k);
+                if (keep < 0) {
+                    double rhs = fabs(am);
+                    for (uint32_t sm = (rest - 1u) & rest;; sm = (sm - 1u) & rest) {
+                        accumulate_magnitude<false>(dp_s[sm], a[(rest ^ sm) << 1], rhs);
+                        if (sm == 0) break;
+                    }
+                    keep = fabs(acc) < dmul(threshold, rhs) ? 0 : 1;
+                }
+                if (keep == 0) acc = 0.0;
+            }
             dp_s[rest] = acc;
         }
         __syncwarp();  // the next level reads this one
@@ -1626,26 +1719,20 @@ static cudaError_t post_assembly(const Problem& p_in, const Scratch& w, int sm_c
     } else if (p.all_subsets && p.max_order <= kAllWarpMaxOrder && p.all_subsets_form != kFormLane &&
                (p.all_subsets_form == kFormWarp ||
                 p.batch < static_cast<int64_t>(all_subsets_lane_form_min_batch(sm_count)))) {
-        // a small batch of all-subset envelopes: one warp per configuration,
-        // one warp per block while that spreads the batch over more SMs
-        const size_t per_warp = 4 * (size_t{1} << p.max_order) * sizeof(double);
-        const int warps = p.batch < 4 * static_cast<int64_t>(sm_count > 0 ? sm_count : 152)
-                              ? 1
-                              : static_cast<int>(std::min<size_t>(4, (200 * 1024) / per_warp));
-        const size_t csmem = per_warp * warps;
-        if (p.fused_cdet) {
-            err = cudaFuncSetAttribute(cdet_all_warp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(csmem));
-            if (err != cudaSuccess) return err;
-            cdet_all_warp<true><<<static_cast<unsigned>((p.batch + warps - 1) / warps), warps * kWarp, csmem,
-                                  stream>>>(p, w);
-        } else {
-            err = cudaFuncSetAttribute(cdet_all_warp<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(csmem));
-            if (err != cudaSuccess) return err;
-            cdet_all_warp<false><<<static_cast<unsigned>((p.batch + warps - 1) / warps), warps * kWarp, csmem,
-                                   stream>>>(p, w);
-        }
+        // a small batch of all-subset envelopes: a block per configuration
+        // while that spreads the batch over more SMs, else up to four per block
+        const size_t per_config = 4 * (size_t{1} << p.max_order) * sizeof(double);
+        const size_t ranks = sizeof(uint16_t) * (size_t{1} << p.max_order);
+        const int64_t sms = sm_count > 0 ? sm_count : 152;
+        int per_block = 1;
+        while (per_block < 4 && p.batch >= 4 * sms * per_block && per_config * per_block * 2 + ranks <= 100 * 1024)
+            per_block *= 2;
+        const size_t csmem = per_config * per_block + ranks;
+        auto kernel = p.fused_cdet ? cdet_all_warp<true> : cdet_all_warp<false>;
+        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(csmem));
+        if (err != cudaSuccess) return err;
+        kernel<<<static_cast<unsigned>((p.batch + per_block - 1) / per_block), kAllThreads, csmem, stream>>>(p, w,
+                                                                                                          per_block);
     } else if (!p.all_subsets && p.max_order > kWarpCdetMaxOrder && p.max_order <= kBlockCdetMaxOrder) {
         // orders 11..14: one block per configuration (slots in decreasing order)
         const bool wide = p.max_order == kBlockCdetMaxOrder;
