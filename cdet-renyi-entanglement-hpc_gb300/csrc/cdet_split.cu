@@ -53,6 +53,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <type_traits>
 
 namespace cdet {
 
@@ -78,6 +79,16 @@ constexpr uint32_t kBStepBytes = kSlices * kTileN * kKStep * 2;       // 28 KiB
 // every byte a balanced digit plus 128; +256 at bit 56 makes the top field
 // (bits 48 and up) the leading digit plus 256, in [0, 512].
 constexpr uint64_t kDigitBias = 0x0100808080808080ull;
+// round(x / 2^6) + kDigitBias of a Q62 value x, |x| <= 2^62 (+ its rounding
+// error), in one shift: the bias moved up six bits keeps the sum non-negative
+__host__ __device__ __forceinline__ constexpr uint64_t biased_digits(int64_t x) {
+    return (static_cast<uint64_t>(x) + (32u + (kDigitBias << 6))) >> 6;
+}
+// the upper word of (t << 26) + kDigitBias for a Q30 value t: the lower word's
+// bias carries where t's low six bits are 32 or more
+__host__ __device__ __forceinline__ constexpr uint32_t biased_top_digits(int32_t t) {
+    return (static_cast<uint32_t>(t) + (32u + (static_cast<uint32_t>(kDigitBias >> 32) << 6))) >> 6;
+}
 
 // ----------------------------------------------------------- PTX helpers --
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
@@ -1226,83 +1237,70 @@ __global__ void __launch_bounds__(kAssemblyThreads, 1) split_assembly(const __gr
                 for (int k = 0; k < b0 / 8; ++k)  // to degrees b0 + j
 #pragma unroll
                     for (int j = 0; j < 8; ++j) ch[j].next(w8);
-                // one K step's digits (biased Q56 values of b = b0 + 16 ks + m:
-                // k = 0..7 hold the even m, k = 8..15 the odd m) into a stage
-                auto emit = [&](int ks, const uint64_t (&ye)[8], const uint64_t (&yo)[8]) -> bool {
+                // A K step: its stage, then the digits of its even columns
+                // b = b0 + 16 ks + 0, 2, .. 14 (k = 0..7, chains 0, 2, 4, 6, two
+                // steps each), then of its odd ones; columns past nv meet zero
+                // coefficients, whatever their digits. (Both parities at once
+                // would keep 16 64-bit values live and spill.)
+                auto begin_kstep = [&]() -> bool {
                     const int sb = static_cast<int>(b_cnt % kBStages);
-                    if (b_cnt >= kBStages && !mbar_wait(&sh.b_empty[sb], ((b_cnt / kBStages) - 1) & 1)) {
-                        sh.error = 1;
-                        return false;
-                    }
-                    // only the basis slices the K step's MMAs read: t' <= 8 - lead
-                    const int tmax = max(1, kSlicesA - tl.lead(ks));
-                    uint16_t* base = sh.basis_ring[sb] + core_offset(l, 0);
+                    return b_cnt < kBStages || mbar_wait(&sh.b_empty[sb], ((b_cnt / kBStages) - 1) & 1);
+                };
+                // only the basis slices the K step's MMAs read: t' <= 8 - lead (at most `most`)
+                auto store_digits = [&](int tmax, int odd, const uint64_t (&y)[8], auto most) {
+                    const uint32_t row = smem_addr(sh.basis_ring[b_cnt % kBStages] + core_offset(l, 0)) + 128u * odd;
 #pragma unroll
-                    for (int t = 1; t <= kSlices; ++t) {
+                    for (int t = 1; t <= decltype(most)::value; ++t) {
                         if (t > tmax) break;
-                        const uint32_t addr = smem_addr(base + (t - 1) * kTileN * kKStep);
-                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr),
-                                     "r"(digit_pair(ye[0], ye[1], t)), "r"(digit_pair(ye[2], ye[3], t)),
-                                     "r"(digit_pair(ye[4], ye[5], t)), "r"(digit_pair(ye[6], ye[7], t))
-                                     : "memory");
-                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr + 128),
-                                     "r"(digit_pair(yo[0], yo[1], t)), "r"(digit_pair(yo[2], yo[3], t)),
-                                     "r"(digit_pair(yo[4], yo[5], t)), "r"(digit_pair(yo[6], yo[7], t))
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row + (t - 1) * kSliceBytes),
+                                     "r"(digit_pair(y[0], y[1], t)), "r"(digit_pair(y[2], y[3], t)),
+                                     "r"(digit_pair(y[4], y[5], t)), "r"(digit_pair(y[6], y[7], t))
                                      : "memory");
                     }
+                };
+                auto end_kstep = [&]() {
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    mbar_arrive(&sh.b_full[sb]);
+                    mbar_arrive(&sh.b_full[b_cnt % kBStages]);
                     ++b_cnt;
-                    return true;
                 };
                 int ks = 0;
-                for (; ks < ks_tail && ok; ++ks) {  // Q62: all seven digits
-                    uint64_t ye[8], yo[8];
-                    const int bs = b0 + ks * kKStep;
+                for (; ks < ks_tail; ++ks) {  // Q62: all seven digits
+                    if (!(ok = begin_kstep())) break;
+                    const int tmax = max(1, kSlicesA - tl.lead(ks));
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const int64_t first = ch[j].next(w8), second = ch[j].next(w8);
-                        const uint64_t y1 = static_cast<uint64_t>(bs + j < p.s.nv ? (first + 32) >> 6 : 0) + kDigitBias;
-                        const uint64_t y2 =
-                            static_cast<uint64_t>(bs + 8 + j < p.s.nv ? (second + 32) >> 6 : 0) + kDigitBias;
-                        if (j & 1) {
-                            yo[j >> 1] = y1;
-                            yo[(j >> 1) + 4] = y2;
-                        } else {
-                            ye[j >> 1] = y1;
-                            ye[(j >> 1) + 4] = y2;
+                    for (int odd = 0; odd < 2; ++odd) {
+                        uint64_t y[8];
+#pragma unroll
+                        for (int m = 0; m < 4; ++m) {
+                            y[m] = biased_digits(ch[2 * m + odd].next(w8));
+                            y[m + 4] = biased_digits(ch[2 * m + odd].next(w8));
                         }
+                        store_digits(tmax, odd, y, std::integral_constant<int, kSlices>());
                     }
-                    ok = emit(ks, ye, yo);
+                    end_kstep();
                 }
-                if (ks < src.ksteps && ok) {  // Q30 from the tail K step on: digits 1 and 2
+                if (ks < src.ksteps && ok) {  // Q30 from the tail K step on: digits 1 and 2, both in the upper word
                     ChebChain30 c30[8];
 #pragma unroll
                     for (int j = 0; j < 8; ++j) c30[j] = ChebChain30{q62_to_q30(ch[j].prev), q62_to_q30(ch[j].cur)};
                     const int32_t w30 = q62_to_q30(w8);
-                    for (; ks < src.ksteps && ok; ++ks) {
-                        uint64_t ye[8], yo[8];
-                        const int bs = b0 + ks * kKStep;
+                    for (; ks < src.ksteps; ++ks) {
+                        if (!(ok = begin_kstep())) break;
+                        const int tmax = max(1, kSlicesA - tl.lead(ks));
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            const int32_t first = c30[j].next(w30), second = c30[j].next(w30);
-                            const uint64_t y1 =
-                                (bs + j < p.s.nv ? static_cast<uint64_t>(static_cast<int64_t>(first) << 26) : 0) +
-                                kDigitBias;
-                            const uint64_t y2 =
-                                (bs + 8 + j < p.s.nv ? static_cast<uint64_t>(static_cast<int64_t>(second) << 26) : 0) +
-                                kDigitBias;
-                            if (j & 1) {
-                                yo[j >> 1] = y1;
-                                yo[(j >> 1) + 4] = y2;
-                            } else {
-                                ye[j >> 1] = y1;
-                                ye[(j >> 1) + 4] = y2;
+                        for (int odd = 0; odd < 2; ++odd) {
+                            uint64_t y[8];
+#pragma unroll
+                            for (int m = 0; m < 4; ++m) {
+                                y[m] = static_cast<uint64_t>(biased_top_digits(c30[2 * m + odd].next(w30))) << 32;
+                                y[m + 4] = static_cast<uint64_t>(biased_top_digits(c30[2 * m + odd].next(w30))) << 32;
                             }
+                            store_digits(tmax, odd, y, std::integral_constant<int, kSlicesA - kTailLead>());
                         }
-                        ok = emit(ks, ye, yo);
+                        end_kstep();
                     }
                 }
+                if (!ok) sh.error = 1;
             }
             if (!ok) break;
             tl = tl_next;
