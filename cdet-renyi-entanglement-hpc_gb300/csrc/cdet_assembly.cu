@@ -25,16 +25,18 @@
 //
 // Measured against one thread per lookup (product on the FP64 pipe, 8-byte
 // loads), whole calls: 8x8 / degree 128 / order 10, 4,096 configurations
-// 106.5 -> 56.6 ms (two FP64 additions per coefficient at the pipe's 527 G/s:
-// 51 ms); 6x6 / degree 96, 4,096 mixed orders 1..10 26.6 -> 5.2 ms (no lanes
-// on entries past a configuration's order); one order-6 configuration 2.08 ->
-// 0.14 ms (all rows at once); 128 chains of envelope 9, a step with reused
-// pairs 3.35 -> 0.86 ms (copies and evaluations in one launch).
+// 106.5 -> 55.5 ms (two FP64 additions per coefficient at the pipe's 527 G/s:
+// 51 ms); 6x6 / degree 96, 4,096 mixed orders 1..10 26.6 -> 5.0 ms (no lanes
+// on entries past a configuration's order); 4x4 / 45 x 37 coefficients, two
+// spins, order 7 x 391 1.47 -> 0.68 ms; one order-6 configuration 2.08 -> 0.13
+// ms (all rows at once); 128 chains of envelope 9, a step with reused pairs
+// 3.35 -> 0.58 ms (copies and evaluations in one launch).
 #include "cdet_device.cuh"
 #include "cdet_kernels.cuh"
 #include "cdet_softmul.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace cdet {
 
@@ -121,13 +123,54 @@ __device__ __forceinline__ void store_entry(const Problem& p, const Scratch& w, 
     }
 }
 
+// What a lane needs of its lookup's x: the recurrence's 2x as a double and
+// unpacked for the integer product.
+struct Argument {
+    double x, two_x;
+    SoftFactor soft;
+};
+__device__ __forceinline__ Argument argument(double x) {
+    Argument a;
+    a.x = x;
+    a.two_x = dmul(2.0, x);
+    a.soft = soft_factor(static_cast<uint32_t>(__double2hiint(a.two_x)), static_cast<uint32_t>(__double2loint(a.two_x)));
+    return a;
+}
+__device__ __forceinline__ bool soft_argument(const Argument& a) {
+    return soft_factor_in_range(static_cast<uint32_t>(__double2hiint(a.two_x)));
+}
+
+// The recurrence's start c + 2x 0 - 0. With a finite x it is c itself unless c
+// is a zero (whose sign 2x decides).
+template <bool kSoft>
+__device__ __forceinline__ double first_step(double c, const Argument& a) {
+    if (kSoft && ((__double2hiint(c) << 1) | __double2loint(c)) != 0) return c;
+    return dsub(dadd(c, dmul(a.two_x, 0.0)), 0.0);
+}
+// The product 2x b (kSoft: on the integer pipes, `bad` set where that may not be the FP64 pipe's).
+template <bool kSoft>
+__device__ __forceinline__ double times_two_x(const Argument& a, double b, bool& bad) {
+    return kSoft ? soft_mul(a.soft, b, bad) : dmul(a.two_x, b);
+}
+// The row's end c_0 + x b_1 - b_2; the integer product is half of 2x b (its
+// exponent one less: never subnormal where soft_mul reports nothing).
+template <bool kSoft>
+__device__ __forceinline__ double last_step(double c, const Argument& a, double b1, double b2, bool& bad) {
+    double t;
+    if (kSoft) {
+        const double twice = soft_mul(a.soft, b1, bad);
+        t = __hiloint2double(__double2hiint(twice) - 0x100000, __double2loint(twice));
+    } else {
+        t = dmul(b1, a.x);
+    }
+    return dsub(dadd(c, t), b2);
+}
+
 // The Clenshaw steps of one full staged chunk (16 columns in decreasing
 // order). kFirst: its top column starts the recurrence; kLast: its lowest
-// column ends it. kSoft: products on the integer pipes, `bad` set where one
-// of them may differ from the FP64 pipe's.
+// column ends it.
 template <bool kSoft, bool kFirst, bool kLast>
-__device__ __forceinline__ void chunk_steps(const double* st, double two_x, const SoftFactor& fx, double x, double& b1,
-                                            double& b2, bool& bad) {
+__device__ __forceinline__ void chunk_steps(const double* st, const Argument& arg, double& b1, double& b2, bool& bad) {
 #pragma unroll
     for (int q = kChunk / 2 - 1; q >= 0; --q) {
         const double2 pair = *reinterpret_cast<const double2*>(st + 2 * q);
@@ -135,14 +178,12 @@ __device__ __forceinline__ void chunk_steps(const double* st, double two_x, cons
         for (int h = 1; h >= 0; --h) {
             const double c = h ? pair.y : pair.x;
             if (kFirst && q == kChunk / 2 - 1 && h == 1) {
-                // c + 2x 0 - 0
-                b1 = dsub(dadd(c, dmul(two_x, 0.0)), 0.0);
+                b1 = first_step<kSoft>(c, arg);
                 b2 = 0.0;
             } else if (kLast && q == 0 && h == 0) {
-                b1 = dsub(dadd(c, dmul(b1, x)), b2);
+                b1 = last_step<kSoft>(c, arg, b1, b2, bad);
             } else {
-                const double t = kSoft ? soft_mul(fx, b1, bad) : dmul(two_x, b1);
-                const double bk = dsub(dadd(c, t), b2);
+                const double bk = dsub(dadd(c, times_two_x<kSoft>(arg, b1, bad)), b2);
                 b2 = b1;
                 b1 = bk;
             }
@@ -151,17 +192,28 @@ __device__ __forceinline__ void chunk_steps(const double* st, double two_x, cons
 }
 
 // The same for a chunk of `count` < 16 columns (the top of a row).
-__device__ __forceinline__ void partial_chunk_steps(const double* st, int count, bool last, double two_x, double x,
-                                                    double& b1, double& b2) {
-    b1 = dsub(dadd(st[count - 1], dmul(two_x, 0.0)), 0.0);
+template <bool kSoft>
+__device__ __forceinline__ void partial_chunk_steps(const double* st, int count, bool last, const Argument& arg,
+                                                    double& b1, double& b2, bool& bad) {
+    b1 = first_step<kSoft>(st[count - 1], arg);
     b2 = 0.0;
     const int end = last ? 1 : 0;
     for (int k = count - 2; k >= end; --k) {
-        const double bk = dsub(dadd(st[k], dmul(two_x, b1)), b2);
+        const double bk = dsub(dadd(st[k], times_two_x<kSoft>(arg, b1, bad)), b2);
         b2 = b1;
         b1 = bk;
     }
-    if (last) b1 = dsub(dadd(st[0], dmul(b1, x)), b2);
+    if (last) b1 = last_step<kSoft>(st[0], arg, b1, b2, bad);
+}
+
+template <bool kSoft>
+__device__ __forceinline__ void row_chunk(const double* st, int count, bool first, bool last, const Argument& arg,
+                                          double& b1, double& b2, bool& bad) {
+    if (count < kChunk) partial_chunk_steps<kSoft>(st, count, last, arg, b1, b2, bad);
+    else if (first && last) chunk_steps<kSoft, true, true>(st, arg, b1, b2, bad);
+    else if (first) chunk_steps<kSoft, true, false>(st, arg, b1, b2, bad);
+    else if (last) chunk_steps<kSoft, false, true>(st, arg, b1, b2, bad);
+    else chunk_steps<kSoft, false, false>(st, arg, b1, b2, bad);
 }
 
 template <bool kVec16>
@@ -290,9 +342,11 @@ __global__ void __launch_bounds__(kThreads, 4) green_assembly_fp64(const __grid_
     const int nu = s.nu, nv = s.nv;
     const int chunks = (nv + kChunk - 1) / kChunk;
     const int top_count = nv - (chunks - 1) * kChunk;  // columns of a row's first (highest) chunk
-    // the outer sum of lookup tid, fed row values in decreasing order
-    OuterClenshaw outer;
-    if (tid < count) outer.init(nu - 1, sm.lookup[tid].u);
+    // the outer sum of lookup tid, fed row values in decreasing order (the
+    // recurrence of a row, over u)
+    Argument outer_arg;
+    double outer_b1 = 0.0, outer_b2 = 0.0;
+    if (tid < count) outer_arg = argument(sm.lookup[tid].u);
 
     for (int hi = nu; hi > 0; hi -= row_block) {
         const int rows = min(row_block, hi);
@@ -328,13 +382,9 @@ __global__ void __launch_bounds__(kThreads, 4) green_assembly_fp64(const __grid_
                 const int task = (warp + m * kWarps) * kWarp + lane;
                 const int task_c = min(task, tasks - 1);
                 const int l = task_c / rows, r = task_c - l * rows;
-                const double x = sm.lookup[l].v;
-                const double two_x = dmul(2.0, x);
-                const SoftFactor fx = soft_factor(static_cast<uint32_t>(__double2hiint(two_x)),
-                                                  static_cast<uint32_t>(__double2loint(two_x)));
-                // all-integer products while every lane's factor allows them and no chunk of this run failed
-                bool soft = __all_sync(0xffffffffu,
-                                       soft_factor_in_range(static_cast<uint32_t>(__double2hiint(two_x))));
+                const Argument arg = argument(sm.lookup[l].v);
+                // integer products while every lane's factor allows them and no chunk of this run failed
+                bool soft = __all_sync(0xffffffffu, soft_argument(arg));
                 double b1 = 0.0, b2 = 0.0;
                 for (int j = 0; j < chunks; ++j) {
                     // stage the next chunk, then wait for this one
@@ -349,30 +399,20 @@ __global__ void __launch_bounds__(kThreads, 4) green_assembly_fp64(const __grid_
                     asm volatile("cp.async.wait_group 1;" ::: "memory");
                     __syncwarp();
                     const double* st = sm.stage[warp][slot] + lane * kStride;
-                    const bool last = j == chunks - 1;
-                    if (j == 0 && top_count < kChunk) {
-                        partial_chunk_steps(st, top_count, last, two_x, x, b1, b2);
-                    } else {
-                        const double b1_in = b1, b2_in = b2;
-                        bool redo = !soft;
-                        if (soft) {
-                            bool bad = false;
-                            if (j == 0 && last) chunk_steps<true, true, true>(st, two_x, fx, x, b1, b2, bad);
-                            else if (j == 0) chunk_steps<true, true, false>(st, two_x, fx, x, b1, b2, bad);
-                            else if (last) chunk_steps<true, false, true>(st, two_x, fx, x, b1, b2, bad);
-                            else chunk_steps<true, false, false>(st, two_x, fx, x, b1, b2, bad);
-                            redo = __any_sync(0xffffffffu, bad);
-                        }
-                        if (redo) {
-                            soft = false;
-                            bool unused = false;
-                            b1 = b1_in;
-                            b2 = b2_in;
-                            if (j == 0 && last) chunk_steps<false, true, true>(st, two_x, fx, x, b1, b2, unused);
-                            else if (j == 0) chunk_steps<false, true, false>(st, two_x, fx, x, b1, b2, unused);
-                            else if (last) chunk_steps<false, false, true>(st, two_x, fx, x, b1, b2, unused);
-                            else chunk_steps<false, false, false>(st, two_x, fx, x, b1, b2, unused);
-                        }
+                    const int columns = j == 0 ? top_count : kChunk;
+                    const double b1_in = b1, b2_in = b2;
+                    bool redo = !soft;
+                    if (soft) {
+                        bool bad = false;
+                        row_chunk<true>(st, columns, j == 0, j == chunks - 1, arg, b1, b2, bad);
+                        redo = __any_sync(0xffffffffu, bad);
+                    }
+                    if (redo) {
+                        soft = false;
+                        bool unused = false;
+                        b1 = b1_in;
+                        b2 = b2_in;
+                        row_chunk<false>(st, columns, j == 0, j == chunks - 1, arg, b1, b2, unused);
                     }
                     __syncwarp();  // the buffer is free for the chunk after next
                     slot ^= 1;
@@ -382,13 +422,41 @@ __global__ void __launch_bounds__(kThreads, 4) green_assembly_fp64(const __grid_
             asm volatile("cp.async.wait_all;" ::: "memory");
         }
         __syncthreads();
-        if (tid < count)
-            for (int r = rows - 1; r >= 0; --r) outer.push(base_row + r, values[tid * value_stride + r]);
+        if (tid < count) {
+            const double* row_value = values + tid * value_stride;
+            const bool first = hi == nu, last = base_row == 0;
+            if (nu < 3) {  // degree 0 or 1: the sum's own short forms
+                outer_b1 = nu == 1 ? row_value[0] : dadd(row_value[0], dmul(row_value[1], outer_arg.x));
+            } else {
+                const double b1_in = outer_b1, b2_in = outer_b2;
+                auto sum = [&](auto use_soft) {
+                    constexpr bool kSoft = decltype(use_soft)::value;
+                    bool bad = false;
+                    int r = rows - 1;
+                    if (first) {
+                        outer_b1 = first_step<kSoft>(row_value[r--], outer_arg);
+                        outer_b2 = 0.0;
+                    }
+                    for (; r >= (last ? 1 : 0); --r) {
+                        const double bk = dsub(dadd(row_value[r], times_two_x<kSoft>(outer_arg, outer_b1, bad)), outer_b2);
+                        outer_b2 = outer_b1;
+                        outer_b1 = bk;
+                    }
+                    if (last) outer_b1 = last_step<kSoft>(row_value[0], outer_arg, outer_b1, outer_b2, bad);
+                    return bad;
+                };
+                if (!soft_argument(outer_arg) || sum(std::true_type())) {
+                    outer_b1 = b1_in;
+                    outer_b2 = b2_in;
+                    sum(std::false_type());
+                }
+            }
+        }
         __syncthreads();
     }
     if (tid < count && sm.lookup[tid].active)
         store_entry(p, w, c, n, sm.lookup[tid].set, sm.lookup[tid].i, sm.lookup[tid].j, sm.lookup[tid].spin,
-                    p.same_spin[sm.lookup[tid].set] != 0, outer.result());
+                    p.same_spin[sm.lookup[tid].set] != 0, outer_b1);
 }
 
 }  // namespace

@@ -79,66 +79,6 @@ __device__ __forceinline__ double clenshaw_row(const double* __restrict__ c, int
     return dsub(dadd(__ldg(c), dmul(b1, x)), b2);
 }
 
-// Two blocks (spin up and down) evaluated together: the row recurrences run
-// interleaved for instruction-level parallelism; the results equal two calls
-// of clenshaw_row.
-__device__ __forceinline__ void clenshaw_row_pair(const double* __restrict__ cu,
-                                                  const double* __restrict__ cd, int degree,
-                                                  double x, double& ru, double& rd) {
-    if (degree < 2) {
-        ru = clenshaw_row(cu, degree, x);
-        rd = clenshaw_row(cd, degree, x);
-        return;
-    }
-    const double two_x = dmul(2.0, x);
-    double u1 = 0.0, u2 = 0.0, d1 = 0.0, d2 = 0.0;
-#pragma unroll 4
-    for (int k = degree; k >= 1; --k) {
-        const double uk = dsub(dadd(__ldg(cu + k), dmul(two_x, u1)), u2);
-        const double dk = dsub(dadd(__ldg(cd + k), dmul(two_x, d1)), d2);
-        u2 = u1;
-        u1 = uk;
-        d2 = d1;
-        d1 = dk;
-    }
-    ru = dsub(dadd(__ldg(cu), dmul(u1, x)), u2);
-    rd = dsub(dadd(__ldg(cd), dmul(d1, x)), d2);
-}
-
-// Streaming form of the outer (u) Clenshaw sum over row values r_{nu-1}, ...,
-// r_0 delivered in descending order. Feeding every row value exactly once
-// gives the same operations as clenshaw_from_contiguous_coeffs over the full
-// row array (g_funcs.h:742-747).
-struct OuterClenshaw {
-    double x, two_x, b1, b2, first, second;
-    int degree;
-    __device__ __forceinline__ void init(int deg, double xv) {
-        degree = deg;
-        x = xv;
-        two_x = dmul(2.0, xv);
-        b1 = b2 = 0.0;
-        first = second = 0.0;
-    }
-    // Row value of index a (a runs from degree down to 0).
-    __device__ __forceinline__ void push(int a, double r) {
-        if (degree >= 2) {
-            if (a >= 1) {
-                const double bk = dsub(dadd(r, dmul(two_x, b1)), b2);
-                b2 = b1;
-                b1 = bk;
-            } else {
-                first = dsub(dadd(r, dmul(b1, x)), b2);
-            }
-        } else if (degree == 1) {
-            if (a == 1) second = r;
-            else first = dadd(r, dmul(second, x));
-        } else {
-            first = r;
-        }
-    }
-    __device__ __forceinline__ double result() const { return first; }
-};
-
 // ------------------------------------------------- integer subset helpers ---
 // Next integer with the same popcount (Gosper), for masks in increasing order.
 __device__ __forceinline__ uint32_t next_same_popcount(uint32_t v) {
