@@ -1586,6 +1586,46 @@ __global__ void order_scatter(const int32_t* __restrict__ orders, int64_t batch,
     }
 }
 
+// The same for a small batch in one block, one thread per configuration
+// (counts, scan and scatter in shared memory), which also resets the queue
+// head: one launch instead of a memset and three, about 2 us each on an
+// otherwise idle GPU; a larger batch has its own work to hide them behind.
+constexpr int64_t kSmallSortBatch = 512;
+__global__ void __launch_bounds__(kSmallSortBatch) order_sort_small(const int32_t* __restrict__ orders, int batch,
+                                                                    int max_order,
+                                                                    uint32_t* __restrict__ queue_head,
+                                                                    int32_t* __restrict__ slot_of,
+                                                                    int32_t* __restrict__ config_at) {
+    __shared__ uint32_t next[kMaxOrder + 2];
+    const int buckets = max_order + 2, c = threadIdx.x;
+    if (c < buckets) next[c] = 0;
+    if (c == 0) *queue_head = 0;
+    __syncthreads();
+    int bucket = 0;
+    if (c < batch) {
+        const int n = __ldg(orders + c);
+        bucket = (n < 1 || n > max_order) ? max_order + 1 : max_order - n;
+        atomicAdd(next + bucket, 1u);
+    }
+    __syncthreads();
+    if (c == 0) {
+        uint32_t run = 0;
+        for (int b = 0; b < buckets; ++b) {
+            const uint32_t k = next[b];
+            next[b] = run;
+            run += k;
+        }
+    }
+    __syncthreads();
+    if (c < batch) {
+        const uint32_t slot = atomicAdd(next + bucket, 1u);
+        slot_of[c] = static_cast<int32_t>(slot);
+        config_at[slot] = static_cast<int32_t>(c);
+    }
+}
+
+int order_sort_launches(int64_t batch) { return batch <= kSmallSortBatch ? 1 : 3; }
+
 size_t scratch_bytes(int64_t batch, int max_order, size_t ws_warps, ScratchRegions regions) {
     const size_t groups = static_cast<size_t>((batch + 31) / 32);
     const size_t n2 = static_cast<size_t>(max_order) * max_order;
@@ -1635,7 +1675,14 @@ static cudaError_t post_assembly(const Problem& p_in, const Scratch& w, int sm_c
     };
     const int threads = 128;
     cudaError_t err = cudaSuccess;
-    if (p.sorted) {
+    if (p.sorted && p.batch <= kSmallSortBatch) {
+        // (a warp per 32 configurations, at least the buckets' threads)
+        const unsigned sort_threads = static_cast<unsigned>((p.batch + 31) / 32 * 32);
+        order_sort_small<<<1, sort_threads, 0, stream>>>(p.orders, static_cast<int>(p.batch), p.max_order,
+                                                         w.order_count + kQueueHeadIndex, w.slot_of, w.config_at);
+        err = cudaGetLastError();
+        if (err != cudaSuccess) return err;
+    } else if (p.sorted) {
         const int buckets = p.max_order + 2;
         const unsigned grid = static_cast<unsigned>(std::min<int64_t>((p.batch + 255) / 256, 4 * 152));
         err = cudaMemsetAsync(w.order_count, 0, 64 * sizeof(uint32_t), stream);  // buckets, queue head
@@ -1685,12 +1732,14 @@ static cudaError_t post_assembly(const Problem& p_in, const Scratch& w, int sm_c
     // warps per block, as many blocks per SM as their chunk buffers allow
     const bool chunked = !use_smem && p.max_order >= kChunkMinOrder && p.max_order <= kChunkMaxOrder;
     const size_t chunk_bytes = chunked ? chunk_doubles_upto(p.max_order) * sizeof(double) : 0;
-    const int warps_per_block = use_smem ? fit : (chunked ? 8 : 4);
     const int64_t items = p.batch * 2;
+    const int sms = sm_count > 0 ? sm_count : 152;
+    // (a batch of fewer warps than the SMs hold spreads over all of them: warps of one SM share its FP64 pipe)
+    const int spread = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(fit, (items + sms - 1) / sms)));
+    const int warps_per_block = use_smem ? spread : (chunked ? 8 : 4);
     int64_t blocks = (items + warps_per_block - 1) / warps_per_block;
     const int64_t max_blocks = static_cast<int64_t>(w.ws_warps) / warps_per_block;
     blocks = std::min<int64_t>(blocks, std::max<int64_t>(1, max_blocks));
-    const int sms = sm_count > 0 ? sm_count : 152;
     if (use_smem) blocks = std::min<int64_t>(blocks, sms);  // one wave
     if (chunked) {
         const int64_t per_sm = std::max<int64_t>(1, (227 * 1024) / (chunk_bytes * warps_per_block + 1024));
@@ -1773,6 +1822,9 @@ void queue_launch_shape(const Problem& p, const Scratch& w, int sm_count, int* w
     const int sms = sm_count > 0 ? sm_count : 152;
     int per_sm = static_cast<int>(std::min<size_t>(32, sm_bytes / (ws_bytes + 16)));
     if (p.queue.warps_per_sm > 0) per_sm = std::min(per_sm, p.queue.warps_per_sm);
+    // (a batch of fewer warps than the SMs hold spreads over all of them: warps of one SM share its FP64 pipe)
+    const int64_t warps_wanted = (p.batch * (p.queue.pair ? 2 : 1) + sms - 1) / sms;
+    if (warps_wanted < per_sm) per_sm = static_cast<int>(warps_wanted + (p.queue.pair ? warps_wanted & 1 : 0));
     if (p.queue.pair) per_sm &= ~1;
     per_sm = std::max(per_sm, p.queue.pair ? 2 : 1);
     // as few blocks per SM as blocks of at most kQueueMaxWarps allow

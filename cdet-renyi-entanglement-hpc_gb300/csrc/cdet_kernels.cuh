@@ -378,9 +378,10 @@ cudaError_t launch_diagonal_order1(const TableDev* const tables[4], int n1, int 
 
 cudaError_t launch_fp64_integrand(const Problem& p, const Scratch& scratch, int sm_count,
                                   cudaStream_t stream, const KernelEvents* events, bool assembly = true);
-// Whether launch_fp64_integrand sorts the batch by order first (three more
-// kernels: the lane CDet of a single-order batch, and the queue form).
+// Whether launch_fp64_integrand sorts the batch by order first (the lane CDet
+// of a single-order batch, and the queue form), and the kernels that takes.
 bool sorts_orders(const Problem& p);
+int order_sort_launches(int64_t batch);
 // Whether the batch runs the queue form (p.integrand_form and the orders it supports).
 bool uses_queue_form(const Problem& p);
 // The double-double integrand after the FP64 assembly (orders <= kDDMaxOrder,
