@@ -247,14 +247,8 @@ int build_problem(cdet_context* ctx, const double* vertices, const int32_t* orde
     p->dd_beta = ctx->dd_beta;
     p->dd_tol = ctx->dd_tol;
     p->dd_fpm_shift = ctx->dd_fpm_shift;
-    for (int set = 0; set < 2; ++set) {
-        const int r = set == 0 ? 2 : 1;
-        for (int n = 0; n <= cdet::kMaxOrder; ++n) {
-            const HostDD dd = n >= 1 ? prefactor_dd(n, s.n1, s.n2, r) : HostDD{0.0, 0.0};
-            p->pref_dd[set][n] = cdet::DDPair{dd.hi, dd.lo};
-            p->pref_ld[set][n] = n >= 2 ? prefactor_ld(n, s.n1, s.n2, r) : 0.0;
-        }
-    }
+    std::memcpy(p->pref_dd, ctx->pref_dd, sizeof(p->pref_dd));
+    std::memcpy(p->pref_ld, ctx->pref_ld, sizeof(p->pref_ld));
     p->values = values;
     p->status = status;
     return CDET_OK;
@@ -634,15 +628,41 @@ int run_host(cdet_context* ctx, const double* vertices, const int32_t* orders, i
     double* d_val = reinterpret_cast<double*>(base + up(vbytes) + up(obytes));
     int32_t* d_s = reinterpret_cast<int32_t*>(base + up(vbytes) + up(obytes) + up(valbytes));
     cudaStream_t stream = nullptr;
-    cudaError_t err = cudaMemcpyAsync(d_v, vertices, vbytes, cudaMemcpyHostToDevice, stream);
-    if (err == cudaSuccess && obytes)
-        err = cudaMemcpyAsync(d_o, orders, obytes, cudaMemcpyHostToDevice, stream);
+    // Small calls go through a pinned mirror of the staging buffer: one copy
+    // each way by DMA, where pageable buffers take a driver-staged copy per
+    // array. Large ones copy the caller's buffers (pinned ones by DMA).
+    constexpr size_t kMirrorBytes = size_t{64} << 10;
+    cudaError_t err = cudaSuccess;
+    if (need <= kMirrorBytes && !ctx->pinned && cudaMallocHost(&ctx->pinned, kMirrorBytes) != cudaSuccess) {
+        ctx->pinned = nullptr;  // without it the caller's buffers are copied
+        cudaGetLastError();
+    }
+    char* mirror = need <= kMirrorBytes ? static_cast<char*>(ctx->pinned) : nullptr;
+    if (mirror) {
+        std::memcpy(mirror, vertices, vbytes);
+        if (obytes) std::memcpy(mirror + up(vbytes), orders, obytes);
+        err = cudaMemcpyAsync(base, mirror, up(vbytes) + obytes, cudaMemcpyHostToDevice, stream);
+    } else {
+        err = cudaMemcpyAsync(d_v, vertices, vbytes, cudaMemcpyHostToDevice, stream);
+        if (err == cudaSuccess && obytes)
+            err = cudaMemcpyAsync(d_o, orders, obytes, cudaMemcpyHostToDevice, stream);
+    }
     if (err != cudaSuccess) return cuda_fail(err, "cudaMemcpyAsync(H2D)");
     int rc = run(ctx, d_v, all_subsets ? nullptr : d_o, batch, order_arg, all_subsets, d_val, d_s, stream);
     if (rc != CDET_OK) return rc;
-    err = cudaMemcpyAsync(values, d_val, valbytes, cudaMemcpyDeviceToHost, stream);
-    if (err == cudaSuccess) err = cudaMemcpyAsync(status, d_s, sbytes, cudaMemcpyDeviceToHost, stream);
-    if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
+    if (mirror) {
+        const size_t at = up(vbytes) + up(obytes);
+        err = cudaMemcpyAsync(mirror + at, base + at, up(valbytes) + sbytes, cudaMemcpyDeviceToHost, stream);
+        if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
+        if (err == cudaSuccess) {
+            std::memcpy(values, mirror + at, valbytes);
+            std::memcpy(status, mirror + at + up(valbytes), sbytes);
+        }
+    } else {
+        err = cudaMemcpyAsync(values, d_val, valbytes, cudaMemcpyDeviceToHost, stream);
+        if (err == cudaSuccess) err = cudaMemcpyAsync(status, d_s, sbytes, cudaMemcpyDeviceToHost, stream);
+        if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
+    }
     if (err != cudaSuccess) return cuda_fail(err, "evaluation");
     if (ctx->assembly == CDET_ASSEMBLY_SPLIT_BF16 && ctx->split_error) {
         int32_t flag = 0;
@@ -741,6 +761,14 @@ int cdet_create(const cdet_runtime_scalars* scalars, int device, cdet_context** 
         delete ctx;
         return cuda_fail(err, "cudaDeviceGetAttribute");
     }
+    for (int set = 0; set < 2; ++set) {
+        const int r = set == 0 ? 2 : 1;
+        for (int n = 0; n <= cdet::kMaxOrder; ++n) {
+            const HostDD dd = n >= 1 ? prefactor_dd(n, s.n1, s.n2, r) : HostDD{0.0, 0.0};
+            ctx->pref_dd[set][n] = cdet::DDPair{dd.hi, dd.lo};
+            ctx->pref_ld[set][n] = n >= 2 ? prefactor_ld(n, s.n1, s.n2, r) : 0.0;
+        }
+    }
     *out = ctx;
     return CDET_OK;
 }
@@ -755,6 +783,7 @@ void cdet_destroy(cdet_context* ctx) {
     for (TableSlot& slot : ctx->tables) release_slot(slot);
     if (ctx->scratch) cudaFree(ctx->scratch);
     if (ctx->staging) cudaFree(ctx->staging);
+    if (ctx->pinned) cudaFreeHost(ctx->pinned);
     if (ctx->split_scratch) cudaFree(ctx->split_scratch);
     for (auto& kv : ctx->sliced) cudaFree(kv.second.mem);
     delete ctx;

@@ -50,9 +50,14 @@ struct cdet_context {
     int scratch_order = 0;
     size_t ws_warps = 0;
     bool scratch_dd = false;  // the scratch holds the double-double lane region
-    // staging for the host-buffer entry points
+    // the order prefactors of both sets (they depend on the lattice alone; the
+    // long double ones are soft-float on hosts whose long double is binary128)
+    cdet::DDPair pref_dd[2][cdet::kMaxOrder + 1]{};
+    double pref_ld[2][cdet::kMaxOrder + 1]{};
+    // staging for the host-buffer entry points, and its pinned mirror for small calls
     void* staging = nullptr;
     size_t staging_bytes = 0;
+    void* pinned = nullptr;
     uint64_t calls = 0, fallbacks = 0;
     int last_launches = 0;
     // split assembly
