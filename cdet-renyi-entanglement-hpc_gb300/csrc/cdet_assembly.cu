@@ -10,27 +10,30 @@
 // lookup runs the outer sum over them.
 //
 // Row sums: each lane walks one row of nv coefficients downwards. The 32 rows
-// of a warp are copied 16 columns at a time with cp.async (two buffers per
+// of a warp are copied eight columns at a time with cp.async (two buffers per
 // warp, the next chunk in flight while one is consumed), so the global reads
-// are whole 128-byte pieces of rows; read straight from global memory each
+// are 64-byte pieces of rows; read straight from global memory each
 // lane's 8-byte loads were 32 separate L1 wavefronts per step, about what the
 // FP64 work of the step takes.
 //
 // Arithmetic: a step b_k = c_k + 2x b_{k+1} - b_{k+2} is a product and two
-// additions, each rounded. The FP64 pipe bounds the kernel (two lane
-// operations per clock and SM), so the product is formed on the integer pipes
-// (cdet_softmul.cuh) and only the additions go to the FP64 pipe. A chunk in
-// which some lane's product may not be the common case is repeated from its
-// first step with the product on the FP64 pipe.
+// additions, each rounded. The FP64 pipe would bound the kernel (two lane
+// operations per clock and SM), so the product and every other step's first
+// addition are formed on the integer pipes (cdet_softmul.cuh): 1.5 FP64
+// operations per step. A chunk in which some lane's operands may not be the
+// common case is repeated from its first step on the FP64 pipe. Chunks of
+// eight columns and 96 registers let five blocks share an SM (a step is a long
+// dependent chain: with chunks of 16 and four blocks the same arithmetic took
+// 51.6 ms instead of 44.0).
 //
 // Measured against one thread per lookup (product on the FP64 pipe, 8-byte
 // loads), whole calls: 8x8 / degree 128 / order 10, 4,096 configurations
-// 106.5 -> 55.5 ms (two FP64 additions per coefficient at the pipe's 527 G/s:
-// 51 ms); 6x6 / degree 96, 4,096 mixed orders 1..10 26.6 -> 5.0 ms (no lanes
-// on entries past a configuration's order); 4x4 / 45 x 37 coefficients, two
-// spins, order 7 x 391 1.47 -> 0.68 ms; one order-6 configuration 2.08 -> 0.13
-// ms (all rows at once); 128 chains of envelope 9, a step with reused pairs
-// 3.35 -> 0.58 ms (copies and evaluations in one launch).
+// 106.5 -> 44.0 ms (three FP64 operations per coefficient at the pipe's 527
+// G/s: 76 ms; one and a half: 38 ms); 6x6 / degree 96, 4,096 mixed orders 1..10
+// 26.6 -> 4.1 ms (no lanes on entries past a configuration's order); 4x4 / 45 x
+// 37 coefficients, two spins, order 7 x 391 1.47 -> 0.55 ms; one order-6
+// configuration 2.08 -> 0.08 ms (all rows at once); 128 chains of envelope 9, a
+// step with reused pairs 3.35 -> 0.54 ms (copies and evaluations in one launch).
 #include "cdet_device.cuh"
 #include "cdet_kernels.cuh"
 #include "cdet_softmul.cuh"
@@ -87,8 +90,8 @@ constexpr int kThreads = 128;
 constexpr int kWarps = kThreads / kWarp;
 constexpr int kMaxLookups = 16;  // lookups of one block: the outer sums run on that many lanes of one warp
 constexpr int kRowBlock = 128;   // row values kept per lookup; more rows are taken block by block
-constexpr int kChunk = 16;       // columns of a staged chunk
-constexpr int kStride = 18;      // doubles between the rows of a staged chunk: 16-byte aligned, 16-byte reads free of bank conflicts
+constexpr int kChunk = 8;        // columns of a staged chunk
+constexpr int kStride = 10;      // doubles between the rows of a staged chunk: 16-byte aligned, 16-byte reads free of bank conflicts
 
 // One lookup of the block.
 struct Lookup {
@@ -166,7 +169,13 @@ __device__ __forceinline__ double last_step(double c, const Argument& a, double 
     return dsub(dadd(c, t), b2);
 }
 
-// The Clenshaw steps of one full staged chunk (16 columns in decreasing
+// The columns of a chunk whose first addition runs on the integer pipes too
+// (soft_add): every other one, where the FP64 pipe and the integer pipes finish
+// about together. 8x8 / degree 128 / order 10, 4,096 configurations: none of
+// eight 55.5 ms, two 49.2, three 46.1, four 44.0, five 45.2, six 48.4.
+constexpr uint32_t kSoftSums = 0x55;
+
+// The Clenshaw steps of one full staged chunk (its columns in decreasing
 // order). kFirst: its top column starts the recurrence; kLast: its lowest
 // column ends it.
 template <bool kSoft, bool kFirst, bool kLast>
@@ -183,7 +192,9 @@ __device__ __forceinline__ void chunk_steps(const double* st, const Argument& ar
             } else if (kLast && q == 0 && h == 0) {
                 b1 = last_step<kSoft>(c, arg, b1, b2, bad);
             } else {
-                const double bk = dsub(dadd(c, times_two_x<kSoft>(arg, b1, bad)), b2);
+                const double t = times_two_x<kSoft>(arg, b1, bad);
+                const bool soft_sum = kSoft && ((kSoftSums >> (2 * q + h)) & 1) != 0;
+                const double bk = dsub(soft_sum ? soft_add(c, t, bad) : dadd(c, t), b2);
                 b2 = b1;
                 b1 = bk;
             }
@@ -191,7 +202,7 @@ __device__ __forceinline__ void chunk_steps(const double* st, const Argument& ar
     }
 }
 
-// The same for a chunk of `count` < 16 columns (the top of a row).
+// The same for a chunk of `count` < kChunk columns (the top of a row).
 template <bool kSoft>
 __device__ __forceinline__ void partial_chunk_steps(const double* st, int count, bool last, const Argument& arg,
                                                     double& b1, double& b2, bool& bad) {
@@ -219,27 +230,18 @@ __device__ __forceinline__ void row_chunk(const double* st, int count, bool firs
 template <bool kVec16>
 __device__ __forceinline__ void stage_chunk(double* st, const double* const* row, int column, int count, int lane) {
     const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(st));
-    if constexpr (kVec16) {  // eight lanes of 16 bytes per row
-        const int part = lane & 7;
-        if (2 * part < count) {
+    // lanes of one row: 16 bytes each where the rows are aligned to it, else 8
+    constexpr int kLanes = kVec16 ? kChunk / 2 : kChunk;
+    const int part = (lane & (kLanes - 1)) * (kVec16 ? 2 : 1);
+    if (part < count) {
 #pragma unroll
-            for (int it = 0; it < kWarp / 4; ++it) {
-                const int r = it * 4 + (lane >> 3);
-                const double* src = row[r] + column + 2 * part;
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst + (r * kStride + 2 * part) * 8),
-                             "l"(src));
-            }
-        }
-    } else {  // sixteen lanes of 8 bytes per row
-        const int part = lane & 15;
-        if (part < count) {
-#pragma unroll
-            for (int it = 0; it < kWarp / 2; ++it) {
-                const int r = it * 2 + (lane >> 4);
-                const double* src = row[r] + column + part;
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + (r * kStride + part) * 8),
-                             "l"(src));
-            }
+        for (int r0 = 0; r0 < kWarp; r0 += kWarp / kLanes) {
+            const int r = r0 + lane / kLanes;
+            const double* src = row[r] + column + part;
+            if constexpr (kVec16)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst + (r * kStride + part) * 8), "l"(src));
+            else
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + (r * kStride + part) * 8), "l"(src));
         }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -252,7 +254,7 @@ __device__ __forceinline__ void stage_chunk(double* st, const double* const* row
 // k..n-1, then rows i >= k at every column), where the blocks with
 // blockIdx.y == 0 also copy the retained ones.
 template <bool kVec16>
-__global__ void __launch_bounds__(kThreads, 4) green_assembly_fp64(const __grid_constant__ Problem p,
+__global__ void __launch_bounds__(kThreads, 5) green_assembly_fp64(const __grid_constant__ Problem p,
                                                                   const __grid_constant__ Scratch w,
                                                                   int lookups_per_block, int row_block) {
     extern __shared__ __align__(16) unsigned char assembly_smem[];

@@ -85,10 +85,87 @@ __host__ __device__ __forceinline__ void soft_mul_bits(const SoftFactor& x, uint
 #endif
 }
 
+// x + y, correctly rounded, on the integer pipes: about 55 of their
+// instructions, more than an FP64 addition's time on its own pipe, so a kernel
+// takes it for a share of its additions only. The operand of larger magnitude
+// keeps its place in a window of three words (21 + 32 bits and 32 guard bits),
+// the other is shifted down to it and added or subtracted. `bad` as for the
+// product: an operand zero, subnormal, infinite, NaN or near the ends of the
+// exponent range, 21 or more bits cancelled, operands whose order the upper
+// words do not tell, or, where a shift by 32 or more has dropped bits below the
+// window, discarded bits within a few units of a tie. Exact ties (frequent:
+// nearby exponents discard a bit or two) round to even here.
+__host__ __device__ __forceinline__ void soft_add_bits(uint32_t x_hi, uint32_t x_lo, uint32_t y_hi, uint32_t y_lo,
+                                                       uint32_t& r_hi, uint32_t& r_lo, bool& bad) {
+    const bool swap = (x_hi & 0x7FFFFFFFu) < (y_hi & 0x7FFFFFFFu);
+    const uint32_t bh = swap ? y_hi : x_hi, bl = swap ? y_lo : x_lo;
+    const uint32_t sh = swap ? x_hi : y_hi, sl = swap ? x_lo : y_lo;
+    const uint32_t small_field = sh & 0x7FF00000u;
+    uint32_t d = ((bh & 0x7FF00000u) - small_field) >> 20;
+    d = d < 63u ? d : 63u;
+    const uint32_t mb = (bh & 0xFFFFFu) | 0x100000u, ms = (sh & 0xFFFFFu) | 0x100000u;
+    const bool far = d >= 32u;
+    const uint32_t w2 = far ? 0u : ms, w1 = far ? ms : sl, w0 = far ? sl : 0u;
+    const uint32_t m = static_cast<uint32_t>(static_cast<int32_t>(bh ^ sh) >> 31);  // all ones: subtract
+#ifdef __CUDA_ARCH__
+    const uint32_t z2 = __funnelshift_r(w2, 0u, d) ^ m, z1 = __funnelshift_r(w1, w2, d) ^ m;
+    const uint32_t z0 = __funnelshift_r(w0, w1, d) ^ m;
+    uint32_t s0, s1, s2;
+    asm("{.reg .u32 t;\n"
+        " add.cc.u32 t, %3, 1;\n"
+        " addc.cc.u32 %0, %4, 0;\n"
+        " addc.cc.u32 %1, %5, %6;\n"
+        " addc.u32 %2, %7, %8;}"
+        : "=&r"(s0), "=&r"(s1), "=r"(s2)
+        : "r"(m), "r"(z0), "r"(z1), "r"(bl), "r"(z2), "r"(mb));
+    const uint32_t n = static_cast<uint32_t>(__clz(static_cast<int>(s2))) - 10u;
+    const uint32_t v2 = __funnelshift_l(s1, s2, n), v1 = __funnelshift_l(s0, s1, n), v0 = s0 << (n & 31u);
+    const uint32_t k1 = __funnelshift_r(v1, v2, 1), rest = __funnelshift_r(v0, v1, 1);
+#else
+    const uint32_t c = d & 31u;
+    auto right = [c](uint32_t lo, uint32_t hi) { return c ? (lo >> c) | (hi << (32 - c)) : lo; };
+    const uint32_t z2 = right(w2, 0u) ^ m, z1 = right(w1, w2) ^ m, z0 = right(w0, w1) ^ m;
+    uint64_t carry = static_cast<uint64_t>(z0) + (m & 1u);
+    const uint32_t s0 = static_cast<uint32_t>(carry);
+    carry = (carry >> 32) + bl + z1;
+    const uint32_t s1 = static_cast<uint32_t>(carry);
+    const uint32_t s2 = static_cast<uint32_t>((carry >> 32) + mb + z2);
+    const uint32_t n = (s2 ? static_cast<uint32_t>(__builtin_clz(s2)) : 32u) - 10u;
+    const uint32_t e = n & 31u;
+    const uint32_t v2 = e ? (s2 << e) | (s1 >> (32 - e)) : s2, v1 = e ? (s1 << e) | (s0 >> (32 - e)) : s1, v0 = s0 << e;
+    const uint32_t k1 = (v1 >> 1) | (v2 << 31), rest = (v0 >> 1) | (v1 << 31);
+#endif
+    bad |= s2 - 1u >= 0x3FFFFFu;                          // negative, or 21 bits and more cancelled
+    bad |= far && rest - 0x7FFFFFFCu <= 8u;
+    bad |= (bh << 1) - (64u << 21) > (1936u << 21);       // the larger exponent field outside 64..2000
+    bad |= small_field == 0u;
+    const uint32_t field = (bh & 0xFFF00000u) - (n << 20);
+    const uint32_t keep = rest == 0x80000000u ? 0xFFFFFFFEu : 0xFFFFFFFFu;  // a tie rounds up, then to even
+#ifdef __CUDA_ARCH__
+    asm("{.reg .u32 t;\n"
+        " add.cc.u32 t, %2, 0x80000000;\n"
+        " addc.cc.u32 %0, %3, 0;\n"
+        " addc.u32 %1, %4, %5;}"
+        : "=&r"(r_lo), "=r"(r_hi)
+        : "r"(rest), "r"(k1), "r"(v2 >> 1), "r"(field));
+    r_lo &= keep;
+#else
+    const uint64_t kept = ((static_cast<uint64_t>(v2 >> 1) << 32) | k1) + (rest >> 31);
+    r_lo = static_cast<uint32_t>(kept) & keep;
+    r_hi = static_cast<uint32_t>(kept >> 32) + field;
+#endif
+}
+
 #ifdef __CUDACC__
 __device__ __forceinline__ double soft_mul(const SoftFactor& x, double b, bool& bad) {
     uint32_t hi, lo;
     soft_mul_bits(x, static_cast<uint32_t>(__double2hiint(b)), static_cast<uint32_t>(__double2loint(b)), hi, lo, bad);
+    return __hiloint2double(static_cast<int>(hi), static_cast<int>(lo));
+}
+__device__ __forceinline__ double soft_add(double x, double y, bool& bad) {
+    uint32_t hi, lo;
+    soft_add_bits(static_cast<uint32_t>(__double2hiint(x)), static_cast<uint32_t>(__double2loint(x)),
+                  static_cast<uint32_t>(__double2hiint(y)), static_cast<uint32_t>(__double2loint(y)), hi, lo, bad);
     return __hiloint2double(static_cast<int>(hi), static_cast<int>(lo));
 }
 #endif
