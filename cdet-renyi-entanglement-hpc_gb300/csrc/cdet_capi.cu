@@ -594,6 +594,7 @@ int run(cdet_context* ctx, const double* vertices, const int32_t* orders, int64_
         err = cdet::launch_fp64_assembly(p, w, ctx->sm_count, stream);
         if (err != cudaSuccess) return cuda_fail(err, "kernel launch");
     }
+    if (!assembly_only && !p.all_subsets && max_order > 10 && max_order <= 14) ++launches;  // the sets' combine
     if (!assembly_only && cdet::sorts_orders(p)) launches += cdet::order_sort_launches(batch);
     ctx->last_launches = launches;  // kernels of this library (the status and bucket resets are memsets)
     if (events) ctx->pending_launches += launches;
@@ -716,7 +717,7 @@ int run_fp64_on_scratch(cdet_context* ctx, const double* vertices, const int32_t
     if (err != cudaSuccess) return cuda_fail(err, "cudaMemsetAsync(status)");
     err = launch_fp64_integrand(p, w, ctx->sm_count, stream, nullptr);
     if (err != cudaSuccess) return cuda_fail(err, "kernel launch");
-    ctx->last_launches = 3 + (sorts_orders(p) ? order_sort_launches(batch) : 0);
+    ctx->last_launches = 3 + (max_order > 10 && max_order <= 14 ? 1 : 0) + (sorts_orders(p) ? order_sort_launches(batch) : 0);
     return CDET_OK;
 }
 

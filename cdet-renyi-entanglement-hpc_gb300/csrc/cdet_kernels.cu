@@ -1111,8 +1111,10 @@ __global__ void __launch_bounds__(kWarpCdetWarps * 32, 2) cdet_split_warp(const 
 // ------------------------------ 3c. single-top CDet, block per configuration
 // compute_dp_ztransform (integrand_replica_randomly_sampled.h:226-290) for
 // orders 11..14, where a batch holds few configurations and a lane's 2^n-entry
-// recursion would leave the SMs nearly empty: one CTA per configuration (256
-// threads; 512 at n = 14, where the shared memory leaves one CTA per SM),
+// recursion would leave the SMs nearly empty: one CTA per configuration and set
+// (256 threads; 512 at n = 14, where the shared memory leaves one CTA per SM; a
+// CTA for both sets made the last wave twice as long: 512 configurations of
+// order 14 5.2 -> 4.6 ms with the split),
 // a of the masks without vertex 0 and dp of the masks with it
 // in shared memory (2^(n-1) doubles each; 128 KiB at n = 14), the masks of
 // each popcount level dealt out by colex rank. FP64 form: each mask's
@@ -1210,7 +1212,8 @@ __global__ void __launch_bounds__(kBlockCdetThreads) cdet_block(const __grid_con
     // FP64 form at order 14: the top levels' products (see fp64_top_level)
     constexpr bool kChains = !Fused && kBlockCdetThreads == 512;
     double* terms = dp_s + half;
-    const int64_t slot = blockIdx.x;
+    const int64_t slot = blockIdx.x >> 1;
+    const int set = static_cast<int>(blockIdx.x & 1);
     const int64_t c = p.sorted ? __ldg(w.config_at + slot) : slot;
     const int64_t g = slot >> 5;
     const int cl = static_cast<int>(slot & 31);
@@ -1226,120 +1229,131 @@ __global__ void __launch_bounds__(kBlockCdetThreads) cdet_block(const __grid_con
     const float thresholdf = static_cast<float>(threshold);
     const int64_t full = int64_t{1} << nmax;
     const double* diag = w.diag + c * 2 * 2 * nmax;
-    int32_t status = 0;
-    DD value[2] = {DD{0.0, 0.0}, DD{0.0, 0.0}};
-    for (int set = 0; set < 2; ++set) {
-        const int r = set == 0 ? 2 : 1;
-        if (n == 1) {
-            value[set] = DD{order1_value(s, diag[(set * 2) * nmax], diag[(set * 2 + 1) * nmax], r), 0.0};
-            continue;
-        }
-        const double* ag = w.a_int + (g * 2 + set) * full * kWarp + cl;
-        const int count = 1 << n;
-        int e = 0;
-        if constexpr (Fused) {
-            const uint64_t bits = static_cast<uint64_t>(__double_as_longlong(ag[1 * kWarp]));
-            const int field = static_cast<int>((bits >> 52) & 0x7FF);
-            if (field != 0 && field != 0x7FF) e = field - 1023;
-            e = e > 60 ? 60 : (e < -60 ? -60 : e);  // |e| * n stays within 1000
-        }
-        for (int m2 = tid; m2 < count / 2; m2 += kBlockCdetThreads) a_s[m2] = ag[static_cast<int64_t>(2 * m2) * kWarp];
-        if (tid == 0) dp_s[0] = ag[1 * kWarp];
-        __syncthreads();
-        const int nbits = n - 1;
-        for (int k = 2; k <= n; ++k) {
-            const int kk = k - 1;            // rest = mask >> 1 has kk of nbits bits
-            const int masks = static_cast<int>(binom[nbits][kk]);
-            const int subs = 1 << kk;        // submasks of rest, rest itself included
-            if constexpr (kChains) {
-                if (masks <= kWarp && subs >= 1024) {
-                    fp64_top_level<kBlockCdetThreads>(ag, a_s, dp_s, terms, half, masks, kk, nbits, binom,
-                                                      threshold, filter, chain_rhs);
-                    __syncthreads();
-                    continue;
-                }
-            }
-            const int field_bias = 127 - 2046 - e * k;
-            for (int base = 0; base < masks;) {
-                const int remaining = masks - base;
-                int L = 1, take = kBlockCdetThreads;
-                if (Fused && remaining < kBlockCdetThreads) {
-                    while (L * 2 * remaining <= kBlockCdetThreads && L * 2 <= subs && L < kWarp) L *= 2;
-                    take = remaining;
-                    if (4 * L * remaining < 3 * kBlockCdetThreads && L * 2 <= subs && L < kWarp) {
-                        L *= 2;  // < 75% of the threads busy
-                        take = kBlockCdetThreads / L;
-                    }
-                }
-                const int q = __ffs(L) - 1;
-                const int idx = base + (tid >> q);
-                const bool active = (tid >> q) < take && idx < masks;
-                if constexpr (!Fused) {
-                    if (active) {
-                        const uint32_t rest = colex_subset_s(static_cast<uint32_t>(idx), kk, nbits, binom);
-                        const uint32_t mask = (rest << 1) | 1u;
-                        double acc = ag[static_cast<int64_t>(mask) * kWarp];
-                        double rhs = fabs(acc);
-                        for (uint32_t sl = (rest - 1u) & rest;; sl = (sl - 1u) & rest) {
-                            const uint32_t sub = (sl << 1) | 1u;
-                            pair_update<false>(dp_s[sub >> 1], a_s[(mask ^ sub) >> 1], acc, rhs);
-                            if (sl == 0) break;
-                        }
-                        if (filter && fabs(acc) < dmul(threshold, rhs)) acc = 0.0;
-                        dp_s[mask >> 1] = acc;
-                    }
-                } else {
-                    const int j = tid & (L - 1);
-                    double part = 0.0;
-                    float rpart = 0.0f;
-                    uint32_t mask = 0;
-                    if (active) {
-                        const uint32_t rest = colex_subset_s(static_cast<uint32_t>(idx), kk, nbits, binom);
-                        mask = (rest << 1) | 1u;
-                        // the top q bits of rest are fixed by the lane's index in its group
-                        uint32_t top = 0, low = rest;
-                        for (int t = 0; t < q; ++t) {
-                            const uint32_t hb = 1u << (31 - __clz(low));
-                            top |= hb;
-                            low ^= hb;
-                        }
-                        uint32_t fixed = 0, tb = top;
-                        for (int t = 0; t < q; ++t) {
-                            const uint32_t lb = tb & (~tb + 1u);
-                            if ((j >> t) & 1) fixed |= lb;
-                            tb ^= lb;
-                        }
-                        fused_submask_sum<false>(dp_s, a_s, rest, fixed, low, field_bias, part, rpart);
-                    }
-                    for (int off = 1; off < L; off <<= 1) {
-                        part = dadd(part, __shfl_xor_sync(0xffffffffu, part, off));
-                        rpart += __shfl_xor_sync(0xffffffffu, rpart, off);
-                    }
-                    if (active && j == 0) {
-                        const double am = ag[static_cast<int64_t>(mask) * kWarp];
-                        double acc = dsub(am, part);
-                        const float rhs = scaled_magnitude(am, -e * k) + rpart;
-                        if (filter && scaled_magnitude(acc, -e * k) < thresholdf * rhs) acc = 0.0;
-                        dp_s[mask >> 1] = acc;
-                    }
-                }
-                base += take;
-            }
-            __syncthreads();
-        }
+    // this set's value goes where its a of masks 0 and 1 were (a[0] is no term, a[1] is read first)
+    double* ag = w.a_int + (g * 2 + set) * full * kWarp + cl;
+    if (n == 1) {
         if (tid == 0) {
-            const DDPair pf = p.pref_dd[set][n];
-            value[set] = dd_mul(DD{pf.hi, pf.lo}, DD{dp_s[(count - 1) >> 1], 0.0});
-            if (!dd_finite(value[set])) status |= kStatusNonFinite;
+            ag[0] = order1_value(s, diag[(set * 2) * nmax], diag[(set * 2 + 1) * nmax], set == 0 ? 2 : 1);
+            ag[kWarp] = 0.0;
         }
-        __syncthreads();  // the next set reuses the arrays
+        return;
+    }
+    const int count = 1 << n;
+    int e = 0;
+    if constexpr (Fused) {
+        const uint64_t bits = static_cast<uint64_t>(__double_as_longlong(ag[1 * kWarp]));
+        const int field = static_cast<int>((bits >> 52) & 0x7FF);
+        if (field != 0 && field != 0x7FF) e = field - 1023;
+        e = e > 60 ? 60 : (e < -60 ? -60 : e);  // |e| * n stays within 1000
+    }
+    for (int m2 = tid; m2 < count / 2; m2 += kBlockCdetThreads) a_s[m2] = ag[static_cast<int64_t>(2 * m2) * kWarp];
+    if (tid == 0) dp_s[0] = ag[1 * kWarp];
+    __syncthreads();
+    const int nbits = n - 1;
+    for (int k = 2; k <= n; ++k) {
+        const int kk = k - 1;            // rest = mask >> 1 has kk of nbits bits
+        const int masks = static_cast<int>(binom[nbits][kk]);
+        const int subs = 1 << kk;        // submasks of rest, rest itself included
+        if constexpr (kChains) {
+            if (masks <= kWarp && subs >= 1024) {
+                fp64_top_level<kBlockCdetThreads>(ag, a_s, dp_s, terms, half, masks, kk, nbits, binom,
+                                                  threshold, filter, chain_rhs);
+                __syncthreads();
+                continue;
+            }
+        }
+        const int field_bias = 127 - 2046 - e * k;
+        for (int base = 0; base < masks;) {
+            const int remaining = masks - base;
+            int L = 1, take = kBlockCdetThreads;
+            if (Fused && remaining < kBlockCdetThreads) {
+                while (L * 2 * remaining <= kBlockCdetThreads && L * 2 <= subs && L < kWarp) L *= 2;
+                take = remaining;
+                if (4 * L * remaining < 3 * kBlockCdetThreads && L * 2 <= subs && L < kWarp) {
+                    L *= 2;  // < 75% of the threads busy
+                    take = kBlockCdetThreads / L;
+                }
+            }
+            const int q = __ffs(L) - 1;
+            const int idx = base + (tid >> q);
+            const bool active = (tid >> q) < take && idx < masks;
+            if constexpr (!Fused) {
+                if (active) {
+                    const uint32_t rest = colex_subset_s(static_cast<uint32_t>(idx), kk, nbits, binom);
+                    const uint32_t mask = (rest << 1) | 1u;
+                    double acc = ag[static_cast<int64_t>(mask) * kWarp];
+                    double rhs = fabs(acc);
+                    for (uint32_t sl = (rest - 1u) & rest;; sl = (sl - 1u) & rest) {
+                        const uint32_t sub = (sl << 1) | 1u;
+                        pair_update<false>(dp_s[sub >> 1], a_s[(mask ^ sub) >> 1], acc, rhs);
+                        if (sl == 0) break;
+                    }
+                    if (filter && fabs(acc) < dmul(threshold, rhs)) acc = 0.0;
+                    dp_s[mask >> 1] = acc;
+                }
+            } else {
+                const int j = tid & (L - 1);
+                double part = 0.0;
+                float rpart = 0.0f;
+                uint32_t mask = 0;
+                if (active) {
+                    const uint32_t rest = colex_subset_s(static_cast<uint32_t>(idx), kk, nbits, binom);
+                    mask = (rest << 1) | 1u;
+                    // the top q bits of rest are fixed by the lane's index in its group
+                    uint32_t top = 0, low = rest;
+                    for (int t = 0; t < q; ++t) {
+                        const uint32_t hb = 1u << (31 - __clz(low));
+                        top |= hb;
+                        low ^= hb;
+                    }
+                    uint32_t fixed = 0, tb = top;
+                    for (int t = 0; t < q; ++t) {
+                        const uint32_t lb = tb & (~tb + 1u);
+                        if ((j >> t) & 1) fixed |= lb;
+                        tb ^= lb;
+                    }
+                    fused_submask_sum<false>(dp_s, a_s, rest, fixed, low, field_bias, part, rpart);
+                }
+                for (int off = 1; off < L; off <<= 1) {
+                    part = dadd(part, __shfl_xor_sync(0xffffffffu, part, off));
+                    rpart += __shfl_xor_sync(0xffffffffu, rpart, off);
+                }
+                if (active && j == 0) {
+                    const double am = ag[static_cast<int64_t>(mask) * kWarp];
+                    double acc = dsub(am, part);
+                    const float rhs = scaled_magnitude(am, -e * k) + rpart;
+                    if (filter && scaled_magnitude(acc, -e * k) < thresholdf * rhs) acc = 0.0;
+                    dp_s[mask >> 1] = acc;
+                }
+            }
+            base += take;
+        }
+        __syncthreads();
     }
     if (tid == 0) {
-        const DD result = dd_sub(value[0], dd_mul(DD{2.0, 0.0}, value[1]));
-        p.values[c] = dadd(result.hi, result.lo);
-        if (status) atomicOr(p.status + c, status);
+        const DDPair pf = p.pref_dd[set][n];
+        const DD value = dd_mul(DD{pf.hi, pf.lo}, DD{dp_s[(count - 1) >> 1], 0.0});
+        if (!dd_finite(value)) atomicOr(p.status + c, kStatusNonFinite);
+        ag[0] = value.hi;
+        ag[kWarp] = value.lo;
     }
 }
+
+// twisted - 2 ordinary of the two sets' values cdet_block left, one thread per slot.
+__global__ void __launch_bounds__(128) combine_sets(const __grid_constant__ Problem p,
+                                                   const __grid_constant__ Scratch w) {
+    const int64_t slot = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (slot >= p.batch) return;
+    const int64_t c = p.sorted ? __ldg(w.config_at + slot) : slot;
+    const int n = __ldg(p.orders + c);
+    if (n < 1 || n > p.max_order) return;
+    const int64_t per_set = (int64_t{1} << p.max_order) * kWarp;
+    const double* t = w.a_int + (slot >> 5) * 2 * per_set + (slot & 31);
+    const double* o = t + per_set;
+    const DD result = dd_sub(DD{t[0], t[kWarp]}, dd_mul(DD{2.0, 0.0}, DD{o[0], o[kWarp]}));
+    p.values[c] = dadd(result.hi, result.lo);
+}
+
 
 // ------------------------------------------ 4. persistent queue form -------
 // Minors, CDet and combine of each configuration in one persistent kernel,
@@ -1735,8 +1749,8 @@ static cudaError_t post_assembly(const Problem& p_in, const Scratch& w, int sm_c
     const int64_t items = p.batch * 2;
     const int sms = sm_count > 0 ? sm_count : 152;
     // (a batch of fewer warps than the SMs hold spreads over all of them: warps of one SM share its FP64 pipe)
-    const int spread = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(fit, (items + sms - 1) / sms)));
-    const int warps_per_block = use_smem ? spread : (chunked ? 8 : 4);
+    const int most = use_smem ? fit : (chunked ? 8 : 4);
+    const int warps_per_block = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(most, (items + sms - 1) / sms)));
     int64_t blocks = (items + warps_per_block - 1) / warps_per_block;
     const int64_t max_blocks = static_cast<int64_t>(w.ws_warps) / warps_per_block;
     blocks = std::min<int64_t>(blocks, std::max<int64_t>(1, max_blocks));
@@ -1783,7 +1797,7 @@ static cudaError_t post_assembly(const Problem& p_in, const Scratch& w, int sm_c
         kernel<<<static_cast<unsigned>((p.batch + per_block - 1) / per_block), kAllThreads, csmem, stream>>>(p, w,
                                                                                                           per_block);
     } else if (!p.all_subsets && p.max_order > kWarpCdetMaxOrder && p.max_order <= kBlockCdetMaxOrder) {
-        // orders 11..14: one block per configuration (slots in decreasing order)
+        // orders 11..14: one block per configuration and set (slots in decreasing order)
         const bool wide = p.max_order == kBlockCdetMaxOrder;
         // a and dp, plus (FP64 form at order 14) as much again / 2 for the top levels' products
         const size_t csmem = sizeof(double) * (size_t{1} << p.max_order) * (wide && !p.fused_cdet ? 3 : 2) / 2;
@@ -1791,7 +1805,8 @@ static cudaError_t post_assembly(const Problem& p_in, const Scratch& w, int sm_c
                                    : (wide ? cdet_block<false, 512> : cdet_block<false, 256>);
         err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(csmem));
         if (err != cudaSuccess) return err;
-        kernel<<<static_cast<unsigned>(p.batch), wide ? 512 : 256, csmem, stream>>>(p, w);
+        kernel<<<static_cast<unsigned>(2 * p.batch), wide ? 512 : 256, csmem, stream>>>(p, w);
+        combine_sets<<<static_cast<unsigned>((p.batch + 127) / 128), 128, 0, stream>>>(p, w);
     } else {
         cdet_fp64<<<static_cast<unsigned>((p.batch + threads - 1) / threads), threads, 0, stream>>>(p, w);
     }
