@@ -19,6 +19,7 @@
 // every lane of every FP64 instruction busy.
 #include "cdet_device.cuh"
 #include "cdet_kernels.cuh"
+#include "cdet_softmul.cuh"
 
 #include <algorithm>
 
@@ -131,6 +132,25 @@ __device__ __forceinline__ void remove_shift_blocked(double* shifted, int n, dou
     __syncwarp();
 }
 
+// The largest |A[k]| of a matrix that is no NaN (0 if none), by a whole warp,
+// compared as integers: like the pivots' test and reciprocal below, work that
+// the FP64 pipe, which bounds the minors, need not do (65,536 order-10
+// configurations, split assembly: minors 5.13 -> 4.48 ms for the three).
+__device__ __forceinline__ double warp_max_abs(const double* A, int msize, int lane) {
+    int64_t best = 0;
+    for (int k = lane; k < msize; k += kWarp) {
+        const int64_t e = __double_as_longlong(A[k]) & 0x7FFFFFFFFFFFFFFFLL;
+        if (e > best && e <= 0x7FF0000000000000LL) best = e;
+    }
+    for (int off = 16; off > 0; off >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, off));
+    return __longlong_as_double(best);
+}
+
+// |pivot| is zero, or at most eps >= 0, given as its bits.
+__device__ __forceinline__ bool pivot_too_small(double pivot, int64_t eps_bits) {
+    return (__double_as_longlong(pivot) & 0x7FFFFFFFFFFFFFFFLL) <= eps_bits;
+}
+
 // mat2pm_from_buffer (fast_principle_minors.h:120-246) for one matrix, by a
 // whole warp. On return shifted[mask] (mask >= 1) holds the principal minor
 // of the rows/columns in mask. Returns true when a pivot sent the matrix to
@@ -143,15 +163,7 @@ __device__ bool mat2pm_warp(const double* A, int n, double tol, double shift_par
                             int lane) {
     const int msize = n * n;
     const uint32_t subsets = 1u << n;
-    double max_abs = 0.0;
-    for (int k = lane; k < msize; k += kWarp) {
-        const double e = fabs(A[k]);
-        if (e > max_abs) max_abs = e;
-    }
-    for (int off = 16; off > 0; off >>= 1) {
-        const double o = __shfl_xor_sync(0xffffffffu, max_abs, off);
-        if (o > max_abs) max_abs = o;
-    }
+    const double max_abs = warp_max_abs(A, msize, lane);
     const bool explicit_shift = !(shift_param < 0.0);
     const double p = explicit_shift ? shift_param : ddiv(max_abs, static_cast<double>(msize));
     if (max_abs == 0.0 && p == 0.0) {
@@ -159,7 +171,7 @@ __device__ bool mat2pm_warp(const double* A, int n, double tol, double shift_par
         __syncwarp();
         return false;
     }
-    const double fallback_eps = (tol > 0.0 && max_abs > 0.0) ? dmul(tol, max_abs) : 0.0;
+    const int64_t eps_bits = (tol > 0.0 && max_abs > 0.0) ? __double_as_longlong(dmul(tol, max_abs)) : 0LL;
 
     // A node's pivot inverse replaces its pivot entry and its first-column
     // factors replace column 0 of rows 1.. (the children take only rows and
@@ -176,6 +188,7 @@ __device__ bool mat2pm_warp(const double* A, int n, double tol, double shift_par
     }
     __syncwarp();
     if (lane == 0) shifted[1] = dadd(compact ? p : shifted[1], old_list[0]);
+    __syncwarp();
 
     uint32_t minor_index = 2;
     bool fell_back = false;
@@ -188,11 +201,10 @@ __device__ bool mat2pm_warp(const double* A, int n, double tol, double shift_par
         // pivots of this level, one per set
         bool bad_pivot = false;
         for (int set = lane; set < sets; set += kWarp) {
-            const double pivot = dadd(old_list[set * old_msize], p);
-            const double pa = fabs(pivot);
-            if (pa == 0.0 || (fallback_eps > 0.0 && pa <= fallback_eps)) bad_pivot = true;
-            // 1.0 / pivot, correctly rounded (IEEE): the same value
-            old_list[set * old_msize] = __drcp_rn(pivot);
+            // the pivot's entry plus p is already there as the node's shifted minor
+            const double pivot = compact ? shifted[sets + set] : dadd(old_list[set * old_msize], p);
+            bad_pivot |= pivot_too_small(pivot, eps_bits);
+            old_list[set * old_msize] = soft_rcp(pivot);
         }
         if (__any_sync(0xffffffffu, bad_pivot)) {
             fell_back = true;
@@ -337,7 +349,7 @@ __host__ __device__ inline int chunk_doubles_upto(int nmax) {
 // shifted minor receives exactly one addition, p + the child's pivot entry,
 // written directly (the whole-level form adds it to the p it initialised).
 __device__ bool schur_level(const double* old_list, double* new_list, double* inv, int nodes, int old_size,
-                            double p, double fallback_eps, double* shifted, uint32_t base, uint32_t c0,
+                            double p, int64_t eps_bits, double* shifted, uint32_t base, uint32_t c0,
                             int log2g, int T, int lane) {
     const int old_msize = old_size * old_size;
     const int new_size = old_size - 1;
@@ -345,9 +357,8 @@ __device__ bool schur_level(const double* old_list, double* new_list, double* in
     bool bad_pivot = false;
     for (int set = lane; set < nodes; set += kWarp) {
         const double pivot = dadd(old_list[set * old_msize], p);
-        const double pa = fabs(pivot);
-        if (pa == 0.0 || (fallback_eps > 0.0 && pa <= fallback_eps)) bad_pivot = true;
-        inv[set] = __drcp_rn(pivot);  // 1.0 / pivot, correctly rounded (IEEE): the same value
+        bad_pivot |= pivot_too_small(pivot, eps_bits);
+        inv[set] = soft_rcp(pivot);
     }
     if (__any_sync(0xffffffffu, bad_pivot)) return false;
     __syncwarp();
@@ -411,15 +422,7 @@ __device__ bool mat2pm_chunked(const double* A, int n, double tol, double shift_
                                double* ws, double* shifted, double* lu_lane, double* chunk, int lane) {
     const int msize = n * n;
     const uint32_t subsets = 1u << n;
-    double max_abs = 0.0;
-    for (int k = lane; k < msize; k += kWarp) {
-        const double e = fabs(A[k]);
-        if (e > max_abs) max_abs = e;
-    }
-    for (int off = 16; off > 0; off >>= 1) {
-        const double o = __shfl_xor_sync(0xffffffffu, max_abs, off);
-        if (o > max_abs) max_abs = o;
-    }
+    const double max_abs = warp_max_abs(A, msize, lane);
     const bool explicit_shift = !(shift_param < 0.0);
     const double p = explicit_shift ? shift_param : ddiv(max_abs, static_cast<double>(msize));
     if (max_abs == 0.0 && p == 0.0) {
@@ -427,7 +430,7 @@ __device__ bool mat2pm_chunked(const double* A, int n, double tol, double shift_
         __syncwarp();
         return false;
     }
-    const double fallback_eps = (tol > 0.0 && max_abs > 0.0) ? dmul(tol, max_abs) : 0.0;
+    const int64_t eps_bits = (tol > 0.0 && max_abs > 0.0) ? __double_as_longlong(dmul(tol, max_abs)) : 0LL;
     double* old_list = ws + lay.old_list;
     double* new_list = ws + lay.new_list;
     double* inv = ws + lay.aux;
@@ -441,7 +444,7 @@ __device__ bool mat2pm_chunked(const double* A, int n, double tol, double shift_
     const ChunkGeom g = chunk_geom(n);
     bool ok = true;
     for (int level = 0; level < g.T && ok; ++level) {
-        ok = schur_level(old_list, new_list, inv, 1 << level, n - level, p, fallback_eps, shifted,
+        ok = schur_level(old_list, new_list, inv, 1 << level, n - level, p, eps_bits, shifted,
                          2u << level, 0u, 30, 0, lane);
         double* t = old_list;
         old_list = new_list;
@@ -456,7 +459,7 @@ __device__ bool mat2pm_chunked(const double* A, int n, double tol, double shift_
         for (int k = lane; k < G * msz; k += kWarp) co[k] = old_list[c0 * msz + k];
         __syncwarp();
         for (int j = 0; j + 1 < m && ok; ++j) {
-            ok = schur_level(co, cn, caux, G << j, m - j, p, fallback_eps, shifted, 2u << (g.T + j), c0,
+            ok = schur_level(co, cn, caux, G << j, m - j, p, eps_bits, shifted, 2u << (g.T + j), c0,
                              g.log2g, g.T, lane);
             double* t = co;
             co = cn;

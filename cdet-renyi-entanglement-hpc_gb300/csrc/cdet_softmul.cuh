@@ -1,4 +1,4 @@
-// A correctly rounded FP64 product on the integer pipes.
+// Correctly rounded FP64 products, sums and reciprocals on the integer pipes.
 //
 // GB300 retires about two FP64 lane operations per clock and SM, so a warp's
 // FP64 instruction holds its sub-partition's FP64 pipe for 64 to 74 clocks.
@@ -156,7 +156,55 @@ __host__ __device__ __forceinline__ void soft_add_bits(uint32_t x_hi, uint32_t x
 #endif
 }
 
+// 1 / b, correctly rounded, on the integer pipes (about 50 instructions, where
+// the FP64 one holds its pipe for eight). From a 24-bit reciprocal a little
+// below 1/b, q0, the residual e = 1 - b q0 in (0, 2^-21) gives q0 (1 + e + e^2)
+// within one unit of the last place; the exact remainder 2^105 - B Q, whose
+// magnitude is below 2^54, then says whether that neighbour or the next is the
+// nearest (a reciprocal is never a tie).
+// seed: the FP32 bits of an approximation, within a unit or so of its last
+// place, of the reciprocal of soft_rcp_arg(b). `bad` (set, never cleared): a
+// power of two, a zero, subnormal, infinite or NaN b, a subnormal result, or a
+// seed further off than that.
+__host__ __device__ __forceinline__ uint32_t soft_rcp_arg(uint32_t b_hi, uint32_t b_lo) {
+    return 0x3F800001u + (((b_hi & 0xFFFFFu) << 3) | (b_lo >> 29));  // rounded up
+}
+
+__host__ __device__ __forceinline__ void soft_rcp_bits(uint32_t b_hi, uint32_t b_lo, uint32_t seed, uint32_t& r_hi,
+                                                       uint32_t& r_lo, bool& bad) {
+    const uint64_t B = (static_cast<uint64_t>((b_hi & 0xFFFFFu) | 0x100000u) << 32) | b_lo;  // 2^52 b
+    const uint32_t top = static_cast<uint32_t>(B >> 21), bottom = b_lo << 11;
+    const uint32_t below = seed - 2u;
+    const uint32_t q0 = ((below > 0x3F000000u ? below : 0x3F000000u) << 8) | 0x80000000u;    // 2^32 / b
+    const uint64_t t = (uint64_t{1} << 63) + 512u -
+                       (static_cast<uint64_t>(top) * q0 + ((static_cast<uint64_t>(bottom) * q0) >> 32));
+    bad |= static_cast<uint32_t>(t >> 42) != 0u;
+    const uint32_t e = static_cast<uint32_t>(t >> 10);                                       // 2^53 e
+    const uint32_t e2 = static_cast<uint32_t>((static_cast<uint64_t>(e) * e) >> 32);         // 2^74 e^2
+    const uint64_t c = static_cast<uint64_t>(q0) * e + ((static_cast<uint64_t>(q0) * e2) >> 21) + 0x80000000u;
+    uint64_t Q = (static_cast<uint64_t>(q0) << 21) + (c >> 32);                              // 2^53 / b
+    const int64_t r2 = static_cast<int64_t>((0u - B * Q) << 1);
+    Q -= static_cast<uint64_t>((static_cast<int64_t>(B) - r2) >> 63);  // 2 R > B: the next above
+    Q += static_cast<uint64_t>((static_cast<int64_t>(B) + r2) >> 63);  // 2 R < -B: the next below
+    const uint32_t field = (b_hi >> 20) & 0x7FFu;
+    bad |= field - 1u >= 2043u;
+    bad |= B == uint64_t{1} << 52;
+    r_lo = static_cast<uint32_t>(Q);
+    r_hi = (b_hi & 0x80000000u) + ((2044u - field) << 20) + static_cast<uint32_t>(Q >> 32);
+}
+
 #ifdef __CUDACC__
+// 1 / b, correctly rounded, for any b.
+__device__ __forceinline__ double soft_rcp(double b) {
+    const uint32_t b_hi = static_cast<uint32_t>(__double2hiint(b)), b_lo = static_cast<uint32_t>(__double2loint(b));
+    uint32_t hi, lo;
+    float seed;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(seed) : "f"(__uint_as_float(soft_rcp_arg(b_hi, b_lo))));
+    bool bad = false;
+    soft_rcp_bits(b_hi, b_lo, __float_as_uint(seed), hi, lo, bad);
+    if (bad) return __drcp_rn(b);
+    return __hiloint2double(static_cast<int>(hi), static_cast<int>(lo));
+}
 __device__ __forceinline__ double soft_mul(const SoftFactor& x, double b, bool& bad) {
     uint32_t hi, lo;
     soft_mul_bits(x, static_cast<uint32_t>(__double2hiint(b)), static_cast<uint32_t>(__double2loint(b)), hi, lo, bad);
