@@ -3,7 +3,8 @@
 // After the Green matrices (cdet_assembly.cu or cdet_split.cu), two launches
 // per batch of vertex configurations:
 //
-//  1. principal_minors_fp64: one warp per (configuration, table set). The
+//  1. principal_minors_shared (two or four warps per (configuration, table set))
+//     or, above order 10, principal_minors_fp64 (one warp). The
 //     warp runs the shifted Schur-complement recursion of mat2pm level by
 //     level, lanes spread over (set, row, column) work items, then the prefix
 //     product and the shift removal, and writes a[mask] = pm_up * pm_down into
@@ -151,24 +152,50 @@ __device__ __forceinline__ bool pivot_too_small(double pivot, int64_t eps_bits) 
     return (__double_as_longlong(pivot) & 0x7FFFFFFFFFFFFFFFLL) <= eps_bits;
 }
 
-// mat2pm_from_buffer (fast_principle_minors.h:120-246) for one matrix, by a
-// whole warp. On return shifted[mask] (mask >= 1) holds the principal minor
+// The threads of one matrix: a warp, or Warps of them that meet at a named barrier.
+template <int Warps>
+__device__ __forceinline__ void group_sync(int barrier) {
+    if constexpr (Warps == 1) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"r"(barrier), "n"(Warps * kWarp) : "memory");
+}
+
+// Whether any thread's predicate holds; every thread's earlier writes are seen after it.
+template <int Warps>
+__device__ __forceinline__ bool group_any(bool mine, int barrier) {
+    if constexpr (Warps == 1) {
+        const bool any = __any_sync(0xffffffffu, mine);
+        __syncwarp();
+        return any;
+    } else {
+        int any;
+        asm volatile("{\n .reg .pred p, q;\n setp.ne.s32 p, %1, 0;\n bar.red.or.pred q, %2, %3, p;\n"
+                     " selp.s32 %0, 1, 0, q;\n}"
+                     : "=r"(any)
+                     : "r"(static_cast<int>(mine)), "r"(barrier), "n"(Warps * kWarp)
+                     : "memory");
+        return any != 0;
+    }
+}
+
+// mat2pm_from_buffer (fast_principle_minors.h:120-246) for one matrix, by
+// Warps warps (lane is the thread's place among them). On return shifted[mask] (mask >= 1) holds the principal minor
 // of the rows/columns in mask. Returns true when a pivot sent the matrix to
 // the whole-matrix LU fallback (which this function then also runs). With
 // the compact layout (lay.arena > 0) the level lists live in shifted's arena
 // (compact_minors_layout), and each shifted minor is written once as p + its
 // pivot entry, the value the initialise-then-add form gives.
-__device__ bool mat2pm_warp(const double* A, int n, double tol, double shift_param,
-                            const WsLayout& lay, double* ws, double* shifted, double* lu_lane,
-                            int lane) {
+template <int Warps>
+__device__ bool mat2pm(const double* A, int n, double tol, double shift_param, const WsLayout& lay, double* ws,
+                       double* shifted, double* lu_lane, int lane, int barrier = 0) {
+    constexpr int kLanes = Warps * kWarp;
     const int msize = n * n;
     const uint32_t subsets = 1u << n;
-    const double max_abs = warp_max_abs(A, msize, lane);
+    const double max_abs = warp_max_abs(A, msize, lane & (kWarp - 1));
     const bool explicit_shift = !(shift_param < 0.0);
     const double p = explicit_shift ? shift_param : ddiv(max_abs, static_cast<double>(msize));
     if (max_abs == 0.0 && p == 0.0) {
-        for (uint32_t m = lane; m < subsets; m += kWarp) shifted[m] = 0.0;
-        __syncwarp();
+        for (uint32_t m = lane; m < subsets; m += kLanes) shifted[m] = 0.0;
+        group_sync<Warps>(barrier);
         return false;
     }
     const int64_t eps_bits = (tol > 0.0 && max_abs > 0.0) ? __double_as_longlong(dmul(tol, max_abs)) : 0LL;
@@ -177,18 +204,18 @@ __device__ bool mat2pm_warp(const double* A, int n, double tol, double shift_par
     // factors replace column 0 of rows 1.. (the children take only rows and
     // columns 1.., and the first minor has read the pivot entry already), so
     // the recursion needs no space besides its two lists.
-    const bool compact = lay.arena > 0;
+    const bool compact = Warps > 1 || lay.arena > 0;
     double* old_list = compact ? shifted + compact_list_offset(n, 0, lay.arena) : ws + lay.old_list;
     double* new_list = compact ? nullptr : ws + lay.new_list;
-    for (int k = lane; k < msize; k += kWarp) old_list[k] = A[k];
+    for (int k = lane; k < msize; k += kLanes) old_list[k] = A[k];
     if (compact) {
         if (lane == 0) shifted[0] = 1.0;
     } else {
-        for (uint32_t m = lane; m < subsets; m += kWarp) shifted[m] = m == 0 ? 1.0 : p;
+        for (uint32_t m = lane; m < subsets; m += kLanes) shifted[m] = m == 0 ? 1.0 : p;
     }
-    __syncwarp();
+    group_sync<Warps>(barrier);
     if (lane == 0) shifted[1] = dadd(compact ? p : shifted[1], old_list[0]);
-    __syncwarp();
+    group_sync<Warps>(barrier);
 
     uint32_t minor_index = 2;
     bool fell_back = false;
@@ -200,35 +227,34 @@ __device__ bool mat2pm_warp(const double* A, int n, double tol, double shift_par
         const int sets = 1 << level;
         // pivots of this level, one per set
         bool bad_pivot = false;
-        for (int set = lane; set < sets; set += kWarp) {
+        for (int set = lane; set < sets; set += kLanes) {
             // the pivot's entry plus p is already there as the node's shifted minor
             const double pivot = compact ? shifted[sets + set] : dadd(old_list[set * old_msize], p);
             bad_pivot |= pivot_too_small(pivot, eps_bits);
             old_list[set * old_msize] = soft_rcp(pivot);
         }
-        if (__any_sync(0xffffffffu, bad_pivot)) {
+        if (group_any<Warps>(bad_pivot, barrier)) {  // (also a barrier)
             fell_back = true;
             break;
         }
-        __syncwarp();
         // first-column factors, one per (set, row), in place of the column
-        for (int item = lane; item < sets * new_size; item += kWarp) {
+        for (int item = lane; item < sets * new_size; item += kLanes) {
             const int set = item / new_size;
             const int row = item - set * new_size;
             double* entry = old_list + set * old_msize + (row + 1) * old_size;
             *entry = dmul(*entry, old_list[set * old_msize]);
         }
-        __syncwarp();
+        group_sync<Warps>(barrier);
         if (compact) {
             if (level == n - 2) {
                 // the last level's 1 x 1 children, straight to their shifted minors
-                for (int set = lane; set < sets; set += kWarp) {
+                for (int set = lane; set < sets; set += kLanes) {
                     const double* m = old_list + set * 4;
                     const double base = m[3];
                     shifted[minor_index + set] = dadd(p, base);
                     shifted[minor_index + sets + set] = dadd(p, dfma(-m[1], m[2], base));
                 }
-                __syncwarp();
+                group_sync<Warps>(barrier);
                 minor_index += 2 * sets;
                 break;
             }
@@ -237,7 +263,7 @@ __device__ bool mat2pm_warp(const double* A, int n, double tol, double shift_par
         // submatrix without the pivot, and its Schur complement
         const int items = sets * new_msize;
 #pragma unroll 4
-        for (int item = lane; item < items; item += kWarp) {  // independent items, several in flight
+        for (int item = lane; item < items; item += kLanes) {  // independent items, several in flight
             const int set = item / new_msize;
             const int e = item - set * new_msize;
             const int row = e / new_size;
@@ -247,42 +273,46 @@ __device__ bool mat2pm_warp(const double* A, int n, double tol, double shift_par
             new_list[item] = base;
             new_list[items + item] = dfma(-old_list[src + 1 + col], old_list[src + (row + 1) * old_size], base);
         }
-        __syncwarp();
-        for (int m = lane; m < 2 * sets; m += kWarp)
+        group_sync<Warps>(barrier);
+        for (int m = lane; m < 2 * sets; m += kLanes)
             shifted[minor_index + m] = dadd(compact ? p : shifted[minor_index + m], new_list[m * new_msize]);
         minor_index += 2 * sets;
         double* t = old_list;
         old_list = new_list;
         new_list = t;
-        __syncwarp();
+        group_sync<Warps>(barrier);
     }
     if (fell_back) {
         // determinant_principal_minors_from_buffer (fast_principle_minors.h:107-115)
-        for (uint32_t m = 1 + lane; m < subsets; m += kWarp) shifted[m] = minor_by_lu(A, n, m, lu_lane);
-        __syncwarp();
+        // (one warp of the group: the LU scratch is one warp's)
+        if (lane < kWarp)
+            for (uint32_t m = 1 + lane; m < subsets; m += kWarp) shifted[m] = minor_by_lu(A, n, m, lu_lane);
+        group_sync<Warps>(barrier);
         return true;
     }
     // prefix product over levels
     for (uint32_t step = 1; step < subsets; step <<= 1) {
 #pragma unroll 4
-        for (uint32_t set = step + 1 + lane; set < 2 * step; set += kWarp)
+        for (uint32_t set = step + 1 + lane; set < 2 * step; set += kLanes)
             shifted[set] = dmul(shifted[set], shifted[set - step]);
-        __syncwarp();
+        group_sync<Warps>(barrier);
     }
     // remove the uniform shift by multilinearity
-    if (n >= 11 && n <= 14) {  // (at order 10 the unblocked loop on shared memory is faster)
-        remove_shift_blocked(shifted, n, p, lane);
-        return false;
+    if constexpr (Warps == 1) {
+        if (n >= 11 && n <= 14) {  // (at order 10 the unblocked loop on shared memory is faster)
+            remove_shift_blocked(shifted, n, p, lane);
+            return false;
+        }
     }
     for (uint32_t step = subsets; step > 1; step >>= 1) {
         const uint32_t half = step >> 1;
         const int hb = __ffs(half) - 1;  // half = 2^hb: the element's bit hb is set, its partner's clear
 #pragma unroll 4
-        for (uint32_t q = lane; q < subsets / 2; q += kWarp) {
+        for (uint32_t q = lane; q < subsets / 2; q += kLanes) {
             const uint32_t ss = ((q >> hb) << (hb + 1)) + half + (q & (half - 1u));
             shifted[ss] = dfma(-p, shifted[ss - half], shifted[ss]);
         }
-        __syncwarp();
+        group_sync<Warps>(barrier);
     }
     return false;
 }
@@ -319,7 +349,7 @@ __host__ __device__ inline ChunkGeom chunk_geom(int n) {
 constexpr int kChunkMinOrder = 11, kChunkMaxOrder = 14;
 
 // The FP64 minors' workspace of a batch of orders up to nmax: the aux region
-// only where the chunked recursion can run (mat2pm_warp needs none).
+// only where the chunked recursion can run (mat2pm needs none).
 __host__ __device__ inline WsLayout fp64_minors_layout(int nmax, bool two_spins) {
     return ws_layout(nmax, two_spins, nmax >= kChunkMinOrder);
 }
@@ -415,7 +445,7 @@ __device__ __forceinline__ void prefix_product_global(double* shifted, uint32_t 
     }
 }
 
-// mat2pm_warp for orders 11..14 with the chunked recursion: the top levels'
+// mat2pm for orders 11..14 with the chunked recursion: the top levels'
 // lists in the global workspace ws, the chunks' in `chunk` (shared memory,
 // chunk_geom(n).doubles()), the shifted minors in global memory.
 __device__ bool mat2pm_chunked(const double* A, int n, double tol, double shift_param, const WsLayout& lay,
@@ -477,12 +507,88 @@ __device__ bool mat2pm_chunked(const double* A, int n, double tol, double shift_
     return false;
 }
 
-// use_smem: 1 = the whole workspace in shared memory; 0 = in the global
-// workspace; 2 = chunked (orders 11..14): lists of the chunks in shared
-// memory, the top levels' lists and the shifted minors in the global workspace.
-__global__ void __launch_bounds__(384) principal_minors_fp64(const __grid_constant__ Problem p,
-                                                            const __grid_constant__ Scratch w,
-                                                            int use_smem) {
+// The minors of one (configuration, set) and the products a[mask] = up[mask-1]
+// * down[mask-1] (integrand_replica_randomly_sampled.h:254-257), by Warps
+// warps: minors(A, n, shifted) computes one spin's.
+template <int Warps, class Minors>
+__device__ __forceinline__ void minors_item(const Problem& p, const Scratch& w, int64_t c, int set, int n,
+                                            const WsLayout& lay, double* ws, int lane, int barrier, Minors minors) {
+    constexpr int kLanes = Warps * kWarp;
+    const int nmax = p.max_order;
+    const uint32_t full = 1u << nmax;
+    const double* green = w.green + (c * 2 + set) * 2 * static_cast<int64_t>(nmax) * nmax;
+    bool fb = false;
+    const bool one_spin = p.same_spin[set] != 0;
+    if (Warps > 1 || lay.arena > 0) {
+        fb |= minors(green, n, ws + lay.shifted_up);
+        if (!one_spin) fb |= minors(green + static_cast<int64_t>(nmax) * nmax, n, ws + lay.shifted_down);
+    } else {
+        double* A = ws + lay.a;
+        for (int k = lane; k < n * n; k += kWarp) A[k] = green[k];
+        __syncwarp();
+        fb |= minors(A, n, ws + lay.shifted_up);
+        if (!one_spin) {
+            for (int k = lane; k < n * n; k += kWarp) A[k] = green[static_cast<int64_t>(nmax) * nmax + k];
+            __syncwarp();
+            fb |= minors(A, n, ws + lay.shifted_down);
+        }
+    }
+    const double* su = ws + lay.shifted_up;
+    const double* sd = one_spin ? su : ws + lay.shifted_down;
+    const int64_t slot = p.sorted ? __ldg(w.slot_of + c) : c;  // lane-interleaved position
+    double* a = w.a_int + ((slot >> 5) * 2 + set) * static_cast<int64_t>(full) * kWarp + (slot & 31);
+    for (uint32_t m0 = 0; m0 < (1u << n); m0 += 8 * kLanes) {  // eight products per lane in flight
+        double x[8], y[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const uint32_t m = m0 + u * kLanes + lane;
+            x[u] = m < (1u << n) ? su[m] : 0.0;
+            y[u] = m < (1u << n) ? sd[m] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const uint32_t m = m0 + u * kLanes + lane;
+            if (m < (1u << n)) a[static_cast<int64_t>(m) * kWarp] = m == 0 ? 0.0 : dmul(x[u], y[u]);
+        }
+    }
+    if (fb && lane == 0) atomicOr(p.status + c, kStatusFpmFallback);
+    group_sync<Warps>(barrier);
+}
+
+// Orders up to 10: Warps warps per (configuration, set), the compact workspace
+// in shared memory. Eleven workspaces of order 10 fill an SM, and one warp each
+// kept its FP64 pipe 64 % busy (2.8 warps per scheduler, waiting on shared
+// memory and on dependent operations); two each: 65,536 order-10
+// configurations 4.48 -> 4.05 ms.
+template <int Warps>
+__global__ void __launch_bounds__(1024) principal_minors_shared(const __grid_constant__ Problem p,
+                                                               const __grid_constant__ Scratch w) {
+    extern __shared__ double smem[];
+    const int lane = threadIdx.x & (Warps * kWarp - 1);
+    const int group = threadIdx.x / (Warps * kWarp);
+    const int groups = blockDim.x / (Warps * kWarp);
+    const int64_t global_group = static_cast<int64_t>(blockIdx.x) * groups + group;
+    const int64_t total_groups = static_cast<int64_t>(gridDim.x) * groups;
+    const int nmax = p.max_order;
+    const WsLayout lay = compact_minors_layout(nmax, !(p.same_spin[0] && p.same_spin[1]));
+    double* ws = smem + static_cast<size_t>(group) * lay.total;
+    double* lu_lane = w.lu_scratch + (static_cast<size_t>(global_group) * kWarp + (lane & (kWarp - 1))) * nmax * nmax;
+    auto minors = [&](const double* A, int n, double* shifted) {
+        return mat2pm<Warps>(A, n, p.s.tol_fpm, p.s.fpm_shift, lay, ws, shifted, lu_lane, lane, group);
+    };
+    for (int64_t item = global_group; item < p.batch * 2; item += total_groups) {
+        const int64_t c = item >> 1;
+        const int n = p.all_subsets ? nmax : __ldg(p.orders + c);
+        if (n < 2 || n > nmax) continue;  // order 1 needs no minors; bad orders are flagged by step 1
+        minors_item<Warps>(p, w, c, static_cast<int>(item & 1), n, lay, ws, lane, group, minors);
+    }
+}
+
+// The other orders: a warp per (configuration, set), the workspace in global
+// memory; chunked (orders 11..14): lists of the chunks in shared memory, the
+// top levels' lists and the shifted minors in the global workspace.
+__global__ void __launch_bounds__(256) principal_minors_fp64(const __grid_constant__ Problem p,
+                                                            const __grid_constant__ Scratch w, bool chunked) {
     extern __shared__ double smem[];
     const int lane = threadIdx.x & (kWarp - 1);
     const int warp_in_block = threadIdx.x / kWarp;
@@ -490,63 +596,20 @@ __global__ void __launch_bounds__(384) principal_minors_fp64(const __grid_consta
     const int64_t global_warp = static_cast<int64_t>(blockIdx.x) * warps_per_block + warp_in_block;
     const int64_t total_warps = static_cast<int64_t>(gridDim.x) * warps_per_block;
     const int nmax = p.max_order;
-    // the global workspace is laid out for two spins; shared memory for what
-    // the sets need, compact up to order 10 (A then read from the Green matrices)
-    const WsLayout lay = minors_layout(nmax, use_smem != 1 || !(p.same_spin[0] && p.same_spin[1]), use_smem == 1);
-    double* ws = use_smem == 1 ? smem + static_cast<size_t>(warp_in_block) * lay.total
-                               : w.ws_global + static_cast<size_t>(global_warp) * lay.total;
+    const WsLayout lay = fp64_minors_layout(nmax, true);
+    double* ws = w.ws_global + static_cast<size_t>(global_warp) * lay.total;
     double* lu_lane = w.lu_scratch + (static_cast<size_t>(global_warp) * kWarp + lane) * nmax * nmax;
-    double* chunk = use_smem == 2 ? smem + static_cast<size_t>(warp_in_block) * chunk_doubles_upto(nmax) : nullptr;
+    double* chunk = smem + static_cast<size_t>(warp_in_block) * chunk_doubles_upto(nmax);
     auto minors = [&](const double* A, int n, double* shifted) {
-        return (chunk && n >= kChunkMinOrder && n <= kChunkMaxOrder)
+        return (chunked && n >= kChunkMinOrder && n <= kChunkMaxOrder)
                    ? mat2pm_chunked(A, n, p.s.tol_fpm, p.s.fpm_shift, lay, ws, shifted, lu_lane, chunk, lane)
-                   : mat2pm_warp(A, n, p.s.tol_fpm, p.s.fpm_shift, lay, ws, shifted, lu_lane, lane);
+                   : mat2pm<1>(A, n, p.s.tol_fpm, p.s.fpm_shift, lay, ws, shifted, lu_lane, lane);
     };
-    const uint32_t full = 1u << nmax;
-    const int64_t items = p.batch * 2;
-    for (int64_t item = global_warp; item < items; item += total_warps) {
+    for (int64_t item = global_warp; item < p.batch * 2; item += total_warps) {
         const int64_t c = item >> 1;
-        const int set = static_cast<int>(item & 1);
         const int n = p.all_subsets ? nmax : __ldg(p.orders + c);
         if (n < 2 || n > nmax) continue;  // order 1 needs no minors; bad orders are flagged by step 1
-        const double* green = w.green + (c * 2 + set) * 2 * static_cast<int64_t>(nmax) * nmax;
-        bool fb = false;
-        const bool one_spin = p.same_spin[set] != 0;
-        if (lay.arena > 0) {
-            fb |= minors(green, n, ws + lay.shifted_up);
-            if (!one_spin) fb |= minors(green + static_cast<int64_t>(nmax) * nmax, n, ws + lay.shifted_down);
-        } else {
-            double* A = ws + lay.a;
-            for (int k = lane; k < n * n; k += kWarp) A[k] = green[k];
-            __syncwarp();
-            fb |= minors(A, n, ws + lay.shifted_up);
-            if (!one_spin) {
-                for (int k = lane; k < n * n; k += kWarp) A[k] = green[static_cast<int64_t>(nmax) * nmax + k];
-                __syncwarp();
-                fb |= minors(A, n, ws + lay.shifted_down);
-            }
-        }
-        const double* su = ws + lay.shifted_up;
-        const double* sd = one_spin ? su : ws + lay.shifted_down;
-        // a[mask] = up[mask-1] * down[mask-1] (integrand_replica_randomly_sampled.h:254-257)
-        const int64_t slot = p.sorted ? __ldg(w.slot_of + c) : c;  // lane-interleaved position
-        double* a = w.a_int + ((slot >> 5) * 2 + set) * static_cast<int64_t>(full) * kWarp + (slot & 31);
-        for (uint32_t m0 = 0; m0 < (1u << n); m0 += 8 * kWarp) {  // eight products per lane in flight
-            double x[8], y[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const uint32_t m = m0 + u * kWarp + lane;
-                x[u] = m < (1u << n) ? su[m] : 0.0;
-                y[u] = m < (1u << n) ? sd[m] : 0.0;
-            }
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const uint32_t m = m0 + u * kWarp + lane;
-                if (m < (1u << n)) a[static_cast<int64_t>(m) * kWarp] = m == 0 ? 0.0 : dmul(x[u], y[u]);
-            }
-        }
-        if (fb && lane == 0) atomicOr(p.status + c, kStatusFpmFallback);
-        __syncwarp();
+        minors_item<1>(p, w, c, static_cast<int>(item & 1), n, lay, ws, lane, 0, minors);
     }
 }
 
@@ -1379,7 +1442,7 @@ __global__ void __launch_bounds__(128) combine_sets(const __grid_constant__ Prob
 // minors in place, a of the even masks and dp of the odd ones take the two
 // list regions (each holds at least 2^(n-1) doubles: the last Schur level has
 // 2^(n-1) lists of one entry). Every set goes through the staged form's
-// operations (mat2pm_warp, a = up * down, split_cdet_recursion or the
+// operations (mat2pm, a = up * down, split_cdet_recursion or the
 // reference's descending submask sums), so the values are the staged form's
 // bit for bit.
 
@@ -1449,7 +1512,7 @@ __device__ __forceinline__ DD queue_set_value(const Problem& p, const Scratch& w
         __syncwarp();
     }
     double* su = ws + lay.shifted_up;
-    fb |= mat2pm_warp(compact ? green : A, n, s.tol_fpm, s.fpm_shift, lay, ws, su, lu_lane, lane);
+    fb |= mat2pm<1>(compact ? green : A, n, s.tol_fpm, s.fpm_shift, lay, ws, su, lu_lane, lane);
     const bool one_spin = p.same_spin[set] != 0;
     if (!one_spin) {
         const double* green_down = green + static_cast<int64_t>(nmax) * nmax;
@@ -1457,7 +1520,7 @@ __device__ __forceinline__ DD queue_set_value(const Problem& p, const Scratch& w
             for (int k = lane; k < n * n; k += kWarp) A[k] = green_down[k];
             __syncwarp();
         }
-        fb |= mat2pm_warp(compact ? green_down : A, n, s.tol_fpm, s.fpm_shift, lay, ws, ws + lay.shifted_down,
+        fb |= mat2pm<1>(compact ? green_down : A, n, s.tol_fpm, s.fpm_shift, lay, ws, ws + lay.shifted_down,
                           lu_lane, lane);
     }
     const double* sd = one_spin ? su : ws + lay.shifted_down;
@@ -1745,40 +1808,46 @@ static cudaError_t post_assembly(const Problem& p_in, const Scratch& w, int sm_c
         return cudaSuccess;
     }
 
-    // Minors: the per-warp workspace goes to shared memory when at least four
-    // warps' worth fits a block (one block per SM, as many warps as fit, at
-    // most 16; the compact arena up to order 10; without the spin-down minors
-    // when both sets have one spin), otherwise to the global workspace (4
-    // warps per block).
+    // Minors: the workspace of a (configuration, set) goes to shared memory
+    // when at least four fit a block (one block per SM, as many as fit, at most
+    // 16; the compact arena up to order 10; without the spin-down minors when
+    // both sets have one spin), otherwise to the global workspace (4 warps per
+    // block).
     const bool two_spins = !(p.same_spin[0] && p.same_spin[1]);
     const size_t ws_bytes = minors_layout(p.max_order, two_spins, true).total * sizeof(double);
     const int fit = minors_warps_in_shared_memory(p.max_order, two_spins);
-    const bool use_smem = fit >= 4;
+    const bool use_smem = fit >= 4;  // (the compact arena only: order 11 fits three)
     // orders 11..14 in the global workspace: the chunked recursion, eight
     // warps per block, as many blocks per SM as their chunk buffers allow
     const bool chunked = !use_smem && p.max_order >= kChunkMinOrder && p.max_order <= kChunkMaxOrder;
     const size_t chunk_bytes = chunked ? chunk_doubles_upto(p.max_order) * sizeof(double) : 0;
     const int64_t items = p.batch * 2;
     const int sms = sm_count > 0 ? sm_count : 152;
-    // (a batch of fewer warps than the SMs hold spreads over all of them: warps of one SM share its FP64 pipe)
+    // (a batch of fewer workspaces than the SMs hold spreads over all of them: warps of one SM share its FP64 pipe)
     const int most = use_smem ? fit : (chunked ? 8 : 4);
-    const int warps_per_block = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(most, (items + sms - 1) / sms)));
-    int64_t blocks = (items + warps_per_block - 1) / warps_per_block;
-    const int64_t max_blocks = static_cast<int64_t>(w.ws_warps) / warps_per_block;
+    const int per_block = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(most, (items + sms - 1) / sms)));
+    int64_t blocks = (items + per_block - 1) / per_block;
+    const int64_t max_blocks = static_cast<int64_t>(w.ws_warps) / per_block;
     blocks = std::min<int64_t>(blocks, std::max<int64_t>(1, max_blocks));
     if (use_smem) blocks = std::min<int64_t>(blocks, sms);  // one wave
     if (chunked) {
-        const int64_t per_sm = std::max<int64_t>(1, (227 * 1024) / (chunk_bytes * warps_per_block + 1024));
+        const int64_t per_sm = std::max<int64_t>(1, (227 * 1024) / (chunk_bytes * per_block + 1024));
         blocks = std::min<int64_t>(blocks, per_sm * sms);  // one wave
     }
-    const size_t smem = use_smem ? ws_bytes * warps_per_block : chunk_bytes * warps_per_block;
+    const size_t smem = use_smem ? ws_bytes * per_block : chunk_bytes * per_block;
+    // an SM whose workspaces leave it few warps: four or two of them share one
+    const int warps = !use_smem ? 1 : per_block <= 7 ? 4 : 2;
+    const void* kernel = !use_smem   ? reinterpret_cast<const void*>(principal_minors_fp64)
+                         : warps > 2 ? reinterpret_cast<const void*>(principal_minors_shared<4>)
+                                     : reinterpret_cast<const void*>(principal_minors_shared<2>);
     if (smem > 48 * 1024) {
-        err = cudaFuncSetAttribute(principal_minors_fp64, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(smem));
+        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (err != cudaSuccess) return err;
     }
-    principal_minors_fp64<<<static_cast<unsigned>(blocks), warps_per_block * kWarp, smem, stream>>>(
-        p, w, use_smem ? 1 : (chunked ? 2 : 0));
+    const unsigned grid = static_cast<unsigned>(blocks), width = static_cast<unsigned>(per_block * warps * kWarp);
+    if (!use_smem) principal_minors_fp64<<<grid, width, smem, stream>>>(p, w, chunked);
+    else if (warps > 2) principal_minors_shared<4><<<grid, width, smem, stream>>>(p, w);
+    else principal_minors_shared<2><<<grid, width, smem, stream>>>(p, w);
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     mark(3);
