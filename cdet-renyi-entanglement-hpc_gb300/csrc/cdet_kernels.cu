@@ -3,9 +3,9 @@
 // After the Green matrices (cdet_assembly.cu or cdet_split.cu), two launches
 // per batch of vertex configurations:
 //
-//  1. principal_minors_shared (two or four warps per (configuration, table set))
-//     or, above order 10, principal_minors_fp64 (one warp). The
-//     warp runs the shifted Schur-complement recursion of mat2pm level by
+//  1. principal_minors_shared (two or four warps per (configuration, table
+//     set)) or, above order 10, principal_minors_fp64 (one or two). The group
+//     runs the shifted Schur-complement recursion of mat2pm level by
 //     level, lanes spread over (set, row, column) work items, then the prefix
 //     product and the shift removal, and writes a[mask] = pm_up * pm_down into
 //     a lane-interleaved array for step 2.
@@ -74,84 +74,6 @@ __device__ double minor_by_lu(const double* a, int n, uint32_t mask, double* m) 
     return sign < 0 ? -det : det;
 }
 
-// The shift removal of mat2pm (fast_principle_minors.h:230-243) for
-// 2^11..2^14 minors, blocked so that each value is read and written twice
-// instead of once per bit: first the bits above 9, a column of 2^(n-10)
-// values per lane in registers, then bits 9..0 on chunks of 1,024 values (32
-// per lane; bits 5..9 between a lane's registers, bits 0..4 across lanes by
-// shuffles). Every value takes the same fma(-p, partner, value) updates in
-// the same (descending-bit) order as the unblocked loop, so the minors are
-// bit for bit the same.
-template <int HighBits>
-__device__ __forceinline__ void remove_shift_high(double* shifted, double p, int lane) {
-    constexpr int kCount = 1 << HighBits;
-    for (uint32_t c = lane; c < 1024u; c += kWarp) {
-        double r[kCount];
-#pragma unroll
-        for (int k = 0; k < kCount; ++k) r[k] = shifted[c + 1024u * k];
-#pragma unroll
-        for (int b = HighBits - 1; b >= 0; --b)
-#pragma unroll
-            for (int k = 0; k < kCount; ++k)
-                if (k & (1 << b)) r[k] = dfma(-p, r[k ^ (1 << b)], r[k]);
-#pragma unroll
-        for (int k = 0; k < kCount; ++k) shifted[c + 1024u * k] = r[k];
-    }
-}
-
-__device__ __forceinline__ void remove_shift_blocked(double* shifted, int n, double p, int lane) {
-    switch (n) {  // n = 11..14
-        case 11: remove_shift_high<1>(shifted, p, lane); break;
-        case 12: remove_shift_high<2>(shifted, p, lane); break;
-        case 13: remove_shift_high<3>(shifted, p, lane); break;
-        case 14: remove_shift_high<4>(shifted, p, lane); break;
-        default: break;
-    }
-    __syncwarp();
-    const uint32_t subsets = 1u << n;
-    for (uint32_t h = 0; h < subsets; h += 1024u) {
-        double r[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) r[j] = shifted[h + lane + kWarp * j];
-#pragma unroll
-        for (int b = 4; b >= 0; --b)  // bits 9..5: between registers
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-                if (j & (1 << b)) r[j] = dfma(-p, r[j ^ (1 << b)], r[j]);
-#pragma unroll
-        for (int b = 4; b >= 0; --b) {  // bits 4..0: across lanes
-            const int m = 1 << b;
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                const double v = __shfl_xor_sync(0xffffffffu, r[j], m);
-                if (lane & m) r[j] = dfma(-p, v, r[j]);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 32; ++j) shifted[h + lane + kWarp * j] = r[j];
-    }
-    __syncwarp();
-}
-
-// The largest |A[k]| of a matrix that is no NaN (0 if none), by a whole warp,
-// compared as integers: like the pivots' test and reciprocal below, work that
-// the FP64 pipe, which bounds the minors, need not do (65,536 order-10
-// configurations, split assembly: minors 5.13 -> 4.48 ms for the three).
-__device__ __forceinline__ double warp_max_abs(const double* A, int msize, int lane) {
-    int64_t best = 0;
-    for (int k = lane; k < msize; k += kWarp) {
-        const int64_t e = __double_as_longlong(A[k]) & 0x7FFFFFFFFFFFFFFFLL;
-        if (e > best && e <= 0x7FF0000000000000LL) best = e;
-    }
-    for (int off = 16; off > 0; off >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, off));
-    return __longlong_as_double(best);
-}
-
-// |pivot| is zero, or at most eps >= 0, given as its bits.
-__device__ __forceinline__ bool pivot_too_small(double pivot, int64_t eps_bits) {
-    return (__double_as_longlong(pivot) & 0x7FFFFFFFFFFFFFFFLL) <= eps_bits;
-}
-
 // The threads of one matrix: a warp, or Warps of them that meet at a named barrier.
 template <int Warps>
 __device__ __forceinline__ void group_sync(int barrier) {
@@ -175,6 +97,86 @@ __device__ __forceinline__ bool group_any(bool mine, int barrier) {
                      : "memory");
         return any != 0;
     }
+}
+
+// The shift removal of mat2pm (fast_principle_minors.h:230-243) for
+// 2^11..2^14 minors, blocked so that each value is read and written twice
+// instead of once per bit: first the bits above 9, a column of 2^(n-10)
+// values per lane in registers, then bits 9..0 on chunks of 1,024 values (32
+// per lane; bits 5..9 between a lane's registers, bits 0..4 across lanes by
+// shuffles). Every value takes the same fma(-p, partner, value) updates in
+// the same (descending-bit) order as the unblocked loop, so the minors are
+// bit for bit the same.
+template <int HighBits, int Warps>
+__device__ __forceinline__ void remove_shift_high(double* shifted, double p, int lane) {
+    constexpr int kCount = 1 << HighBits;
+    for (uint32_t c = lane; c < 1024u; c += Warps * kWarp) {
+        double r[kCount];
+#pragma unroll
+        for (int k = 0; k < kCount; ++k) r[k] = shifted[c + 1024u * k];
+#pragma unroll
+        for (int b = HighBits - 1; b >= 0; --b)
+#pragma unroll
+            for (int k = 0; k < kCount; ++k)
+                if (k & (1 << b)) r[k] = dfma(-p, r[k ^ (1 << b)], r[k]);
+#pragma unroll
+        for (int k = 0; k < kCount; ++k) shifted[c + 1024u * k] = r[k];
+    }
+}
+
+template <int Warps>
+__device__ __forceinline__ void remove_shift_blocked(double* shifted, int n, double p, int lane, int barrier) {
+    switch (n) {  // n = 11..14
+        case 11: remove_shift_high<1, Warps>(shifted, p, lane); break;
+        case 12: remove_shift_high<2, Warps>(shifted, p, lane); break;
+        case 13: remove_shift_high<3, Warps>(shifted, p, lane); break;
+        case 14: remove_shift_high<4, Warps>(shifted, p, lane); break;
+        default: break;
+    }
+    group_sync<Warps>(barrier);
+    const uint32_t subsets = 1u << n;
+    const int warp_lane = lane & (kWarp - 1);
+    for (uint32_t h = 1024u * (lane / kWarp); h < subsets; h += 1024u * Warps) {
+        double r[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) r[j] = shifted[h + warp_lane + kWarp * j];
+#pragma unroll
+        for (int b = 4; b >= 0; --b)  // bits 9..5: between registers
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+                if (j & (1 << b)) r[j] = dfma(-p, r[j ^ (1 << b)], r[j]);
+#pragma unroll
+        for (int b = 4; b >= 0; --b) {  // bits 4..0: across lanes
+            const int m = 1 << b;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+                const double v = __shfl_xor_sync(0xffffffffu, r[j], m);
+                if (warp_lane & m) r[j] = dfma(-p, v, r[j]);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 32; ++j) shifted[h + warp_lane + kWarp * j] = r[j];
+    }
+    group_sync<Warps>(barrier);
+}
+
+// The largest |A[k]| of a matrix that is no NaN (0 if none), by a whole warp,
+// compared as integers: like the pivots' test and reciprocal below, work that
+// the FP64 pipe, which bounds the minors, need not do (65,536 order-10
+// configurations, split assembly: minors 5.13 -> 4.48 ms for the three).
+__device__ __forceinline__ double warp_max_abs(const double* A, int msize, int lane) {
+    int64_t best = 0;
+    for (int k = lane; k < msize; k += kWarp) {
+        const int64_t e = __double_as_longlong(A[k]) & 0x7FFFFFFFFFFFFFFFLL;
+        if (e > best && e <= 0x7FF0000000000000LL) best = e;
+    }
+    for (int off = 16; off > 0; off >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, off));
+    return __longlong_as_double(best);
+}
+
+// |pivot| is zero, or at most eps >= 0, given as its bits.
+__device__ __forceinline__ bool pivot_too_small(double pivot, int64_t eps_bits) {
+    return (__double_as_longlong(pivot) & 0x7FFFFFFFFFFFFFFFLL) <= eps_bits;
 }
 
 // mat2pm_from_buffer (fast_principle_minors.h:120-246) for one matrix, by
@@ -204,7 +206,7 @@ __device__ bool mat2pm(const double* A, int n, double tol, double shift_param, c
     // factors replace column 0 of rows 1.. (the children take only rows and
     // columns 1.., and the first minor has read the pivot entry already), so
     // the recursion needs no space besides its two lists.
-    const bool compact = Warps > 1 || lay.arena > 0;
+    const bool compact = lay.arena > 0;
     double* old_list = compact ? shifted + compact_list_offset(n, 0, lay.arena) : ws + lay.old_list;
     double* new_list = compact ? nullptr : ws + lay.new_list;
     for (int k = lane; k < msize; k += kLanes) old_list[k] = A[k];
@@ -300,7 +302,7 @@ __device__ bool mat2pm(const double* A, int n, double tol, double shift_param, c
     // remove the uniform shift by multilinearity
     if constexpr (Warps == 1) {
         if (n >= 11 && n <= 14) {  // (at order 10 the unblocked loop on shared memory is faster)
-            remove_shift_blocked(shifted, n, p, lane);
+            remove_shift_blocked<1>(shifted, n, p, lane, barrier);
             return false;
         }
     }
@@ -378,29 +380,30 @@ __host__ __device__ inline int chunk_doubles_upto(int nmax) {
 // Returns false when a pivot sends the matrix to the LU fallback. Each
 // shifted minor receives exactly one addition, p + the child's pivot entry,
 // written directly (the whole-level form adds it to the p it initialised).
+template <int Warps>
 __device__ bool schur_level(const double* old_list, double* new_list, double* inv, int nodes, int old_size,
                             double p, int64_t eps_bits, double* shifted, uint32_t base, uint32_t c0,
-                            int log2g, int T, int lane) {
+                            int log2g, int T, int lane, int barrier) {
+    constexpr int kLanes = Warps * kWarp;
     const int old_msize = old_size * old_size;
     const int new_size = old_size - 1;
     const int new_msize = new_size * new_size;
     bool bad_pivot = false;
-    for (int set = lane; set < nodes; set += kWarp) {
+    for (int set = lane; set < nodes; set += kLanes) {
         const double pivot = dadd(old_list[set * old_msize], p);
         bad_pivot |= pivot_too_small(pivot, eps_bits);
         inv[set] = soft_rcp(pivot);
     }
-    if (__any_sync(0xffffffffu, bad_pivot)) return false;
-    __syncwarp();
+    if (group_any<Warps>(bad_pivot, barrier)) return false;  // (also a barrier)
     double* factor = inv + nodes;
-    for (int item = lane; item < nodes * new_size; item += kWarp) {
+    for (int item = lane; item < nodes * new_size; item += kLanes) {
         const int set = item / new_size;
         const int row = item - set * new_size;
         factor[item] = dmul(old_list[set * old_msize + (row + 1) * old_size], inv[set]);
     }
-    __syncwarp();
+    group_sync<Warps>(barrier);
     const int items = nodes * new_msize;
-    for (int item = lane; item < items; item += kWarp) {
+    for (int item = lane; item < items; item += kLanes) {
         const int set = item / new_msize;
         const int e = item - set * new_msize;
         const int row = e / new_size;
@@ -410,72 +413,76 @@ __device__ bool schur_level(const double* old_list, double* new_list, double* in
         new_list[item] = b;
         new_list[items + item] = dfma(-old_list[src + 1 + col], factor[set * new_size + row], b);
     }
-    __syncwarp();
+    group_sync<Warps>(barrier);
     const uint32_t gmask = (1u << log2g) - 1u;
-    for (int q = lane; q < 2 * nodes; q += kWarp) {
+    for (int q = lane; q < 2 * nodes; q += kLanes) {
         const uint32_t idx = base + c0 + (static_cast<uint32_t>(q) & gmask) +
                              ((static_cast<uint32_t>(q) >> log2g) << T);
         shifted[idx] = dadd(p, new_list[q * new_msize]);
     }
-    __syncwarp();
+    group_sync<Warps>(barrier);
     return true;
 }
 
 // The prefix product of mat2pm (fast_principle_minors.h:217-228) on a global
 // array: shifted[step + 1 + t] *= shifted[1 + t], eight elements per lane in
 // flight.
-__device__ __forceinline__ void prefix_product_global(double* shifted, uint32_t subsets, int lane) {
+template <int Warps>
+__device__ __forceinline__ void prefix_product_global(double* shifted, uint32_t subsets, int lane, int barrier) {
+    constexpr int kLanes = Warps * kWarp;
     for (uint32_t step = 2; step < subsets; step <<= 1) {
         const uint32_t count = step - 1;
-        for (uint32_t t0 = 0; t0 < count; t0 += 8 * kWarp) {
+        for (uint32_t t0 = 0; t0 < count; t0 += 8 * kLanes) {
             double x[8], y[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-                const uint32_t t = t0 + u * kWarp + lane;
+                const uint32_t t = t0 + u * kLanes + lane;
                 x[u] = t < count ? shifted[step + 1 + t] : 0.0;
                 y[u] = t < count ? shifted[1 + t] : 0.0;
             }
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-                const uint32_t t = t0 + u * kWarp + lane;
+                const uint32_t t = t0 + u * kLanes + lane;
                 if (t < count) shifted[step + 1 + t] = dmul(x[u], y[u]);
             }
         }
-        __syncwarp();
+        group_sync<Warps>(barrier);
     }
 }
 
 // mat2pm for orders 11..14 with the chunked recursion: the top levels'
 // lists in the global workspace ws, the chunks' in `chunk` (shared memory,
 // chunk_geom(n).doubles()), the shifted minors in global memory.
+template <int Warps>
 __device__ bool mat2pm_chunked(const double* A, int n, double tol, double shift_param, const WsLayout& lay,
-                               double* ws, double* shifted, double* lu_lane, double* chunk, int lane) {
+                               double* ws, double* shifted, double* lu_lane, double* chunk, int lane, int barrier) {
+    constexpr int kLanes = Warps * kWarp;
     const int msize = n * n;
     const uint32_t subsets = 1u << n;
-    const double max_abs = warp_max_abs(A, msize, lane);
+    const double max_abs = warp_max_abs(A, msize, lane & (kWarp - 1));
     const bool explicit_shift = !(shift_param < 0.0);
     const double p = explicit_shift ? shift_param : ddiv(max_abs, static_cast<double>(msize));
     if (max_abs == 0.0 && p == 0.0) {
-        for (uint32_t m = lane; m < subsets; m += kWarp) shifted[m] = 0.0;
-        __syncwarp();
+        for (uint32_t m = lane; m < subsets; m += kLanes) shifted[m] = 0.0;
+        group_sync<Warps>(barrier);
         return false;
     }
     const int64_t eps_bits = (tol > 0.0 && max_abs > 0.0) ? __double_as_longlong(dmul(tol, max_abs)) : 0LL;
     double* old_list = ws + lay.old_list;
     double* new_list = ws + lay.new_list;
     double* inv = ws + lay.aux;
-    for (int k = lane; k < msize; k += kWarp) old_list[k] = A[k];
+    for (int k = lane; k < msize; k += kLanes) old_list[k] = A[k];
     // every shifted minor from 2 on is written once by its node below
     if (lane == 0) {
         shifted[0] = 1.0;
         shifted[1] = dadd(p, A[0]);
     }
-    __syncwarp();
+    group_sync<Warps>(barrier);
     const ChunkGeom g = chunk_geom(n);
     bool ok = true;
     for (int level = 0; level < g.T && ok; ++level) {
-        ok = schur_level(old_list, new_list, inv, 1 << level, n - level, p, eps_bits, shifted,
-                         2u << level, 0u, 30, 0, lane);
+        ok = schur_level<Warps>(old_list, new_list, inv, 1 << level, n - level, p, eps_bits, shifted,
+                         2u << level, 0u, 30, 0, lane, barrier);
         double* t = old_list;
         old_list = new_list;
         new_list = t;
@@ -486,11 +493,11 @@ __device__ bool mat2pm_chunked(const double* A, int n, double tol, double shift_
         double* co = chunk;
         double* cn = chunk + g.list;
         double* caux = chunk + 2 * g.list;
-        for (int k = lane; k < G * msz; k += kWarp) co[k] = old_list[c0 * msz + k];
-        __syncwarp();
+        for (int k = lane; k < G * msz; k += kLanes) co[k] = old_list[c0 * msz + k];
+        group_sync<Warps>(barrier);
         for (int j = 0; j + 1 < m && ok; ++j) {
-            ok = schur_level(co, cn, caux, G << j, m - j, p, eps_bits, shifted, 2u << (g.T + j), c0,
-                             g.log2g, g.T, lane);
+            ok = schur_level<Warps>(co, cn, caux, G << j, m - j, p, eps_bits, shifted, 2u << (g.T + j), c0,
+                             g.log2g, g.T, lane, barrier);
             double* t = co;
             co = cn;
             cn = t;
@@ -498,12 +505,14 @@ __device__ bool mat2pm_chunked(const double* A, int n, double tol, double shift_
     }
     if (!ok) {
         // determinant_principal_minors_from_buffer (fast_principle_minors.h:107-115)
-        for (uint32_t mk = 1 + lane; mk < subsets; mk += kWarp) shifted[mk] = minor_by_lu(A, n, mk, lu_lane);
-        __syncwarp();
+        // (one warp of the group: the LU scratch is one warp's)
+        if (lane < kWarp)
+            for (uint32_t mk = 1 + lane; mk < subsets; mk += kWarp) shifted[mk] = minor_by_lu(A, n, mk, lu_lane);
+        group_sync<Warps>(barrier);
         return true;
     }
-    prefix_product_global(shifted, subsets, lane);
-    remove_shift_blocked(shifted, n, p, lane);
+    prefix_product_global<Warps>(shifted, subsets, lane, barrier);
+    remove_shift_blocked<Warps>(shifted, n, p, lane, barrier);
     return false;
 }
 
@@ -519,17 +528,17 @@ __device__ __forceinline__ void minors_item(const Problem& p, const Scratch& w, 
     const double* green = w.green + (c * 2 + set) * 2 * static_cast<int64_t>(nmax) * nmax;
     bool fb = false;
     const bool one_spin = p.same_spin[set] != 0;
-    if (Warps > 1 || lay.arena > 0) {
+    if (lay.arena > 0) {
         fb |= minors(green, n, ws + lay.shifted_up);
         if (!one_spin) fb |= minors(green + static_cast<int64_t>(nmax) * nmax, n, ws + lay.shifted_down);
     } else {
         double* A = ws + lay.a;
-        for (int k = lane; k < n * n; k += kWarp) A[k] = green[k];
-        __syncwarp();
+        for (int k = lane; k < n * n; k += kLanes) A[k] = green[k];
+        group_sync<Warps>(barrier);
         fb |= minors(A, n, ws + lay.shifted_up);
         if (!one_spin) {
-            for (int k = lane; k < n * n; k += kWarp) A[k] = green[static_cast<int64_t>(nmax) * nmax + k];
-            __syncwarp();
+            for (int k = lane; k < n * n; k += kLanes) A[k] = green[static_cast<int64_t>(nmax) * nmax + k];
+            group_sync<Warps>(barrier);
             fb |= minors(A, n, ws + lay.shifted_down);
         }
     }
@@ -584,32 +593,40 @@ __global__ void __launch_bounds__(1024) principal_minors_shared(const __grid_con
     }
 }
 
-// The other orders: a warp per (configuration, set), the workspace in global
-// memory; chunked (orders 11..14): lists of the chunks in shared memory, the
-// top levels' lists and the shifted minors in the global workspace.
-__global__ void __launch_bounds__(256) principal_minors_fp64(const __grid_constant__ Problem p,
-                                                            const __grid_constant__ Scratch w, bool chunked) {
+// The other orders, the workspace in global memory: a warp per (configuration,
+// set) above order 14; Chunked (batches of orders up to 14) two warps, the
+// chunks' lists in shared memory, the top levels' lists and the shifted minors
+// in the global workspace.
+// (512 configurations of order 14, one warp each: seven per SM, the minors 1.04
+// ms, the call 5.31; two warps each: 0.84 and 5.12.)
+template <bool Chunked>
+__global__ void __launch_bounds__(Chunked ? 512 : 256) principal_minors_fp64(const __grid_constant__ Problem p,
+                                                                            const __grid_constant__ Scratch w) {
+    constexpr int kWarps = Chunked ? 2 : 1;
     extern __shared__ double smem[];
-    const int lane = threadIdx.x & (kWarp - 1);
-    const int warp_in_block = threadIdx.x / kWarp;
-    const int warps_per_block = blockDim.x / kWarp;
-    const int64_t global_warp = static_cast<int64_t>(blockIdx.x) * warps_per_block + warp_in_block;
-    const int64_t total_warps = static_cast<int64_t>(gridDim.x) * warps_per_block;
+    const int lane = threadIdx.x & (kWarps * kWarp - 1);
+    const int group = threadIdx.x / (kWarps * kWarp);
+    const int groups = blockDim.x / (kWarps * kWarp);
+    const int64_t global_group = static_cast<int64_t>(blockIdx.x) * groups + group;
+    const int64_t total_groups = static_cast<int64_t>(gridDim.x) * groups;
     const int nmax = p.max_order;
     const WsLayout lay = fp64_minors_layout(nmax, true);
-    double* ws = w.ws_global + static_cast<size_t>(global_warp) * lay.total;
-    double* lu_lane = w.lu_scratch + (static_cast<size_t>(global_warp) * kWarp + lane) * nmax * nmax;
-    double* chunk = smem + static_cast<size_t>(warp_in_block) * chunk_doubles_upto(nmax);
+    double* ws = w.ws_global + static_cast<size_t>(global_group) * lay.total;
+    double* lu_lane = w.lu_scratch + (static_cast<size_t>(global_group) * kWarp + (lane & (kWarp - 1))) * nmax * nmax;
     auto minors = [&](const double* A, int n, double* shifted) {
-        return (chunked && n >= kChunkMinOrder && n <= kChunkMaxOrder)
-                   ? mat2pm_chunked(A, n, p.s.tol_fpm, p.s.fpm_shift, lay, ws, shifted, lu_lane, chunk, lane)
-                   : mat2pm<1>(A, n, p.s.tol_fpm, p.s.fpm_shift, lay, ws, shifted, lu_lane, lane);
+        if constexpr (Chunked) {
+            double* chunk = smem + static_cast<size_t>(group) * chunk_doubles_upto(nmax);
+            if (n >= kChunkMinOrder)
+                return mat2pm_chunked<kWarps>(A, n, p.s.tol_fpm, p.s.fpm_shift, lay, ws, shifted, lu_lane, chunk, lane,
+                                              group);
+        }
+        return mat2pm<kWarps>(A, n, p.s.tol_fpm, p.s.fpm_shift, lay, ws, shifted, lu_lane, lane, group);
     };
-    for (int64_t item = global_warp; item < p.batch * 2; item += total_warps) {
+    for (int64_t item = global_group; item < p.batch * 2; item += total_groups) {
         const int64_t c = item >> 1;
         const int n = p.all_subsets ? nmax : __ldg(p.orders + c);
         if (n < 2 || n > nmax) continue;  // order 1 needs no minors; bad orders are flagged by step 1
-        minors_item<1>(p, w, c, static_cast<int>(item & 1), n, lay, ws, lane, 0, minors);
+        minors_item<kWarps>(p, w, c, static_cast<int>(item & 1), n, lay, ws, lane, group, minors);
     }
 }
 
@@ -1836,18 +1853,15 @@ static cudaError_t post_assembly(const Problem& p_in, const Scratch& w, int sm_c
     }
     const size_t smem = use_smem ? ws_bytes * per_block : chunk_bytes * per_block;
     // an SM whose workspaces leave it few warps: four or two of them share one
-    const int warps = !use_smem ? 1 : per_block <= 7 ? 4 : 2;
-    const void* kernel = !use_smem   ? reinterpret_cast<const void*>(principal_minors_fp64)
-                         : warps > 2 ? reinterpret_cast<const void*>(principal_minors_shared<4>)
-                                     : reinterpret_cast<const void*>(principal_minors_shared<2>);
+    const int warps = use_smem ? (per_block <= 7 ? 4 : 2) : (chunked ? 2 : 1);
+    const auto kernel = use_smem ? (warps > 2 ? principal_minors_shared<4> : principal_minors_shared<2>)
+                                 : (chunked ? principal_minors_fp64<true> : principal_minors_fp64<false>);
     if (smem > 48 * 1024) {
         err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (err != cudaSuccess) return err;
     }
     const unsigned grid = static_cast<unsigned>(blocks), width = static_cast<unsigned>(per_block * warps * kWarp);
-    if (!use_smem) principal_minors_fp64<<<grid, width, smem, stream>>>(p, w, chunked);
-    else if (warps > 2) principal_minors_shared<4><<<grid, width, smem, stream>>>(p, w);
-    else principal_minors_shared<2><<<grid, width, smem, stream>>>(p, w);
+    kernel<<<grid, width, smem, stream>>>(p, w);
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     mark(3);
