@@ -571,7 +571,7 @@ int run(cdet_context* ctx, const double* vertices, const int32_t* orders, int64_
             if (err != cudaSuccess) return cuda_fail(err, "kernel launch");
             // descriptors, scan, scatter, tiles and per-CTA ranges, tensor assembly + minors,
             // CDet (or the queue kernel, or the double-double kernel)
-            launches = 5 + ((cdet::uses_queue_form(p) || p.dd_mode) ? 1 : 2);
+            launches = 5 + (p.dd_mode ? cdet::wide_launches(p, w, ctx->sm_count) : cdet::uses_queue_form(p) ? 1 : 2);
         } else {
             launches = 5;
         }

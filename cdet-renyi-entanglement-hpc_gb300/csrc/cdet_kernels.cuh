@@ -145,7 +145,7 @@ constexpr uint32_t kQueueHeadIndex = 48;  // the queue head's uint32 slot in Scr
 
 // all-subsets CDet work layouts, the values of the C ABI's CDET_FORM_*
 constexpr int kFormAuto = 0, kFormLane = 1, kFormWarp = 2;
-constexpr int kAllWarpMaxOrder = 11;  // the warp form holds a and dp of one set in shared memory
+constexpr int kAllWarpMaxOrder = 11;  // the warp form holds a and dp of both sets in shared memory
 
 // How a single-top batch runs after its Green matrices (the values of the C
 // ABI's CDET_INTEGRAND_*): staged (minors kernel, global a array, CDet
@@ -155,7 +155,7 @@ constexpr int kAllWarpMaxOrder = 11;  // the warp form holds a and dp of one set
 constexpr int kIntegrandAuto = 0, kIntegrandStaged = 1, kIntegrandQueue = 2;
 constexpr int kQueueMaxOrder = 10;  // the queue form keeps a configuration's workspace in shared memory
 constexpr int kQueueMaxWarps = 12;  // warps per block of the queue kernel (384 threads)
-constexpr int kMinorsMaxWarps = 12;  // warps per block (one block per SM) of the shared-memory minors kernel
+constexpr int kMinorsMaxWarps = 12;  // workspaces per block (one block per SM) of the shared-memory minors kernel
 struct QueueShape {
     int warps_per_sm = 0;  // resident warps per SM (0: as many as the shared memory holds)
     int pair = 0;          // 1: two warps per configuration (one per set)
@@ -359,12 +359,12 @@ struct McmcmcStepArgs {
 };
 cudaError_t launch_mcmcmc_init(int64_t chains, int envelope, const uint64_t* seeds, uint64_t* mt, int32_t* mt_index,
                                double* vertices, cudaStream_t stream);
-// Launches the step: for small batches one warp-per-chain kernel; otherwise
+// Launches the step: up to 16,384 chains one warp-per-chain kernel; otherwise
 // one thread-per-chain kernel, preceded for the histogram seed kernel by the
 // warp-per-chain conditional probabilities. *kernels = the kernels launched.
 cudaError_t launch_mcmcmc_step(const McmcmcStepArgs& args, cudaStream_t stream, int* kernels);
 // Smallest all-subsets batch for which the FP64 CDet runs one lane per
-// configuration; smaller batches run one warp per configuration.
+// configuration; smaller batches run blocks of one to four configurations.
 int all_subsets_lane_form_min_batch(int sm_count);
 // *row = (*row + 1) % rows, after a step (one thread)
 cudaError_t launch_mcmcmc_advance_row(int64_t* row, int64_t rows, cudaStream_t stream);
@@ -392,6 +392,7 @@ constexpr int kDDMaxWarps = 8;  // warps per block of the double-double minors a
 cudaError_t launch_integrand_dd(const Problem& p, const Scratch& scratch, int sm_count, cudaStream_t stream);
 // The same integrand behind the split assembly, in 113-bit integer arithmetic.
 cudaError_t launch_integrand_wide(const Problem& p, const Scratch& scratch, int sm_count, cudaStream_t stream);
+int wide_launches(const Problem& p, const Scratch& scratch, int sm_count);  // the kernels it launches
 // The post-assembly stages alone (sort, minors, CDet, or the queue kernel),
 // on Green matrices already in scratch: what the autotuner times.
 cudaError_t launch_post_assembly(const Problem& p, const Scratch& scratch, int sm_count, cudaStream_t stream);

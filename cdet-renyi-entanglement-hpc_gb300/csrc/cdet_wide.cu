@@ -7,10 +7,11 @@
 // double-double pair update of the recursion is 16 operations of 64 to 74
 // clocks. Here every step runs on the 32-bit integer pipes, to 113 bits.
 //
-// One block of four warps runs a configuration, both sets in turn: the
+// One block of four warps (of one warp up to order 7) runs a configuration,
+// both sets in turn: the
 // compact Schur recursion of the minors (the FP64 form's layout, 16-byte
 // elements: 39 KB at order 10, five blocks per SM), a level's items dealt to
-// all 128 threads, then a[mask] = up * down and the connected recursion in the
+// all of its threads, then a[mask] = up * down and the connected recursion in the
 // same shared memory. In the recursion a and dp are kept unpacked (mantissa
 // and exponent arrays), and a mask's sum is a 192-bit integer on a scale that
 // bounds every term of its popcount level: integer addition is associative, so
@@ -34,7 +35,14 @@ namespace cdet {
 
 namespace {
 
-constexpr int kThreads = 128;
+// Orders up to 7 keep four warps waiting on one another and run a warp per
+// configuration, 20 of them per SM (a lone configuration takes as long): order
+// 7, 4,096 configurations, one spin, 911 us with four warps each, 510 with one;
+// order 2: 478 and 269. Order 1 needs neither, only a thread. Four-warp blocks leave the small configurations of a mixed batch to a second launch of
+// one-warp blocks when more than kWideTail per block remain; fewer they take
+// along while the others still run the large ones.
+constexpr int kWideWarpMaxOrder = 7;
+constexpr int64_t kWideTail = 8;
 constexpr int kAccWords = 6;    // the recursion's sums: 192 bits, two's complement
 constexpr int kHeadroom = 12;   // bits between a term's bound and the sign: 2^9 terms and a[mask] itself
 constexpr int32_t kNoExponent = -(1 << 24);
@@ -74,6 +82,7 @@ __device__ __forceinline__ int div_magic(int item, uint32_t magic) {
 // mat2pm_from_buffer (fast_principle_minors.h:120-246) of one n x n matrix A
 // (in shared memory) by the whole block; shifted[mask] ends as the principal
 // minor of mask. Returns true when the LU fallback ran.
+template <int Threads>
 __device__ bool wide_minors(const DD* A, int n, const Problem& p, WidePacked* shifted, int arena, DD* lu_lane) {
     const int tid = threadIdx.x;
     const int msize = n * n;
@@ -83,7 +92,7 @@ __device__ bool wide_minors(const DD* A, int n, const Problem& p, WidePacked* sh
     const DD thresh{p.dd_fpm_shift.hi, p.dd_fpm_shift.lo}, tol{p.dd_tol.hi, p.dd_tol.lo}, zero{0.0, 0.0};
     const DD shift = !dd_lt(thresh, zero) ? thresh : dd_div(DD{max_abs, 0.0}, DD{static_cast<double>(msize), 0.0});
     if (max_abs == 0.0 && dd_zero(shift)) {
-        for (uint32_t m = tid; m < subsets; m += kThreads) shifted[m] = WidePacked{0u, 0u, 0u, 0u};
+        for (uint32_t m = tid; m < subsets; m += Threads) shifted[m] = WidePacked{0u, 0u, 0u, 0u};
         __syncthreads();
         return false;
     }
@@ -92,7 +101,7 @@ __device__ bool wide_minors(const DD* A, int n, const Problem& p, WidePacked* sh
     const WidePacked eps = wide_pack(from_dd(eps_on ? dd_mul(tol, DD{max_abs, 0.0}) : zero));
 
     WidePacked* old_list = shifted + compact_list_offset(n, 0, arena);
-    for (int k = tid; k < msize; k += kThreads) old_list[k] = wide_pack(from_double(A[k].hi));
+    for (int k = tid; k < msize; k += Threads) old_list[k] = wide_pack(from_double(A[k].hi));
     if (tid == 0) {
         shifted[0] = wide_pack(from_double(1.0));
         shifted[1] = wide_pack(wide_add(ps, from_double(A[0].hi)));
@@ -106,7 +115,7 @@ __device__ bool wide_minors(const DD* A, int n, const Problem& p, WidePacked* sh
         const int sets = 1 << level;
         // pivots' inverses, then the first-column factors, in place
         bool bad_pivot = false;
-        for (int set = tid; set < sets; set += kThreads) {
+        for (int set = tid; set < sets; set += Threads) {
             const Wide pivot = wide_add(ps, wide_unpack(old_list[set * old_msize]));
             const WidePacked pa = wide_pack(pivot);
             if ((pa.x | pa.y | pa.z | pa.w) == 0u || (eps_on && wide_abs_le(pa, eps))) bad_pivot = true;
@@ -117,14 +126,14 @@ __device__ bool wide_minors(const DD* A, int n, const Problem& p, WidePacked* sh
             break;
         }
         const uint32_t by_size = 0xFFFFFFFFu / static_cast<uint32_t>(new_size) + 1u;
-        for (int item = tid; item < sets * new_size; item += kThreads) {
+        for (int item = tid; item < sets * new_size; item += Threads) {
             const int set = new_size == 1 ? item : div_magic(item, by_size);
             WidePacked* entry = old_list + set * old_msize + (item - set * new_size + 1) * old_size;
             *entry = wide_pack(wide_mul(wide_unpack(*entry), wide_unpack(old_list[set * old_msize])));
         }
         __syncthreads();
         if (level == n - 2) {  // the 1 x 1 children, straight to their shifted minors
-            for (int set = tid; set < sets; set += kThreads) {
+            for (int set = tid; set < sets; set += Threads) {
                 const WidePacked* m = old_list + set * 4;
                 const Wide base = wide_unpack(m[3]);
                 const Wide l = wide_unpack(m[1]), r = wide_unpack(m[2]);
@@ -139,7 +148,7 @@ __device__ bool wide_minors(const DD* A, int n, const Problem& p, WidePacked* sh
         WidePacked* new_list = shifted + compact_list_offset(n, level + 1, arena);
         const int items = sets * new_msize;
         const uint32_t by_msize = 0xFFFFFFFFu / static_cast<uint32_t>(new_msize) + 1u;
-        for (int item = tid; item < items; item += kThreads) {
+        for (int item = tid; item < items; item += Threads) {
             const int set = div_magic(item, by_msize);
             const int e = item - set * new_msize;
             const int row = div_magic(e, by_size);
@@ -151,29 +160,30 @@ __device__ bool wide_minors(const DD* A, int n, const Problem& p, WidePacked* sh
                 wide_sub_prod(wide_unpack(src[1 + col]), wide_unpack(src[(row + 1) * old_size]), wide_unpack(base)));
         }
         __syncthreads();
-        for (int m = tid; m < 2 * sets; m += kThreads)
+        for (int m = tid; m < 2 * sets; m += Threads)
             shifted[minor_index + m] = wide_pack(wide_add(ps, wide_unpack(new_list[m * new_msize])));
         minor_index += 2 * sets;
         old_list = new_list;
         __syncthreads();
     }
     if (fell_back) {
-        // determinant_principal_minors_from_buffer<DoubleDouble> (fast_principle_minors.h:107-115), on the two
-        // warps that have LU scratch
-        if (tid < 64)
-            for (uint32_t m = 1 + tid; m < subsets; m += 64) shifted[m] = wide_pack(from_dd(minor_by_lu_dd(A, n, m, lu_lane)));
+        // determinant_principal_minors_from_buffer<DoubleDouble> (fast_principle_minors.h:107-115), on the (at
+        // most two) warps that have LU scratch
+        constexpr int kLu = Threads < 64 ? Threads : 64;
+        if (tid < kLu)
+            for (uint32_t m = 1 + tid; m < subsets; m += kLu) shifted[m] = wide_pack(from_dd(minor_by_lu_dd(A, n, m, lu_lane)));
         __syncthreads();
         return true;
     }
     for (uint32_t step = 1; step < subsets; step <<= 1) {  // the prefix product over levels
-        for (uint32_t set = step + 1 + tid; set < 2 * step; set += kThreads)
+        for (uint32_t set = step + 1 + tid; set < 2 * step; set += Threads)
             shifted[set] = wide_pack(wide_mul(wide_unpack(shifted[set]), wide_unpack(shifted[set - step])));
         __syncthreads();
     }
     for (uint32_t step = subsets; step > 1; step >>= 1) {  // the shift removal, bit by bit from the top
         const uint32_t half = step >> 1;
         const int hb = __ffs(half) - 1;
-        for (uint32_t q = tid; q < subsets / 2; q += kThreads) {
+        for (uint32_t q = tid; q < subsets / 2; q += Threads) {
             const uint32_t ss = ((q >> hb) << (hb + 1)) + half + (q & (half - 1u));
             shifted[ss] = wide_pack(wide_sub_prod(ps, wide_unpack(shifted[ss - half]), wide_unpack(shifted[ss])));
         }
@@ -214,6 +224,7 @@ __device__ __forceinline__ int bit_length(const uint32_t* t, int words) {
 // compute_dp_ztransform (integrand_replica_randomly_sampled.h:226-290) by the
 // whole block, order n >= 2, a in place; returns dp of the full mask on every
 // thread.
+template <int Threads>
 __device__ Wide wide_recursion(const RecursionArrays& r, int n, double threshold, LevelBounds& bounds) {
     const int tid = threadIdx.x;
     const int nbits = n - 1;
@@ -235,13 +246,13 @@ __device__ Wide wide_recursion(const RecursionArrays& r, int n, double threshold
         for (int j = 1; j < k; ++j) bound = max(bound, bounds.dp[j] + bounds.even[k - j]);
         for (int base = 0; base < masks;) {
             const int remaining = masks - base;
-            int L = 1, take = kThreads;
-            if (remaining < kThreads) {
-                while (L * 2 * remaining <= kThreads && L * 2 <= subs && L < kWarp) L *= 2;
+            int L = 1, take = Threads;
+            if (remaining < Threads) {
+                while (L * 2 * remaining <= Threads && L * 2 <= subs && L < kWarp) L *= 2;
                 take = remaining;
-                if (4 * L * remaining < 3 * kThreads && L * 2 <= subs && L < kWarp) {  // < 75 % of the threads busy
+                if (4 * L * remaining < 3 * Threads && L * 2 <= subs && L < kWarp) {  // < 75 % of the threads busy
                     L *= 2;
-                    take = kThreads / L;
+                    take = Threads / L;
                 }
             }
             const int q = __ffs(L) - 1;
@@ -340,8 +351,10 @@ __device__ Wide wide_recursion(const RecursionArrays& r, int n, double threshold
     return top;
 }
 
-__global__ void __launch_bounds__(kThreads, 5) integrand_wide(const __grid_constant__ Problem p,
-                                                             const __grid_constant__ Scratch w, int arena) {
+template <int Threads, int MaxOrder>
+__global__ void __launch_bounds__(Threads, 640 / Threads) integrand_wide(const __grid_constant__ Problem p,
+                                                                           const __grid_constant__ Scratch w, int arena,
+                                                                           bool singles, uint32_t leave) {
     extern __shared__ __align__(16) unsigned char wide_smem[];
     __shared__ DD A[kDDMaxOrder * kDDMaxOrder];
     __shared__ LevelBounds bounds;
@@ -350,10 +363,20 @@ __global__ void __launch_bounds__(kThreads, 5) integrand_wide(const __grid_const
     WidePacked* up_minors = minors + arena;  // the spin-up minors while the spin-down ones are formed
     const int tid = threadIdx.x;
     const int nmax = p.max_order;
-    // a lane's LU-fallback matrix: two lanes' FP64 regions of the scratch, two of the block's warps
-    DD* lu_lane = reinterpret_cast<DD*>(w.lu_scratch + (static_cast<size_t>(blockIdx.x) * 64 + (tid & 63)) * 2 * nmax * nmax);
+    // a lane's LU-fallback matrix: two lanes' FP64 regions of the scratch, at most two of the block's warps
+    constexpr int kLu = Threads < 64 ? Threads : 64;
+    DD* lu_lane =
+        reinterpret_cast<DD*>(w.lu_scratch + (static_cast<size_t>(blockIdx.x) * kLu + tid % kLu) * 2 * nmax * nmax);
     uint32_t* head = w.order_count + kQueueHeadIndex;
-    for (;;) {
+    if (singles) {  // order 1, a product of two diagonal entries: a thread per configuration
+        for (int64_t c = static_cast<int64_t>(blockIdx.x) * Threads + tid; c < p.batch;
+             c += static_cast<int64_t>(gridDim.x) * Threads) {
+            if (__ldg(p.orders + c) != 1) continue;
+            const DD result = dd_sub(dd_order1_value(p, w, c, 0), dd_mul(DD{2.0, 0.0}, dd_order1_value(p, w, c, 1)));
+            p.values[c] = dadd(result.hi, result.lo);
+        }
+    }
+    for (bool last = false; !last;) {
         if (tid == 0) next_slot = atomicAdd(head, 1u);
         __syncthreads();
         const uint32_t slot = next_slot;
@@ -361,32 +384,29 @@ __global__ void __launch_bounds__(kThreads, 5) integrand_wide(const __grid_const
         const int64_t c = __ldg(w.config_at + slot);
         const int n = __ldg(p.orders + c);
         __syncthreads();  // next_slot is read before the next pop
-        if (n < 1 || n > nmax) continue;  // flagged by the assembly
+        if (n <= 1 || n > nmax) break;  // the slots' end: order 1 (above), then invalid orders (flagged by the assembly)
+        last = n <= kWideWarpMaxOrder && static_cast<uint32_t>(p.batch) - slot > leave;
         int32_t status = 0;
         DD value[2];
         for (int set = 0; set < 2; ++set) {
-            if (n == 1) {
-                value[set] = dd_order1_value(p, w, c, set);
-                continue;
-            }
             const double* green = w.green + (c * 2 + set) * 2 * static_cast<int64_t>(nmax) * nmax;
             const bool one_spin = p.same_spin[set] != 0;
             const uint32_t count = 1u << n, half = count / 2;
             bool fell_back = false, finite = true;
             for (int spin = 0; spin < (one_spin ? 1 : 2); ++spin) {
                 bool bad = false;
-                for (int k = tid; k < n * n; k += kThreads) {
+                for (int k = tid; k < n * n; k += Threads) {
                     const double x = green[spin * static_cast<int64_t>(nmax) * nmax + k];
                     bad |= !isfinite(x);
                     A[k] = DD{x, 0.0};
                 }
                 if (spin == 1)
-                    for (uint32_t m = tid; m < count; m += kThreads) up_minors[m] = minors[m];
+                    for (uint32_t m = tid; m < count; m += Threads) up_minors[m] = minors[m];
                 if (__syncthreads_or(bad)) {
                     finite = false;
                     break;
                 }
-                fell_back |= wide_minors(A, n, p, minors, arena, lu_lane);
+                fell_back |= wide_minors<Threads>(A, n, p, minors, arena, lu_lane);
             }
             if (!finite) {  // no number to compute: the double-double arithmetic would end in NaN
                 value[set] = DD{__longlong_as_double(0x7FF8000000000000ll), 0.0};
@@ -396,11 +416,11 @@ __global__ void __launch_bounds__(kThreads, 5) integrand_wide(const __grid_const
             }
             // a[mask] = up[mask] * down[mask] (:254-257), unpacked into the recursion's arrays
             const RecursionArrays r = recursion_arrays(minors, n);
-            constexpr int kPer = (1 << kDDMaxOrder) / kThreads;
+            constexpr int kPer = (1 << MaxOrder) / Threads;
             Wide a[kPer];
 #pragma unroll
             for (int i = 0; i < kPer; ++i) {
-                const uint32_t m = tid + i * kThreads;
+                const uint32_t m = tid + i * Threads;
                 if (m < count) {
                     const Wide down = wide_unpack(minors[m]);
                     a[i] = wide_mul(one_spin ? down : wide_unpack(up_minors[m]), down);
@@ -410,7 +430,7 @@ __global__ void __launch_bounds__(kThreads, 5) integrand_wide(const __grid_const
             __syncthreads();
 #pragma unroll
             for (int i = 0; i < kPer; ++i) {
-                const uint32_t m = tid + i * kThreads;
+                const uint32_t m = tid + i * Threads;
                 if (m > 0 && m < count) {
                     const uint32_t at = ((m & 1u) ? half : 0u) + (m >> 1);
                     r.a[at] = make_uint4(a[i].m[0], a[i].m[1], a[i].m[2], a[i].m[3]);
@@ -419,7 +439,7 @@ __global__ void __launch_bounds__(kThreads, 5) integrand_wide(const __grid_const
                 }
             }
             __syncthreads();
-            const Wide top = wide_recursion(r, n, p.dd_threshold.hi, bounds);
+            const Wide top = wide_recursion<Threads>(r, n, p.dd_threshold.hi, bounds);
             value[set] = dd_mul(DD{p.pref_dd[set][n].hi, p.pref_dd[set][n].lo}, to_dd(top.m, top.e, top.sign));
             if (!dd_finite(value[set])) status |= kStatusNonFinite;
             if (fell_back) status |= kStatusFpmFallback;
@@ -436,22 +456,63 @@ __global__ void __launch_bounds__(kThreads, 5) integrand_wide(const __grid_const
 
 }  // namespace
 
+namespace {
+struct WideGrid {
+    int arena, threads;
+    size_t smem;
+    int64_t blocks;
+};
+
+WideGrid wide_grid(const Problem& p, const Scratch& w, int sm_count, int max_order, int threads) {
+    const bool two_spins = !(p.same_spin[0] && p.same_spin[1]);
+    WideGrid g;
+    g.threads = threads;
+    g.arena = compact_minors_layout(max_order, false).arena;
+    g.smem = (static_cast<size_t>(g.arena) + (two_spins ? size_t{1} << max_order : 0)) * sizeof(WidePacked);
+    const int sms = sm_count > 0 ? sm_count : 152;
+    // as many blocks as the shared memory holds (five of four warps at order 10)
+    const int per_sm = static_cast<int>(
+        std::max<size_t>(1, std::min<size_t>(threads == kWarp ? 20 : 12, (227 * 1024) / (g.smem + 4096))));
+    g.blocks = std::min<int64_t>(static_cast<int64_t>(sms) * per_sm, p.batch);
+    // the LU-fallback regions of the scratch: two lanes' for each lane of a block's first (at most two) warps
+    const int64_t lu_warps = threads == kWarp ? 2 : 4;
+    g.blocks = std::min<int64_t>(g.blocks, std::max<int64_t>(1, static_cast<int64_t>(w.ws_warps) / lu_warps));
+    return g;
+}
+
+template <int Threads, int MaxOrder>
+cudaError_t launch_wide(const Problem& p, const Scratch& w, const WideGrid& g, bool singles, uint32_t leave,
+                        cudaStream_t stream) {
+    const auto kernel = integrand_wide<Threads, MaxOrder>;
+    const cudaError_t err =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(g.smem));
+    if (err != cudaSuccess) return err;
+    kernel<<<static_cast<unsigned>(g.blocks), Threads, g.smem, stream>>>(p, w, g.arena, singles, leave);
+    return cudaGetLastError();
+}
+
+// A batch so large that a warp per small configuration pays a second launch.
+bool wide_splits(const Problem& p, int64_t blocks) {
+    return p.max_order > kWideWarpMaxOrder && p.batch > kWideTail * blocks;
+}
+}  // namespace
+
+int wide_launches(const Problem& p, const Scratch& w, int sm_count) {
+    return wide_splits(p, wide_grid(p, w, sm_count, p.max_order, 4 * kWarp).blocks) ? 2 : 1;
+}
+
 cudaError_t launch_integrand_wide(const Problem& p, const Scratch& w, int sm_count, cudaStream_t stream) {
     if (p.batch <= 0) return cudaSuccess;
-    const bool two_spins = !(p.same_spin[0] && p.same_spin[1]);
-    const int arena = compact_minors_layout(p.max_order, false).arena;
-    const size_t smem = (static_cast<size_t>(arena) + (two_spins ? size_t{1} << p.max_order : 0)) * sizeof(WidePacked);
-    const int sms = sm_count > 0 ? sm_count : 152;
-    // small orders: up to 16 blocks of four warps per SM; the shared memory holds five at order 10
-    const int per_sm = static_cast<int>(std::max<size_t>(1, std::min<size_t>(12, (227 * 1024) / (smem + 4096))));
-    int64_t blocks = std::min<int64_t>(static_cast<int64_t>(sms) * per_sm, p.batch);
-    // each block takes four warps' LU-fallback regions of the scratch
-    blocks = std::min<int64_t>(blocks, std::max<int64_t>(1, static_cast<int64_t>(w.ws_warps) / 4));
-    const cudaError_t err =
-        cudaFuncSetAttribute(integrand_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (err != cudaSuccess) return err;
-    integrand_wide<<<static_cast<unsigned>(blocks), kThreads, smem, stream>>>(p, w, arena);
-    return cudaGetLastError();
+    const int small = std::min(p.max_order, kWideWarpMaxOrder);
+    const WideGrid warps = wide_grid(p, w, sm_count, small, kWarp);
+    if (p.max_order <= kWideWarpMaxOrder)
+        return launch_wide<kWarp, kWideWarpMaxOrder>(p, w, warps, true, static_cast<uint32_t>(p.batch), stream);
+    const WideGrid g = wide_grid(p, w, sm_count, p.max_order, 4 * kWarp);
+    const bool split = wide_splits(p, g.blocks);
+    const uint32_t leave = static_cast<uint32_t>(split ? kWideTail * g.blocks : p.batch);
+    const cudaError_t err = launch_wide<4 * kWarp, kDDMaxOrder>(p, w, g, true, leave, stream);
+    if (err != cudaSuccess || !split) return err;
+    return launch_wide<kWarp, kWideWarpMaxOrder>(p, w, warps, false, static_cast<uint32_t>(p.batch), stream);
 }
 
 }  // namespace cdet
