@@ -299,8 +299,8 @@ def time_dd_forms(integrand, d_vertices, d_orders, stream, args, flush):
             "flagged_configs": int((st.cpu().numpy() & 5).astype(bool).sum())}
     integrand.set_assembly("split")
     out["note"] = ("fp64_assembly is the reference's INTEGRAND_REAL=double_double mode with VECTOR_REAL=double, "
-                   "bit-identical to it; split_assembly runs the same double-double recursion on the tensor-core "
-                   "Green matrices; their errors per order are in precision_by_order (dd_vs_truth_filter_on "
+                   "bit-identical to it; split_assembly runs minors and recursion in 113-bit integer floats on the "
+                   "tensor-core Green matrices; their errors per order are in precision_by_order (dd_vs_truth_filter_on "
                    "is the reference mode's)")
     return out
 
@@ -585,8 +585,7 @@ def run_gpu(args):
         # the literal contract: relative error <= 1e-10 at every order, met by
         # the double-double recursion on the split assembly's Green matrices
         dd = line["dd_path"]["split_assembly"]
-        summary = {"form": "split tcgen05 assembly + double-double minors and CDet recursion (lighter "
-                           "double-double steps: FMA products, one renormalisation per sum; lane layout)",
+        summary = {"form": "split tcgen05 assembly + minors and CDet recursion in 113-bit integer floats",
                    "value": dd["value"], "unit": UNIT, "ms_per_step": dd["ms_per_step"],
                    "over_fp64_path": dd["value"] / line["fp64_path"]["value"]}
         if "precision_by_order" in line:

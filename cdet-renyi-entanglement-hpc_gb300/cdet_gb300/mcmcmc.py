@@ -2,7 +2,7 @@
 
 The batch counterpart of run_single_mcmcmc_chain (mcmcmc_sampler.h:994-1088):
 every step evaluates the all-subset integrand of each chain's envelope on the
-GPU and runs run_mcmcmc_step (:524-577) in one thread per chain, with each
+GPU and runs run_mcmcmc_step (:524-577) for every chain, with each
 chain's std::mt19937_64 stream reproduced on the device. With the FP64
 assembly the chains are the reference's chains, step for step.
 `learn_histogram` is learn_factorized_histogram_seed (:607-664) and

@@ -23,22 +23,21 @@
 // 64 and 3.8e-16 at degree 160 (the FP64 Clenshaw sum: 4e-15 to 1.2e-14):
 // FP64-level accuracy without the FP64 pipe.
 //
-// Both bases come from the stride-2 Chebyshev recurrence
-// T_{n+2} = 2 T_2 T_n - T_{n-2} in Q62 fixed point, one thread of a pair for
-// the even and one for the odd degrees. To let each thread write whole
-// core-matrix rows, the coefficient slices order each K step of 16 columns as
-// the eight even b followed by the eight odd b; the contraction over k is
-// indifferent to the order.
+// Both bases come from eight chains of the stride-8 Chebyshev recurrence
+// T_{n+8} = 2 T_8 T_n - T_{n-8} in Q62 fixed point, begun with the stride-1
+// one. To write whole core-matrix rows, the coefficient slices order each K
+// step of 16 columns as the eight even b followed by the eight odd b; the
+// contraction over k is indifferent to the order.
 //
-// Pipeline per evaluation: split_descriptors (one thread per vertex pair:
-// branch, u, v, block ids; corner entries written directly), a counting sort
-// of lookups by block (histogram, single-CTA scan, scatter), a tile list of
-// up to 64 lookups of one block, and split_assembly, a persistent kernel with
-// one CTA per SM that runs the tcgen05 GEMM of each tile. A-operand slices
-// stream from HBM with bulk asynchronous copies (cp.async.bulk) into a
-// three-stage shared-memory ring; the basis slices are generated in shared
-// memory by four producer warps while a single thread issues the MMAs and
-// four epilogue warps drain the previous tile.
+// Pipeline per evaluation: split_descriptors (each vertex decoded once, then
+// the vertex pairs: branch, u, v, block ids; corner entries written
+// directly), a counting sort of lookups by block (histogram, scan, scatter),
+// a tile list of up to 128 lookups of one block, and split_assembly, a
+// persistent kernel with one CTA per SM that runs the tcgen05 GEMM of each
+// tile. Coefficient slices stream from HBM with bulk asynchronous copies
+// (cp.async.bulk) into a three-stage shared-memory ring; the basis slices are
+// generated in shared memory by four producer warps, one warp issues the MMAs
+// and eight epilogue warps drain the accumulators.
 //
 // Degrees above 128 (up to 256) cut each coefficient block into sub-blocks of
 // 128 rows x 128 columns (the last ones shorter: the K steps of a column

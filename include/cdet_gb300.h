@@ -193,7 +193,7 @@ int cdet_load_chunks(cdet_context* ctx, const char* dir, double* order1);
  * resident on the GPU, with the uniform seed kernel (MCMCMC_SEED_MODE=uniform,
  * mcmcmc_seed.h:41-61). Every step evaluates the all-subset integrand of each
  * chain's envelope with the context's assembly and runs run_mcmcmc_step
- * (:524-577) in one thread per chain. Each chain keeps the reference's
+ * (:524-577) for every chain. Each chain keeps the reference's
  * std::mt19937_64 stream and draws from it as libstdc++'s distributions do,
  * so with the FP64 assembly the chains follow the reference's chains step for
  * step. The lambda adaptation (adapt_mcmcmc_lambdas, :579-600) runs on the
@@ -413,7 +413,8 @@ int cdet_set_assembly(cdet_context* ctx, int mode);
 enum cdet_all_subsets_form {
     CDET_FORM_AUTO = 0, /* the warp form below 8 warps' worth of configurations per SM, else the lane form */
     CDET_FORM_LANE = 1, /* one lane per configuration (full FP64 warps; for large batches) */
-    CDET_FORM_WARP = 2  /* one warp per configuration (small batches; orders <= 11, else the lane form) */
+    CDET_FORM_WARP = 2  /* warps over the masks of one to four configurations, in shared memory (small
+                           batches; orders <= 11, else the lane form) */
 };
 
 int cdet_set_all_subsets_form(cdet_context* ctx, int form);
@@ -433,7 +434,7 @@ int cdet_all_subsets_form_tuned(const cdet_context* ctx, int max_order, int fuse
  * these are the batched layouts of that call. */
 enum cdet_integrand_form {
     CDET_INTEGRAND_AUTO = 0,   /* measured per (order, assembly, batch size class); see below */
-    CDET_INTEGRAND_STAGED = 1, /* minors kernel (a warp per configuration and set), a[] in HBM, CDet kernel */
+    CDET_INTEGRAND_STAGED = 1, /* minors kernel (warps per configuration and set), a[] in HBM, CDet kernel */
     CDET_INTEGRAND_QUEUE = 2   /* one persistent kernel: minors and CDet of a configuration in shared
                                   memory, configurations taken from order-sorted slots (decreasing
                                   order) through an atomic queue head */
