@@ -13,17 +13,21 @@
 // elements: 39 KB at order 10, five blocks per SM), a level's items dealt to
 // all of its threads, then a[mask] = up * down and the connected recursion in the
 // same shared memory. In the recursion a and dp are kept unpacked (mantissa
-// and exponent arrays), and a mask's sum is a 192-bit integer on a scale that
-// bounds every term of its popcount level: integer addition is associative, so
-// the submasks of a mask are split over up to 32 lanes and the parts added in
-// any order without changing the value. Blocks take configurations from the
-// order-sorted slots (decreasing order) through an atomic queue head.
+// and exponent arrays), and a mask's sum is a 192-bit integer (WideSum) on a scale
+// that bounds every term of its popcount level, or, where the mask's terms may lie
+// far below that (a vertex far from all others), its own largest term: integer
+// addition is associative, so the submasks of a mask are split over up to 32 lanes
+// and the parts added in any order without changing the value. Blocks take
+// configurations from the order-sorted slots (decreasing order) through an atomic
+// queue head.
 //
 // Bound: the integer pipes and, next to them, shared-memory bandwidth (two
 // 16-byte reads of scattered masks per pair update). Measured at 6x6 / degree
 // 96 / order 10, 8,192 configurations, against double-double minors by warps
-// and one lane per configuration for the recursion: 35.2 -> 4.0 ms after the
-// assembly. Against a binary128 evaluation both have the same errors (256
+// and one lane per configuration for the recursion: 35.2 -> 4.1 ms after the
+// assembly (5.32 ms the call; with the level's scale for every mask, which leaves a
+// graded matrix fewer bits than double-double steps, 5.27; with a scale of its own
+// for every mask 5.53). Against a binary128 evaluation both have the same errors (256
 // configurations per order 2..10 on three lattices: medians 4e-16 to 2e-15,
 // maxima below 2e-12): the Green entries set them.
 #include "cdet_dd.cuh"
@@ -43,8 +47,6 @@ namespace {
 // along while the others still run the large ones.
 constexpr int kWideWarpMaxOrder = 7;
 constexpr int64_t kWideTail = 8;
-constexpr int kAccWords = 6;    // the recursion's sums: 192 bits, two's complement
-constexpr int kHeadroom = 12;   // bits between a term's bound and the sign: 2^9 terms and a[mask] itself
 constexpr int32_t kNoExponent = -(1 << 24);
 
 __device__ __forceinline__ Wide from_double(double x) {
@@ -215,12 +217,6 @@ struct LevelBounds {
     int32_t even[kDDMaxOrder + 1], odd[kDDMaxOrder + 1], dp[kDDMaxOrder + 1];
 };
 
-__device__ __forceinline__ int bit_length(const uint32_t* t, int words) {
-    for (int i = words - 1; i >= 0; --i)
-        if (t[i]) return 32 * i + 32 - __clz(static_cast<int>(t[i]));
-    return 0;
-}
-
 // compute_dp_ztransform (integrand_replica_randomly_sampled.h:226-290) by the
 // whole block, order n >= 2, a in place; returns dp of the full mask on every
 // thread.
@@ -229,8 +225,7 @@ __device__ Wide wide_recursion(const RecursionArrays& r, int n, double threshold
     const int tid = threadIdx.x;
     const int nbits = n - 1;
     const uint32_t half = 1u << nbits;
-    const bool filter = threshold > 0.0;
-    const int thr_log = filter ? ilogb(threshold) : 0;
+    const int thr_log = threshold > 0.0 ? ilogb(threshold) : 0;
     if (tid == 0) {
         r.dp[0] = r.a[half];
         r.de[0] = r.ae[half];
@@ -241,9 +236,9 @@ __device__ Wide wide_recursion(const RecursionArrays& r, int n, double threshold
         const int kk = k - 1;
         const int masks = static_cast<int>(kBinomial.c[nbits][kk]);
         const int subs = 1 << kk;
-        // every |a[mask]| and |dp[sub] a[mask ^ sub]| of the level is below 2^(bound + 1)
-        int32_t bound = bounds.odd[k];
-        for (int j = 1; j < k; ++j) bound = max(bound, bounds.dp[j] + bounds.even[k - j]);
+        // every |a[mask]| and |dp[sub] a[mask ^ sub]| of the level is below 2^(level_bound + 1)
+        int32_t level_bound = bounds.odd[k];
+        for (int j = 1; j < k; ++j) level_bound = max(level_bound, bounds.dp[j] + bounds.even[k - j]);
         for (int base = 0; base < masks;) {
             const int remaining = masks - base;
             int L = 1, take = Threads;
@@ -259,37 +254,46 @@ __device__ Wide wide_recursion(const RecursionArrays& r, int n, double threshold
             const int idx = base + (tid >> q);
             const int j = tid & (L - 1);
             const bool active = (tid >> q) < take && idx < masks;
-            uint32_t acc[kAccWords] = {}, mag[3] = {};
-            uint32_t rest = 0;
-            auto add_term = [&](uint32_t (&t)[kAccWords], int32_t exponent, bool negative) {
-                shift_right_words(t, bound - exponent + kHeadroom);
-                const uint32_t top[3] = {t[3], t[4], t[5]};
-                add_words(mag, top, 0u);
-                const uint32_t m = negative ? 0xFFFFFFFFu : 0u;
-#pragma unroll
-                for (int i = 0; i < kAccWords; ++i) t[i] ^= m;
-                add_words(acc, t, m & 1u);
-            };
+            uint32_t rest = 0, low = 0, fixed = 0;
             if (active) {
                 rest = colex_subset(static_cast<uint32_t>(idx), kk, nbits);
                 // the lane fixes the q highest bits of rest and walks the submasks of the others
-                uint32_t top = 0, low = rest;
+                uint32_t top = 0;
+                low = rest;
                 for (int t = 0; t < q; ++t) {
                     const uint32_t hb = 1u << (31 - __clz(static_cast<int>(low)));
                     top |= hb;
                     low ^= hb;
                 }
-                uint32_t fixed = 0, tb = top;
+                uint32_t tb = top;
                 for (int t = 0; t < q; ++t) {
                     const uint32_t lb = tb & (~tb + 1u);
                     if ((j >> t) & 1) fixed |= lb;
                     tb ^= lb;
                 }
+            }
+            // the sum's scale: the level's where a[mask] alone shows that the terms come near it, else the
+            // largest exponent among the mask's own terms
+            int32_t bound = level_bound;
+            const int32_t own = active ? (r.ae[half + rest] >> 1) - 1 : level_bound;
+            const bool far = own < level_bound - kSumSlack;
+            if (__any_sync(0xffffffffu, far)) {
+                if (far) {
+                    bound = own;
+                    for (uint32_t sl = low;; sl = (sl - 1u) & low) {
+                        const uint32_t sm = fixed | sl;
+                        if (sm != rest) bound = max(bound, (r.de[sm] >> 1) + (r.ae[rest ^ sm] >> 1));
+                        if (sl == 0) break;
+                    }
+                }
+                for (int off = 1; off < L; off <<= 1) bound = max(bound, __shfl_xor_sync(0xffffffffu, bound, off));
+            }
+            WideSum sum;
+            if (active) {
                 if (j == 0) {  // a[mask]: m 2^(e - 127) = m 2^((e - 1) - 126)
                     const uint4 m = r.a[half + rest];
-                    const int32_t es = r.ae[half + rest];
-                    uint32_t t[kAccWords] = {0u, 0u, m.x, m.y, m.z, m.w};
-                    add_term(t, (es >> 1) - 1, es & 1);
+                    const uint32_t am[4] = {m.x, m.y, m.z, m.w};
+                    sum.add(am, bound - own, r.ae[half + rest] & 1);
                 }
                 for (uint32_t sl = low;; sl = (sl - 1u) & low) {
                     const uint32_t sm = fixed | sl;
@@ -299,41 +303,24 @@ __device__ Wide wide_recursion(const RecursionArrays& r, int n, double threshold
                         const uint32_t xm[4] = {x.x, x.y, x.z, x.w}, ym[4] = {y.x, y.y, y.z, y.w};
                         uint32_t pm[4];
                         mul_top(xm, ym, pm);
-                        uint32_t t[kAccWords] = {0u, 0u, pm[0], pm[1], pm[2], pm[3]};
-                        add_term(t, (ex >> 1) + (ey >> 1), ((ex ^ ey) & 1) == 0);  // acc -= dp a
+                        sum.add(pm, bound - ((ex >> 1) + (ey >> 1)), ((ex ^ ey) & 1) == 0);  // sum -= dp a
                     }
                     if (sl == 0) break;
                 }
             }
             for (int off = 1; off < L; off <<= 1) {
-                uint32_t oa[kAccWords], om[3];
+                WideSum other;
 #pragma unroll
-                for (int i = 0; i < kAccWords; ++i) oa[i] = __shfl_xor_sync(0xffffffffu, acc[i], off);
+                for (int i = 0; i < kSumWords; ++i) other.acc[i] = __shfl_xor_sync(0xffffffffu, sum.acc[i], off);
 #pragma unroll
-                for (int i = 0; i < 3; ++i) om[i] = __shfl_xor_sync(0xffffffffu, mag[i], off);
-                add_words(acc, oa, 0u);
-                add_words(mag, om, 0u);
+                for (int i = 0; i < kMagWords; ++i) other.mag[i] = __shfl_xor_sync(0xffffffffu, sum.mag[i], off);
+                sum.merge(other);
             }
             if (active && j == 0) {
-                const bool negative = acc[kAccWords - 1] >> 31;
-                negate_if(acc, negative);
-                bool keep = true;
-                if (filter) {
-                    const int la = bit_length(acc, kAccWords), lm = 96 + bit_length(mag, 3);
-                    if (la < lm + thr_log + 2) {  // near or below the threshold: compare as doubles
-                        double av = 0.0, mv = 0.0;
-                        for (int i = kAccWords - 1; i >= 0; --i) av = dadd(dmul(av, 4294967296.0), static_cast<double>(acc[i]));
-                        for (int i = 2; i >= 0; --i) mv = dadd(dmul(mv, 4294967296.0), static_cast<double>(mag[i]));
-                        keep = !(av < dmul(threshold, dmul(mv, 79228162514264337593543950336.0)));  // 2^96
-                    }
-                }
-                const int shift = normalise_words(acc);
-                const bool zero = !keep || shift >= 32 * kAccWords - 1;
-                // acc 2^(bound + 12 - 190) = m 2^(e - 127), m = the upper four words
-                const int32_t e = zero ? kWideZero : bound + kHeadroom + 1 - shift;
-                r.dp[rest] = make_uint4(acc[2], acc[3], acc[4], acc[5]);
-                r.de[rest] = (e << 1) | (negative ? 1 : 0);
-                atomicMax(&bounds.dp[k], e);
+                const Wide v = sum.value(bound, threshold, thr_log);
+                r.dp[rest] = make_uint4(v.m[0], v.m[1], v.m[2], v.m[3]);
+                r.de[rest] = (v.e << 1) | static_cast<int32_t>(v.sign);
+                atomicMax(&bounds.dp[k], v.e);
             }
             base += take;
         }

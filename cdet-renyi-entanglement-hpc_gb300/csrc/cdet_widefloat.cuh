@@ -323,6 +323,73 @@ __host__ __device__ __forceinline__ Wide wide_inverse(const Wide& a, Reciprocal 
     return out;
 }
 
+__host__ __device__ __forceinline__ int bit_length(const uint32_t* t, int words) {
+    for (int i = words - 1; i >= 0; --i)
+        if (t[i]) return 32 * i + 32 - leading_zeros(t[i]);
+    return 0;
+}
+
+// A sum of up to 2^9 + 1 terms on a fixed-point scale: 192 bits in two's
+// complement with a unit of 2^(bound - 178), `bound` at least every term's
+// exponent, and the sum of the terms' magnitudes with a unit of 2^(bound - 114).
+// Integer additions: the terms may be taken in any order and in parts (merge)
+// without changing a bit. Terms far below the bound lose bits: it has to lie
+// within kSumSlack of some term's exponent, so that the magnitudes reach
+// 2^(bound - 50); the sum's error is then below 2^-118 of them, theirs below
+// 2^-54.
+constexpr int kSumWords = 6;
+constexpr int kSumHeadroom = 12;  // bits between the largest term and the sign
+constexpr int kMagWords = 4;      // the magnitudes keep the upper four words
+constexpr int kSumSlack = 48;
+struct WideSum {
+    uint32_t acc[kSumWords] = {}, mag[kMagWords] = {};
+
+    // +-m 2^(bound - below - 126), m < 2^127, below >= 0
+    __host__ __device__ __forceinline__ void add(const uint32_t (&m)[4], int below, bool negative) {
+        uint32_t t[kSumWords] = {0u, 0u, m[0], m[1], m[2], m[3]};
+        shift_right_words(t, below + kSumHeadroom);
+        const uint32_t top[kMagWords] = {t[2], t[3], t[4], t[5]};
+        add_words(mag, top, 0u);
+        const uint32_t x = negative ? 0xFFFFFFFFu : 0u;
+#pragma unroll
+        for (int i = 0; i < kSumWords; ++i) t[i] ^= x;
+        add_words(acc, t, x & 1u);
+    }
+    __host__ __device__ __forceinline__ void merge(const WideSum& o) {
+        add_words(acc, o.acc, 0u);
+        add_words(mag, o.mag, 0u);
+    }
+    // The sum; zero where its magnitude is below threshold (> 0; thr_log its
+    // ilogb) times the sum of the terms' magnitudes, and where all terms are
+    // the zeros of wide_unpack.
+    __host__ __device__ __forceinline__ Wide value(int32_t bound, double threshold, int thr_log) const {
+        uint32_t a[kSumWords];
+#pragma unroll
+        for (int i = 0; i < kSumWords; ++i) a[i] = acc[i];
+        const bool negative = a[kSumWords - 1] >> 31;
+        negate_if(a, negative);
+        bool keep = bound > kWideZero / 2;
+        if (threshold > 0.0) {
+            constexpr int kLow = 32 * (kSumWords - kMagWords);
+            if (bit_length(a, kSumWords) < kLow + bit_length(mag, kMagWords) + thr_log + 2) {
+                // near or below the threshold: compare as doubles
+                double av = 0.0, mv = 0.0;
+                for (int i = kSumWords - 1; i >= 0; --i) av = av * 4294967296.0 + static_cast<double>(a[i]);
+                for (int i = kMagWords - 1; i >= 0; --i) mv = mv * 4294967296.0 + static_cast<double>(mag[i]);
+                keep = keep && !(av < threshold * (mv * 18446744073709551616.0));  // 2^kLow
+            }
+        }
+        const int shift = normalise_words(a);
+        Wide r;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) r.m[i] = a[i + 2];
+        // a 2^(bound - 178), its leading one moved to bit 190 = m 2^(e - 127), m the upper four words
+        r.e = keep && shift < 32 * kSumWords - 1 ? bound + kSumHeadroom + 1 - shift : kWideZero;
+        r.sign = negative ? 1u : 0u;
+        return r;
+    }
+};
+
 // |a| <= |b| for stored numbers
 __host__ __device__ __forceinline__ bool wide_abs_le(const WidePacked& a, const WidePacked& b) {
     const uint64_t ah = (static_cast<uint64_t>(a.w & 0x7FFFFFFFu) << 32) | a.z;
