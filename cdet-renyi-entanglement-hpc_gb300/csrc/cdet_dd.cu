@@ -366,45 +366,37 @@ __global__ void __launch_bounds__(32) cdet_dd_lane(const __grid_constant__ Probl
 // Smallest batch that runs the lane form (a warp of configurations per SM).
 static int64_t dd_lane_min_batch(int sm_count) { return static_cast<int64_t>(sm_count > 0 ? sm_count : 152) * kWarp; }
 
+DDShape dd_launch_shape(const Problem& p, bool lanes, size_t ws_warps, int sm_count) {
+    const bool two_spins = !(p.same_spin[0] && p.same_spin[1]);
+    const size_t ws_bytes = compact_minors_layout(p.max_order, two_spins, true).total * sizeof(DD);
+    const size_t budget = 227 * 1024;
+    const int64_t warps = std::max<int64_t>(1, static_cast<int64_t>(ws_warps) / 2);  // warps the LU regions are enough for
+    DDShape d;
+    d.wpb = static_cast<int>(std::max<int64_t>(
+        1, std::min<int64_t>({kDDMaxWarps, static_cast<int64_t>(budget / ws_bytes), warps})));
+    const int sms = sm_count > 0 ? sm_count : 152;
+    const int per_sm = std::max(1, static_cast<int>(budget / (ws_bytes * d.wpb + 1024)));
+    const int64_t items = p.batch * (lanes ? 2 : 1);
+    d.blocks = std::min<int64_t>({static_cast<int64_t>(sms) * per_sm, (items + d.wpb - 1) / d.wpb, warps / d.wpb});
+    d.smem = ws_bytes * d.wpb;
+    return d;
+}
+
 cudaError_t launch_integrand_dd(const Problem& p, const Scratch& w, int sm_count, cudaStream_t stream) {
     if (p.batch <= 0) return cudaSuccess;
     // on the split assembly the reference's DoubleDouble steps are not the contract: 113-bit integer arithmetic
     if (p.fused_cdet) return launch_integrand_wide(p, w, sm_count, stream);
-    const bool two_spins = !(p.same_spin[0] && p.same_spin[1]);
-    const bool lanes = p.integrand_form == kIntegrandStaged ||
-                       (p.integrand_form == kIntegrandAuto && p.batch >= dd_lane_min_batch(sm_count));
-    if (w.dd_lanes && lanes) {
-        const size_t ws_bytes = compact_minors_layout(p.max_order, two_spins, true).total * sizeof(DD);
-        const int wpb = static_cast<int>(std::max<size_t>(1, std::min<size_t>(kDDMaxWarps, (227 * 1024) / ws_bytes)));
-        const int sms = sm_count > 0 ? sm_count : 152;
-        const int per_sm = std::max(1, static_cast<int>((227 * 1024) / (ws_bytes * wpb + 1024)));
-        int64_t blocks = std::min<int64_t>(static_cast<int64_t>(sms) * per_sm, (p.batch * 2 + wpb - 1) / wpb);
-        blocks = std::min<int64_t>(blocks, std::max<int64_t>(1, static_cast<int64_t>(w.ws_warps) / (2 * wpb)));
-        const size_t smem = ws_bytes * wpb;
-        cudaError_t err = cudaFuncSetAttribute(principal_minors_dd, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               static_cast<int>(smem));
-        if (err != cudaSuccess) return err;
-        principal_minors_dd<<<static_cast<unsigned>(blocks), wpb * kWarp, smem, stream>>>(p, w);
-        err = cudaGetLastError();
-        if (err != cudaSuccess) return err;
-        // one warp per block, so that a small batch still spreads over every SM
-        cdet_dd_lane<<<static_cast<unsigned>((p.batch + kWarp - 1) / kWarp), kWarp, 0, stream>>>(p, w);
-        return cudaGetLastError();
-    }
-    const size_t ws_bytes = compact_minors_layout(p.max_order, two_spins, true).total * sizeof(DD);
-    const size_t budget = 227 * 1024;
-    const int wpb = static_cast<int>(std::max<size_t>(1, std::min<size_t>(kDDMaxWarps, budget / ws_bytes)));
-    const int sms = sm_count > 0 ? sm_count : 152;
-    const int per_sm = std::max(1, static_cast<int>(budget / (ws_bytes * wpb + 1024)));
-    int64_t blocks = static_cast<int64_t>(sms) * per_sm;
-    // each warp takes two warps' LU-fallback regions of the scratch
-    blocks = std::min<int64_t>(blocks, std::max<int64_t>(1, static_cast<int64_t>(w.ws_warps) / (2 * wpb)));
-    blocks = std::min<int64_t>(blocks, (p.batch + wpb - 1) / wpb);
-    const size_t smem = ws_bytes * wpb;
-    cudaError_t err = cudaFuncSetAttribute(integrand_dd, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           static_cast<int>(smem));
+    const bool lanes = w.dd_lanes && (p.integrand_form == kIntegrandStaged ||
+                                      (p.integrand_form == kIntegrandAuto && p.batch >= dd_lane_min_batch(sm_count)));
+    const DDShape d = dd_launch_shape(p, lanes, w.ws_warps, sm_count);
+    const auto kernel = lanes ? principal_minors_dd : integrand_dd;
+    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(d.smem));
     if (err != cudaSuccess) return err;
-    integrand_dd<<<static_cast<unsigned>(blocks), wpb * kWarp, smem, stream>>>(p, w);
+    kernel<<<static_cast<unsigned>(d.blocks), d.wpb * kWarp, d.smem, stream>>>(p, w);
+    err = cudaGetLastError();
+    if (err != cudaSuccess || !lanes) return err;
+    // one warp per block, so that a small batch still spreads over every SM
+    cdet_dd_lane<<<static_cast<unsigned>((p.batch + kWarp - 1) / kWarp), kWarp, 0, stream>>>(p, w);
     return cudaGetLastError();
 }
 

@@ -1771,6 +1771,38 @@ void carve_scratch(void* base, int64_t batch, int max_order, size_t ws_warps, Sc
     out->dd_lanes = regions.dd_lanes ? take(3 * groups * 2 * subsets * kWarp) : nullptr;
 }
 
+// Minors: the workspace of a (configuration, set) goes to shared memory when
+// at least four fit a block (one block per SM, as many as fit, at most
+// kMinorsMaxWarps; the compact arena up to order 10; without the spin-down
+// minors when both sets have one spin), otherwise to the global workspace. No
+// block holds more workspaces than the scratch has LU-fallback regions.
+MinorsShape minors_launch_shape(const Problem& p, size_t ws_warps, int sm_count) {
+    MinorsShape m;
+    const bool two_spins = !(p.same_spin[0] && p.same_spin[1]);
+    const size_t ws_bytes = minors_layout(p.max_order, two_spins, true).total * sizeof(double);
+    const int fit = minors_warps_in_shared_memory(p.max_order, two_spins);
+    m.use_smem = fit >= 4;  // (the compact arena only: order 11 fits three)
+    // orders 11..14 in the global workspace: the chunked recursion, up to eight
+    // workspaces per block, as many blocks per SM as their chunk buffers allow
+    m.chunked = !m.use_smem && p.max_order >= kChunkMinOrder && p.max_order <= kChunkMaxOrder;
+    const size_t chunk_bytes = m.chunked ? chunk_doubles_upto(p.max_order) * sizeof(double) : 0;
+    const int64_t items = p.batch * 2, regions = std::max<int64_t>(1, static_cast<int64_t>(ws_warps));
+    const int sms = sm_count > 0 ? sm_count : 152;
+    // (a batch of fewer workspaces than the SMs hold spreads over all of them: warps of one SM share its FP64 pipe)
+    const int64_t most = std::min<int64_t>(m.use_smem ? fit : (m.chunked ? 8 : 4), regions);
+    m.per_block = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(most, (items + sms - 1) / sms)));
+    m.blocks = std::min<int64_t>((items + m.per_block - 1) / m.per_block, regions / m.per_block);
+    if (m.use_smem) m.blocks = std::min<int64_t>(m.blocks, sms);  // one wave
+    if (m.chunked) {
+        const int64_t per_sm = std::max<int64_t>(1, (227 * 1024) / (chunk_bytes * m.per_block + 1024));
+        m.blocks = std::min<int64_t>(m.blocks, per_sm * sms);  // one wave
+    }
+    m.smem = (m.use_smem ? ws_bytes : chunk_bytes) * m.per_block;
+    // an SM whose workspaces leave it few warps: four or two of them share one
+    m.warps = m.use_smem ? (m.per_block <= 7 ? 4 : 2) : (m.chunked ? 2 : 1);
+    return m;
+}
+
 // Sort, minors and CDet (or the queue kernel) on the Green matrices in scratch.
 static cudaError_t post_assembly(const Problem& p_in, const Scratch& w, int sm_count, cudaStream_t stream,
                                  const KernelEvents* events) {
@@ -1825,43 +1857,14 @@ static cudaError_t post_assembly(const Problem& p_in, const Scratch& w, int sm_c
         return cudaSuccess;
     }
 
-    // Minors: the workspace of a (configuration, set) goes to shared memory
-    // when at least four fit a block (one block per SM, as many as fit, at most
-    // 16; the compact arena up to order 10; without the spin-down minors when
-    // both sets have one spin), otherwise to the global workspace (4 warps per
-    // block).
-    const bool two_spins = !(p.same_spin[0] && p.same_spin[1]);
-    const size_t ws_bytes = minors_layout(p.max_order, two_spins, true).total * sizeof(double);
-    const int fit = minors_warps_in_shared_memory(p.max_order, two_spins);
-    const bool use_smem = fit >= 4;  // (the compact arena only: order 11 fits three)
-    // orders 11..14 in the global workspace: the chunked recursion, eight
-    // warps per block, as many blocks per SM as their chunk buffers allow
-    const bool chunked = !use_smem && p.max_order >= kChunkMinOrder && p.max_order <= kChunkMaxOrder;
-    const size_t chunk_bytes = chunked ? chunk_doubles_upto(p.max_order) * sizeof(double) : 0;
-    const int64_t items = p.batch * 2;
-    const int sms = sm_count > 0 ? sm_count : 152;
-    // (a batch of fewer workspaces than the SMs hold spreads over all of them: warps of one SM share its FP64 pipe)
-    const int most = use_smem ? fit : (chunked ? 8 : 4);
-    const int per_block = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(most, (items + sms - 1) / sms)));
-    int64_t blocks = (items + per_block - 1) / per_block;
-    const int64_t max_blocks = static_cast<int64_t>(w.ws_warps) / per_block;
-    blocks = std::min<int64_t>(blocks, std::max<int64_t>(1, max_blocks));
-    if (use_smem) blocks = std::min<int64_t>(blocks, sms);  // one wave
-    if (chunked) {
-        const int64_t per_sm = std::max<int64_t>(1, (227 * 1024) / (chunk_bytes * per_block + 1024));
-        blocks = std::min<int64_t>(blocks, per_sm * sms);  // one wave
-    }
-    const size_t smem = use_smem ? ws_bytes * per_block : chunk_bytes * per_block;
-    // an SM whose workspaces leave it few warps: four or two of them share one
-    const int warps = use_smem ? (per_block <= 7 ? 4 : 2) : (chunked ? 2 : 1);
-    const auto kernel = use_smem ? (warps > 2 ? principal_minors_shared<4> : principal_minors_shared<2>)
-                                 : (chunked ? principal_minors_fp64<true> : principal_minors_fp64<false>);
-    if (smem > 48 * 1024) {
-        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    const MinorsShape m = minors_launch_shape(p, w.ws_warps, sm_count);
+    const auto kernel = m.use_smem ? (m.warps > 2 ? principal_minors_shared<4> : principal_minors_shared<2>)
+                                   : (m.chunked ? principal_minors_fp64<true> : principal_minors_fp64<false>);
+    if (m.smem > 48 * 1024) {
+        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(m.smem));
         if (err != cudaSuccess) return err;
     }
-    const unsigned grid = static_cast<unsigned>(blocks), width = static_cast<unsigned>(per_block * warps * kWarp);
-    kernel<<<grid, width, smem, stream>>>(p, w);
+    kernel<<<static_cast<unsigned>(m.blocks), static_cast<unsigned>(m.per_block * m.warps * kWarp), m.smem, stream>>>(p, w);
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     mark(3);
@@ -1935,6 +1938,8 @@ void queue_launch_shape(const Problem& p, const Scratch& w, int sm_count, int* w
     // (a batch of fewer warps than the SMs hold spreads over all of them: warps of one SM share its FP64 pipe)
     const int64_t warps_wanted = (p.batch * (p.queue.pair ? 2 : 1) + sms - 1) / sms;
     if (warps_wanted < per_sm) per_sm = static_cast<int>(warps_wanted + (p.queue.pair ? warps_wanted & 1 : 0));
+    // (each warp has an LU-fallback region of the scratch, which holds ws_warps of them)
+    per_sm = static_cast<int>(std::min<int64_t>(per_sm, std::max<int64_t>(1, static_cast<int64_t>(w.ws_warps))));
     if (p.queue.pair) per_sm &= ~1;
     per_sm = std::max(per_sm, p.queue.pair ? 2 : 1);
     // as few blocks per SM as blocks of at most kQueueMaxWarps allow
@@ -1945,7 +1950,7 @@ void queue_launch_shape(const Problem& p, const Scratch& w, int sm_count, int* w
     int per_sm_blocks = std::max(1, per_sm / wpb);
     while (per_sm_blocks > 1 && per_sm_blocks * (bytes + 1024) > sm_bytes + 1024) --per_sm_blocks;
     int64_t grid = static_cast<int64_t>(sms) * per_sm_blocks;
-    // the LU-fallback scratch holds ws_warps warps; no more warps than configurations need
+    // no more warps than the scratch has regions or the configurations need
     grid = std::min<int64_t>(grid, std::max<int64_t>(1, static_cast<int64_t>(w.ws_warps) / wpb));
     const int64_t warps_needed = p.batch * (p.queue.pair ? 2 : 1);
     grid = std::min<int64_t>(grid, std::max<int64_t>(1, (warps_needed + wpb - 1) / wpb));

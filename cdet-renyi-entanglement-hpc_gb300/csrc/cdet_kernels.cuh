@@ -303,6 +303,16 @@ cudaError_t launch_split_assembly(const Problem& p, const Scratch& w, const Spli
 // retained pairs copied), by the reference's FP64 Clenshaw recurrences.
 cudaError_t launch_fp64_assembly(const Problem& p, const Scratch& scratch, int sm_count, cudaStream_t stream);
 size_t minors_workspace_doubles(int max_order);
+// How a batch's staged minors are launched: `blocks` blocks of `per_block`
+// workspaces, `warps` warps each; blocks * per_block <= ws_warps, the scratch's
+// LU-fallback regions.
+struct MinorsShape {
+    int per_block = 1, warps = 1;
+    int64_t blocks = 1;
+    size_t smem = 0;
+    bool use_smem = false, chunked = false;
+};
+MinorsShape minors_launch_shape(const Problem& p, size_t ws_warps, int sm_count);
 // Whether the minors kernel keeps its per-warp workspace in global memory
 // (orders whose workspace does not fit four warps' worth of shared memory).
 bool minors_use_global_workspace(int max_order, bool two_spins);
@@ -389,6 +399,15 @@ bool uses_queue_form(const Problem& p);
 // (the sort already launched), its workspace in shared memory.
 constexpr int kDDMaxOrder = 10;
 constexpr int kDDMaxWarps = 8;  // warps per block of the double-double minors and warp-form kernels
+// Its launch: warps per block and blocks of the lane form's minors (per
+// configuration and set) or of the warp form (per configuration). A warp takes
+// two warps' LU-fallback regions: 2 * blocks * wpb <= ws_warps.
+struct DDShape {
+    int wpb = 1;
+    int64_t blocks = 1;
+    size_t smem = 0;
+};
+DDShape dd_launch_shape(const Problem& p, bool lanes, size_t ws_warps, int sm_count);
 cudaError_t launch_integrand_dd(const Problem& p, const Scratch& scratch, int sm_count, cudaStream_t stream);
 // The same integrand behind the split assembly, in 113-bit integer arithmetic.
 cudaError_t launch_integrand_wide(const Problem& p, const Scratch& scratch, int sm_count, cudaStream_t stream);

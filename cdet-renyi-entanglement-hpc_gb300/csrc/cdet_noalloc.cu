@@ -56,7 +56,7 @@ namespace {
 
 constexpr size_t kNoAllocScratchBytes = size_t{64} << 20;  // 64 MiB per device
 constexpr int kMaxDevices = 64;
-constexpr size_t kMinWarps = 8;  // one block of the shared-memory minors kernel
+constexpr size_t kMinWarps = 8;  // the fewest warps' regions a batch may leave (the minors then run one block of so many workspaces)
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
