@@ -164,7 +164,8 @@ cdet::ScratchRegions scratch_regions(const cdet_context* ctx) {
 }
 
 int ensure_scratch(cdet_context* ctx, int64_t batch, int max_order) {
-    const bool dd = ctx->integrand_real == CDET_INTEGRAND_REAL_DOUBLE_DOUBLE;
+    // (the double-double integrand behind the split assembly has no lane form)
+    const bool dd = ctx->integrand_real == CDET_INTEGRAND_REAL_DOUBLE_DOUBLE && ctx->assembly == CDET_ASSEMBLY_FP64;
     if (ctx->scratch && batch <= ctx->scratch_batch && max_order <= ctx->scratch_order && (!dd || ctx->scratch_dd))
         return CDET_OK;
     const int64_t new_batch = batch > ctx->scratch_batch ? batch : ctx->scratch_batch;
@@ -511,8 +512,9 @@ int run(cdet_context* ctx, const double* vertices, const int32_t* orders, int64_
     bool tune_post = false;
     std::tuple<int, int, int> post_key;
     if (p.dd_mode) {
-        // the double-double integrand: STAGED = its lane form, QUEUE = its warp
-        // form, AUTO = the lane form from one warp of configurations per SM
+        // the double-double integrand on the FP64 assembly: STAGED = its lane form,
+        // QUEUE = its warp form, AUTO = the lane form from one warp of configurations
+        // per SM; on the split assembly there is one form
         p.integrand_form = ctx->integrand_form;
     } else if (!p.all_subsets && !assembly_only && max_order <= cdet::kQueueMaxOrder) {
         if (ctx->integrand_form != CDET_INTEGRAND_AUTO) {
