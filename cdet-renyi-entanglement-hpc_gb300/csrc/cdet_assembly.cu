@@ -2,12 +2,12 @@
 // reference's Clenshaw recurrences (g_funcs.h:395-463, 609-763), bit for bit.
 //
 // A lookup is one 2-D Chebyshev sum: nu independent row sums over v, then one
-// sum of the row values over u. One block of four warps takes up to
-// kMaxLookups lookups of one configuration. Its row sums (lookups x rows) are
-// dealt to lanes in runs of 32, so a single configuration already fills a
-// block with independent chains and no lane idles on an invalid entry of a
-// mixed-order batch; the row values go to shared memory, and one lane per
-// lookup runs the outer sum over them.
+// sum of the row values over u. One block of four warps takes up to 16 lookups
+// (more where the rows are few) of one configuration, or of several whose lookups
+// are fewer. Its row sums (lookups x rows) are dealt to lanes in runs of 32, so a
+// single configuration already fills a block with independent chains and no lane
+// idles on an invalid entry of a mixed-order batch; the row values go to shared
+// memory, and one lane per lookup runs the outer sum over them.
 //
 // Row sums: each lane walks one row of nv coefficients downwards. The 32 rows
 // of a warp are copied eight columns at a time with cp.async (two buffers per
@@ -32,7 +32,7 @@
 // G/s: 76 ms; one and a half: 38 ms); 6x6 / degree 96, 4,096 mixed orders 1..10
 // 26.6 -> 4.1 ms (no lanes on entries past a configuration's order); 4x4 / 45 x
 // 37 coefficients, two spins, order 7 x 391 1.47 -> 0.55 ms; one order-6
-// configuration 2.08 -> 0.08 ms (all rows at once); 128 chains of envelope 9, a
+// configuration 2.08 -> 0.14 ms (all rows at once); 128 chains of envelope 9, a
 // step with reused pairs 3.35 -> 0.54 ms (copies and evaluations in one launch).
 #include "cdet_device.cuh"
 #include "cdet_kernels.cuh"
@@ -88,7 +88,8 @@ __device__ __forceinline__ double clamp_unit(double value) {
 
 constexpr int kThreads = 128;
 constexpr int kWarps = kThreads / kWarp;
-constexpr int kMaxLookups = 16;  // lookups of one block: the outer sums run on that many lanes of one warp
+constexpr int kMaxLookups = 128;  // lookups of one block, a thread each for the decode and the outer sum
+constexpr int kMaxConfigs = kWarp;  // configurations of one block
 constexpr int kRowBlock = 128;   // row values kept per lookup; more rows are taken block by block
 constexpr int kChunk = 8;        // columns of a staged chunk
 constexpr int kStride = 10;      // doubles between the rows of a staged chunk: 16-byte aligned, 16-byte reads free of bank conflicts
@@ -97,15 +98,16 @@ constexpr int kStride = 10;      // doubles between the rows of a staged chunk: 
 struct Lookup {
     const double* coeffs;  // its block of nu x nv coefficients
     double u, v;
-    int set, i, j;
-    int spin;    // the spin evaluated
-    int active;  // 0: nothing to evaluate (value already written, or a rejected vertex)
+    int8_t config;  // which of the block's configurations, and its order
+    int8_t n;
+    int8_t set, i, j;
+    int8_t spin;    // the spin evaluated
+    int8_t active;  // 0: nothing to evaluate (value already written, or a rejected vertex)
 };
 
 struct Shared {
     double stage[kWarps][2][kWarp * kStride];
     const double* row[kWarps][2][kWarp];  // the rows of the run being staged
-    Lookup lookup[kMaxLookups];
 };
 
 // fill_pair_range (integrand_replica_randomly_sampled.h:467-473) for one
@@ -247,40 +249,46 @@ __device__ __forceinline__ void stage_chunk(double* st, const double* const* row
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
-// One block: lookups [first, first + count) of configuration blockIdx.x,
-// first = blockIdx.y * lookups_per_block. The lookups of a configuration of
-// order n, set by set and spin by spin: its n^2 entries, or, with Green-pair
-// reuse, the entries of pairs not both retained (rows i < k at columns
-// k..n-1, then rows i >= k at every column), where the blocks with
-// blockIdx.y == 0 also copy the retained ones.
+// One block: lookups [first, first + count) of configuration blockIdx.x, first =
+// blockIdx.y * lookups_per_block, or (per_block > 1, gridDim.y == 1) all lookups
+// of per_block configurations. The lookups of a configuration of order n, set by
+// set and spin by spin: its n^2 entries, or, with Green-pair reuse, the entries
+// of pairs not both retained (rows i < k at columns k..n-1, then rows i >= k at
+// every column), where the blocks with blockIdx.y == 0 also copy the retained
+// ones.
 template <bool kVec16>
 __global__ void __launch_bounds__(kThreads, 5) green_assembly_fp64(const __grid_constant__ Problem p,
                                                                   const __grid_constant__ Scratch w,
-                                                                  int lookups_per_block, int row_block) {
+                                                                  int lookups_per_block, int per_block, int row_block) {
     extern __shared__ __align__(16) unsigned char assembly_smem[];
+    __shared__ int s_start[kMaxConfigs + 1];  // per_block > 1: first lookup of each configuration, and the total
     Shared& sm = *reinterpret_cast<Shared*>(assembly_smem);
-    double* values = reinterpret_cast<double*>(assembly_smem + sizeof(Shared));  // [lookup][row_block | 1]
+    Lookup* lookups = reinterpret_cast<Lookup*>(assembly_smem + sizeof(Shared));
+    double* values = reinterpret_cast<double*>(lookups + lookups_per_block);  // [lookup][row_block | 1]
     const int value_stride = row_block | 1;
     const Scalars& s = p.s;
     const int nmax = p.max_order;
-    const int64_t c = blockIdx.x;
     const int tid = threadIdx.x, lane = tid & (kWarp - 1), warp = tid / kWarp;
-    const int n = p.all_subsets ? nmax : __ldg(p.orders + c);
-    if (n < 1 || n > nmax) {
-        if (blockIdx.y == 0 && tid == 0) atomicOr(p.status + c, kStatusBadInput);
-        return;
-    }
-    const double* vbase = p.vertices + c * static_cast<int64_t>(nmax) * 4;
-    const int kept = p.reuse_mask ? __popcll(__ldg(p.reuse_mask + c)) : 0;
-    const int per = n * n - kept * kept;  // evaluated entries of one set and spin
+    const int64_t c0 = static_cast<int64_t>(blockIdx.x) * per_block;
+    const int configs = static_cast<int>(min(static_cast<int64_t>(per_block), p.batch - c0));
     const int spins0 = p.same_spin[0] ? 1 : 2, spins1 = p.same_spin[1] ? 1 : 2;
-    const int total = per * (spins0 + spins1);
+    auto order_of = [&](int64_t c) { return p.all_subsets ? nmax : __ldg(p.orders + c); };
+    auto kept_of = [&](int64_t c) { return p.reuse_mask ? __popcll(__ldg(p.reuse_mask + c)) : 0; };
+    auto evaluated = [&](int n, int kept) { return n < 1 || n > nmax ? 0 : n * n - kept * kept; };  // of a set and spin
 
-    if (kept > 0 && blockIdx.y == 0) {
-        for (int e = tid; e < 2 * kept * kept; e += kThreads) {
-            const int set = e >= kept * kept ? 1 : 0;
-            const int r = e - set * kept * kept;
-            const int i = r / kept, j = r - (r / kept) * kept;
+    if (blockIdx.y == 0 && tid < configs) {
+        const int n = order_of(c0 + tid);
+        if (n < 1 || n > nmax) atomicOr(p.status + c0 + tid, kStatusBadInput);
+    }
+    if (p.reuse_mask && blockIdx.y == 0) {
+        const int per_config = 2 * nmax * nmax;
+        for (int t = tid; t < configs * per_config; t += kThreads) {
+            const int64_t c = c0 + t / per_config;
+            const int e = t % per_config, n = order_of(c), kept = kept_of(c);
+            const int set = e >= nmax * nmax ? 1 : 0;
+            const int r = e - set * nmax * nmax, i = r / nmax, j = r - i * nmax;
+            if (n < 1 || n > nmax || i >= kept || j >= kept) continue;
+            const double* vbase = p.vertices + c * static_cast<int64_t>(nmax) * 4;
             bool bad = false;  // the decode's checks, so the status bits are a fresh evaluation's
             decode_vertex(vbase + 4 * i, s, set == 0 ? 2 : 1, bad);
             decode_vertex(vbase + 4 * j, s, set == 0 ? 2 : 1, bad);
@@ -290,10 +298,32 @@ __global__ void __launch_bounds__(kThreads, 5) green_assembly_fp64(const __grid_
     }
 
     const int first = blockIdx.y * lookups_per_block;
+    int total, config = 0, e = first + tid;
+    if (per_block == 1) {
+        total = evaluated(order_of(c0), kept_of(c0)) * (spins0 + spins1);
+    } else {
+        if (warp == 0) {
+            const int mine = lane < configs ? evaluated(order_of(c0 + lane), kept_of(c0 + lane)) * (spins0 + spins1) : 0;
+            int end = mine;
+            for (int off = 1; off < kWarp; off <<= 1) {
+                const int below = __shfl_up_sync(0xffffffffu, end, off);
+                if (lane >= off) end += below;
+            }
+            s_start[lane] = end - mine;
+            if (lane == kWarp - 1) s_start[kMaxConfigs] = end;
+        }
+        __syncthreads();
+        total = s_start[kMaxConfigs];
+        for (int half = kMaxConfigs / 2; half > 0; half /= 2)  // the last configuration that starts at or before e
+            if (s_start[config + half] <= e) config += half;
+        e -= s_start[config];
+    }
     if (first >= total) return;
     const int count = min(lookups_per_block, total - first);
     if (tid < count) {
-        int e = first + tid;
+        const int64_t c = c0 + config;
+        const int n = order_of(c), kept = kept_of(c), per = evaluated(n, kept);
+        const double* vbase = p.vertices + c * static_cast<int64_t>(nmax) * 4;
         const int set = e >= per * spins0 ? 1 : 0;
         e -= set * per * spins0;
         const int spin = e >= per ? 1 : 0;
@@ -308,10 +338,12 @@ __global__ void __launch_bounds__(kThreads, 5) green_assembly_fp64(const __grid_
             j = q - (q / n) * n;
         }
         Lookup l;
-        l.set = set;
-        l.spin = spin;
-        l.i = i;
-        l.j = j;
+        l.config = static_cast<int8_t>(config);
+        l.n = static_cast<int8_t>(n);
+        l.set = static_cast<int8_t>(set);
+        l.spin = static_cast<int8_t>(spin);
+        l.i = static_cast<int8_t>(i);
+        l.j = static_cast<int8_t>(j);
         l.u = l.v = 1.0;  // a lookup with nothing to evaluate walks its rows harmlessly
         l.active = 0;
         bool bad = false;
@@ -337,7 +369,7 @@ __global__ void __launch_bounds__(kThreads, 5) green_assembly_fp64(const __grid_
             l.v = clamp_unit(dsub(ddiv(dmul(2.0, t_inner), t_outer), 1.0));
             l.active = 1;
         }
-        sm.lookup[tid] = l;
+        lookups[tid] = l;
     }
     __syncthreads();
 
@@ -348,7 +380,7 @@ __global__ void __launch_bounds__(kThreads, 5) green_assembly_fp64(const __grid_
     // recurrence of a row, over u)
     Argument outer_arg;
     double outer_b1 = 0.0, outer_b2 = 0.0;
-    if (tid < count) outer_arg = argument(sm.lookup[tid].u);
+    if (tid < count) outer_arg = argument(lookups[tid].u);
 
     for (int hi = nu; hi > 0; hi -= row_block) {
         const int rows = min(row_block, hi);
@@ -359,7 +391,7 @@ __global__ void __launch_bounds__(kThreads, 5) green_assembly_fp64(const __grid_
             for (int task = tid; task < tasks; task += kThreads) {
                 const int l = task / rows, r = task - l * rows;
                 values[l * value_stride + r] = clenshaw_row(
-                    sm.lookup[l].coeffs + static_cast<int64_t>(base_row + r) * nv, nv - 1, sm.lookup[l].v);
+                    lookups[l].coeffs + static_cast<int64_t>(base_row + r) * nv, nv - 1, lookups[l].v);
             }
         } else {
             // this warp's runs warp, warp + 4, ...: a flat sequence of (run, chunk) with one chunk staged ahead
@@ -367,7 +399,7 @@ __global__ void __launch_bounds__(kThreads, 5) green_assembly_fp64(const __grid_
             auto point_rows = [&](int m) {  // the m-th run's rows; lanes past the end repeat the last task
                 const int task = min((warp + m * kWarps) * kWarp + lane, tasks - 1);
                 const int l = task / rows, r = task - l * rows;
-                sm.row[warp][m & 1][lane] = sm.lookup[l].coeffs + static_cast<int64_t>(base_row + r) * nv;
+                sm.row[warp][m & 1][lane] = lookups[l].coeffs + static_cast<int64_t>(base_row + r) * nv;
                 __syncwarp();
             };
             auto stage = [&](int m, int j, int slot) {  // chunk j of run m: columns from the top
@@ -384,7 +416,7 @@ __global__ void __launch_bounds__(kThreads, 5) green_assembly_fp64(const __grid_
                 const int task = (warp + m * kWarps) * kWarp + lane;
                 const int task_c = min(task, tasks - 1);
                 const int l = task_c / rows, r = task_c - l * rows;
-                const Argument arg = argument(sm.lookup[l].v);
+                const Argument arg = argument(lookups[l].v);
                 // integer products while every lane's factor allows them and no chunk of this run failed
                 bool soft = __all_sync(0xffffffffu, soft_argument(arg));
                 double b1 = 0.0, b2 = 0.0;
@@ -456,9 +488,10 @@ __global__ void __launch_bounds__(kThreads, 5) green_assembly_fp64(const __grid_
         }
         __syncthreads();
     }
-    if (tid < count && sm.lookup[tid].active)
-        store_entry(p, w, c, n, sm.lookup[tid].set, sm.lookup[tid].i, sm.lookup[tid].j, sm.lookup[tid].spin,
-                    p.same_spin[sm.lookup[tid].set] != 0, outer_b1);
+    if (tid < count && lookups[tid].active) {
+        const Lookup& l = lookups[tid];
+        store_entry(p, w, c0 + l.config, l.n, l.set, l.i, l.j, l.spin, p.same_spin[l.set] != 0, outer_b1);
+    }
 }
 
 }  // namespace
@@ -467,14 +500,20 @@ cudaError_t launch_fp64_assembly(const Problem& p, const Scratch& w, int sm_coun
     if (p.batch <= 0) return cudaSuccess;
     const int spins = (p.same_spin[0] ? 1 : 2) + (p.same_spin[1] ? 1 : 2);
     const int64_t per_config = static_cast<int64_t>(spins) * p.max_order * p.max_order;
-    // lookups per block: 16 once the batch gives every SM its four blocks several times over (the outer
-    // sum's one busy warp per block is then 1/512th of its work at degree 128), fewer for small batches,
-    // down to one lookup per block, so that they spread over all SMs
+    // lookups per block: 16 (or 512 row sums, four runs of each warp, where the rows are fewer than 32) once the
+    // batch gives every SM its five blocks several times over, fewer for small batches, down to one lookup per
+    // block, so that they spread over all SMs
     const int64_t blocks_wanted = 16 * static_cast<int64_t>(sm_count > 0 ? sm_count : 152);
-    const int lookups = static_cast<int>(
-        std::max<int64_t>(1, std::min<int64_t>(kMaxLookups, p.batch * per_config / blocks_wanted)));
+    const int64_t most = std::max<int64_t>(16, std::min<int64_t>(kMaxLookups, 512 / p.s.nu));
+    const int lookups =
+        static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(most, p.batch * per_config / blocks_wanted)));
+    // as many configurations as have at most that many (a block costs about 5 us whatever it has to do; Green
+    // matrices alone, one thread per lookup / a block per configuration of 16 lookups / this rule: order 1 x
+    // 65,536 at degree 12 444 / 707 / 180 us, at degree 32 2,500 / 1,234 / 609; order 8 x 4,096 at degree 4 226 /
+    // 295 / 174; from order 3 on at degree 32 the rule changes nothing)
+    const int per_block = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(kMaxConfigs, lookups / per_config)));
     const int row_block = std::min(p.s.nu, kRowBlock);
-    const size_t smem = sizeof(Shared) + static_cast<size_t>(lookups) * (row_block | 1) * sizeof(double);
+    const size_t smem = sizeof(Shared) + lookups * (sizeof(Lookup) + static_cast<size_t>(row_block | 1) * sizeof(double));
     // 16-byte copies need 16-byte aligned rows
     bool vec16 = p.s.nv % 2 == 0;
     for (int set = 0; set < 2; ++set)
@@ -485,8 +524,9 @@ cudaError_t launch_fp64_assembly(const Problem& p, const Scratch& w, int sm_coun
     const cudaError_t err =
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (err != cudaSuccess) return err;
-    const dim3 grid(static_cast<unsigned>(p.batch), static_cast<unsigned>((per_config + lookups - 1) / lookups));
-    kernel<<<grid, kThreads, smem, stream>>>(p, w, lookups, row_block);
+    const dim3 grid(static_cast<unsigned>((p.batch + per_block - 1) / per_block),
+                    static_cast<unsigned>((per_config + lookups - 1) / lookups));
+    kernel<<<grid, kThreads, smem, stream>>>(p, w, lookups, per_block, row_block);
     return cudaGetLastError();
 }
 
