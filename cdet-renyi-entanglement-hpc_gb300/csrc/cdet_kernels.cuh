@@ -369,9 +369,9 @@ struct McmcmcStepArgs {
 };
 cudaError_t launch_mcmcmc_init(int64_t chains, int envelope, const uint64_t* seeds, uint64_t* mt, int32_t* mt_index,
                                double* vertices, cudaStream_t stream);
-// Launches the step: up to 16,384 chains one warp-per-chain kernel; otherwise
-// one thread-per-chain kernel, preceded for the histogram seed kernel by the
-// warp-per-chain conditional probabilities. *kernels = the kernels launched.
+// Launches the step: below a number of chains that depends on the envelope
+// (2,048 to 16,384) one warp-per-chain kernel; otherwise one thread-per-chain
+// kernel, preceded for the histogram seed kernel by the warp-per-chain conditional probabilities. *kernels = the kernels launched.
 cudaError_t launch_mcmcmc_step(const McmcmcStepArgs& args, cudaStream_t stream, int* kernels);
 // Smallest all-subsets batch for which the FP64 CDet runs one lane per
 // configuration; smaller batches run blocks of one to four configurations.

@@ -1,5 +1,5 @@
-// Device-resident MCMCMC chains: run_mcmcmc_step (mcmcmc_sampler.h:524-577) on the all-subset integrand values of its
-// envelope, so a batch of chains advances one step per launch pair
+// Device-resident MCMCMC chains: run_mcmcmc_step (mcmcmc_sampler.h:524-577) on
+// the all-subset integrand values of each chain's envelope, so a batch of chains advances one step per launch pair
 // (integrand, step) with no host round trip. The seed kernel is the uniform
 // one (mcmcmc_seed.h:41-61) or the factorized histogram (:71-229), whose
 // conditional generation probabilities (mcmcmc_sampler.h:252-335) weight the
@@ -16,6 +16,8 @@
 // consecutive addresses.
 #include "cdet_device.cuh"
 #include "cdet_kernels.cuh"
+
+#include <algorithm>
 
 namespace cdet {
 
@@ -381,8 +383,8 @@ __global__ void __launch_bounds__(128) mcmcmc_step(const __grid_constant__ Mcmcm
     finish_step<Hist>(a, c, row, Hist ? a.cprob + c * (int64_t{1} << a.envelope) : nullptr);
 }
 
-// The step with one warp per chain (up to kStepWarpMaxChains chains), one to
-// eight chains per block. Everything elementwise runs on the chain's lanes:
+// The step with one warp per chain (fewer than step_warp_max_chains chains), one
+// to eight chains per block. Everything elementwise runs on the chain's lanes:
 // the fluxes and selection weights, the signal terms, the search for the drawn
 // mask, the generator. What the reference adds up in mask order stays a serial
 // sum, but shares its FP64 instructions: the local normalisations of the
@@ -397,7 +399,6 @@ __global__ void __launch_bounds__(128) mcmcmc_step(const __grid_constant__ Mcmcm
 // divisions and global generator state: 128 chains 215 -> 50 us, 2,048 chains 588 -> 74 us (one
 // thread per chain before).
 constexpr int kStepWarpMaxEnvelope = 12;
-constexpr int64_t kStepWarpMaxChains = 16384;
 constexpr int kStepMaxChainsPerBlock = 8;
 
 // Doubles of shared memory per chain: fluxes and weight prefixes (each padded
@@ -406,6 +407,24 @@ constexpr int kStepMaxChainsPerBlock = 8;
 __host__ __device__ inline size_t step_doubles(int env, bool hist) {
     const size_t subsets = size_t{1} << env;
     return 2 * (subsets + 1) + (hist ? subsets + static_cast<size_t>(env) * (env + 1) : 0);
+}
+
+// From how many chains on a thread per chain is the faster step. A warp per
+// chain loses its lead where the envelope leaves its lanes nothing to do (2, 3)
+// and where the shared memory of few chains fills an SM, so that many chains are
+// many rounds (from envelope 11; earlier with the histogram seed, whose
+// probabilities the other form makes on full SMs). Whole steps, thread form over
+// warp form (2x2, degree 8; uniform seed, then histogram): envelope 2, 2,048 chains
+// 1.00 and 0.98, 8,192 0.94 and 0.90; envelope 3, 4,096 1.05 and 1.04, 8,192 1.02 and
+// 0.96; 4 to 10, 8,192 1.11 to 1.26 and 1.08 to 1.17, 16,383 1.05 to 1.14 and 0.99 to
+// 1.07; 11 (six and four chains per SM), 3,000 1.31 and 1.05, 4,096 1.21 and 0.96,
+// 12,000 1.02 and 0.81; 12 (three and two), 3,000 1.01 and 0.95, 8,192 1.00 and 0.88.
+int64_t step_warp_max_chains(int env, bool hist) {
+    if (env > kStepWarpMaxEnvelope) return 0;
+    constexpr int64_t kLeast = 2048, kMost = 16384;
+    if (env <= 3) return env <= 2 ? kLeast : 4 * kLeast;
+    const int64_t per_sm = (227 * 1024) / static_cast<int64_t>(step_doubles(env, hist) * sizeof(double));
+    return per_sm >= 8 ? kMost : std::max<int64_t>(kLeast, per_sm * (hist ? 768 : 2048));
 }
 
 template <bool Hist>
@@ -604,7 +623,7 @@ cudaError_t launch_mcmcmc_step(const McmcmcStepArgs& args, cudaStream_t stream, 
     *kernels = 0;
     if (args.chains <= 0) return cudaSuccess;
     const bool hist = args.tau_bins > 0;
-    if (args.chains < kStepWarpMaxChains && args.envelope <= kStepWarpMaxEnvelope) {
+    if (args.chains < step_warp_max_chains(args.envelope, hist)) {
         // as many chains per block as leave every SM a block, while shared memory holds them
         const size_t per_chain = step_doubles(args.envelope, hist) * sizeof(double);
         int per_block = 1;
