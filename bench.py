@@ -6,6 +6,8 @@ seeded configurations at order n = 10 per step (uniform vertices, both spins).
 One step evaluates the whole batch; `value` is configurations per second over
 the whole job with the inputs resident in HBM, `e2e` the same through the
 host-buffer C-ABI call with the host<->device copies inside the timed region.
+The last line of standard output is the result; the whole record (per-order
+precision, both forms' stages, notes) is one JSON object on standard error.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--path both|split|fp64]
   python bench.py --impl reference ...   # the CPU integrand on the host cores
@@ -55,6 +57,29 @@ SPLIT_TRAFFIC_RULE = ("model (distinct coefficient blocks x slice bytes + 88 B p
 ORDER = 10
 L2_FLUSH_BYTES = 512 << 20
 PRESET = "8x8-d128"
+
+
+# What the last line of standard output takes of the whole record (which goes
+# to standard error as one JSON object): a line of tens of kilobytes is cut by
+# programs that keep the end of the output.
+HEADLINE_KEYS = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+                 "vs_baseline", "dtype", "data", "config", "e2e", "gpu_launches", "stages_ms_per_step", "clocks",
+                 "flagged_configs", "e2e_bit_identical", "split_over_fp64")
+HEADLINE_PARTS = {
+    "roofline": ("kernel", "bound", "achieved", "peak", "unit", "frac", "traffic"),
+    "fp64_path": ("value", "ms_per_step", "bit_identical_to_reference"),
+    "cpu_baseline": ("value", "unit", "cores", "kind"),
+    "precision_by_order": ("worst_condition_scaled", "contract_met"),
+    "at_1e-10_relative": ("value", "ms_per_step", "worst_relative_error_orders_2_10", "contract_met"),
+}
+
+
+def headline(line):
+    out = {k: line[k] for k in HEADLINE_KEYS if k in line}
+    for key, parts in HEADLINE_PARTS.items():
+        if line.get(key) is not None:
+            out[key] = {k: line[key][k] for k in parts if k in line[key]}
+    return out
 
 
 def workload_params():
@@ -598,7 +623,8 @@ def run_gpu(args):
             summary["against"] = "the oracle's long double truth, pinned to the reference's high-precision mode"
         line["at_1e-10_relative"] = summary
     if rank == 0:
-        print(json.dumps(line))
+        print(json.dumps({"details": line}), file=sys.stderr, flush=True)
+        print(json.dumps(headline(line)), flush=True)
     integrand.close()
     if world > 1:
         dist.destroy_process_group()
