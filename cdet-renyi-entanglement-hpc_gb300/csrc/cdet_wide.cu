@@ -8,11 +8,10 @@
 // clocks. Here every step runs on the 32-bit integer pipes, to 113 bits.
 //
 // One block of four warps (of one warp up to order 7) runs a configuration,
-// both sets in turn: the
-// compact Schur recursion of the minors (the FP64 form's layout, 16-byte
-// elements: 39 KB at order 10, five blocks per SM), a level's items dealt to
-// all of its threads, then a[mask] = up * down and the connected recursion in the
-// same shared memory. In the recursion a and dp are kept unpacked (mantissa
+// both sets in turn: the compact Schur recursion of the minors (the FP64 form's
+// layout, 16-byte elements: 39 KB at order 10, five blocks per SM), a level's
+// items dealt to all of its threads, then a[mask] = up * down and the connected
+// recursion in the same shared memory. In the recursion a and dp are kept unpacked (mantissa
 // and exponent arrays), and a mask's sum is a 192-bit integer (WideSum) on a scale
 // that bounds every term of its popcount level, or, where the mask's terms may lie
 // far below that (a vertex far from all others), its own largest term: integer
@@ -42,11 +41,15 @@ namespace {
 // Orders up to 7 keep four warps waiting on one another and run a warp per
 // configuration, 20 of them per SM (a lone configuration takes as long): order
 // 7, 4,096 configurations, one spin, 911 us with four warps each, 510 with one;
-// order 2: 478 and 269. Order 1 needs neither, only a thread. Four-warp blocks leave the small configurations of a mixed batch to a second launch of
-// one-warp blocks when more than kWideTail per block remain; fewer they take
-// along while the others still run the large ones.
+// order 2: 478 and 269. Order 1 needs neither, only a thread. Four-warp blocks
+// leave the small configurations of a mixed batch to a second launch of one-warp
+// blocks when more than wide_tail per block are there; fewer they take along while
+// the others still run the large ones. Truncated-geometric orders, one launch and
+// two: up to 8, one spin, 4,096 (2.2 per block) 478 and 470 us, 6,500 650 and 531;
+// up to 9, 4,096 (3.4) 501 and 526, 6,500 688 and 590; up to 10, 4,096 (5.4) 547
+// and 742, two spins, 2,800 (6.1) 750 and 970.
 constexpr int kWideWarpMaxOrder = 7;
-constexpr int64_t kWideTail = 8;
+__host__ __device__ inline int64_t wide_tail(int max_order) { return max_order <= 8 ? 3 : max_order == 9 ? 5 : 8; }
 constexpr int32_t kNoExponent = -(1 << 24);
 
 __device__ __forceinline__ Wide from_double(double x) {
@@ -341,7 +344,7 @@ __device__ Wide wide_recursion(const RecursionArrays& r, int n, double threshold
 template <int Threads, int MaxOrder>
 __global__ void __launch_bounds__(Threads, 640 / Threads) integrand_wide(const __grid_constant__ Problem p,
                                                                            const __grid_constant__ Scratch w, int arena,
-                                                                           bool singles, uint32_t leave) {
+                                                                           bool singles, bool split) {
     extern __shared__ __align__(16) unsigned char wide_smem[];
     __shared__ DD A[kDDMaxOrder * kDDMaxOrder];
     __shared__ LevelBounds bounds;
@@ -355,6 +358,10 @@ __global__ void __launch_bounds__(Threads, 640 / Threads) integrand_wide(const _
     DD* lu_lane =
         reinterpret_cast<DD*>(w.lu_scratch + (static_cast<size_t>(blockIdx.x) * kLu + tid % kLu) * 2 * nmax * nmax);
     uint32_t* head = w.order_count + kQueueHeadIndex;
+    // every block leaves the small configurations to the second launch, or none does: the sort left the end of the
+    // order-8 slots in its bucket
+    const bool leave = split && static_cast<uint32_t>(p.batch) - __ldg(w.order_count + nmax - kWideWarpMaxOrder - 1) >
+                                    static_cast<uint32_t>(wide_tail(nmax)) * gridDim.x;
     if (singles) {  // order 1, a product of two diagonal entries: a thread per configuration
         for (int64_t c = static_cast<int64_t>(blockIdx.x) * Threads + tid; c < p.batch;
              c += static_cast<int64_t>(gridDim.x) * Threads) {
@@ -372,7 +379,7 @@ __global__ void __launch_bounds__(Threads, 640 / Threads) integrand_wide(const _
         const int n = __ldg(p.orders + c);
         __syncthreads();  // next_slot is read before the next pop
         if (n <= 1 || n > nmax) break;  // the slots' end: order 1 (above), then invalid orders (flagged by the assembly)
-        last = n <= kWideWarpMaxOrder && static_cast<uint32_t>(p.batch) - slot > leave;
+        last = leave && n <= kWideWarpMaxOrder;
         int32_t status = 0;
         DD value[2];
         for (int set = 0; set < 2; ++set) {
@@ -468,19 +475,20 @@ WideGrid wide_grid(const Problem& p, const Scratch& w, int sm_count, int max_ord
 }
 
 template <int Threads, int MaxOrder>
-cudaError_t launch_wide(const Problem& p, const Scratch& w, const WideGrid& g, bool singles, uint32_t leave,
+cudaError_t launch_wide(const Problem& p, const Scratch& w, const WideGrid& g, bool singles, bool split,
                         cudaStream_t stream) {
     const auto kernel = integrand_wide<Threads, MaxOrder>;
     const cudaError_t err =
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(g.smem));
     if (err != cudaSuccess) return err;
-    kernel<<<static_cast<unsigned>(g.blocks), Threads, g.smem, stream>>>(p, w, g.arena, singles, leave);
+    kernel<<<static_cast<unsigned>(g.blocks), Threads, g.smem, stream>>>(p, w, g.arena, singles, split);
     return cudaGetLastError();
 }
 
-// A batch so large that a warp per small configuration pays a second launch.
+// A batch so large that a warp per small configuration may pay a second launch (the kernel knows how many are
+// small; a sort in one launch leaves no bucket ends).
 bool wide_splits(const Problem& p, int64_t blocks) {
-    return p.max_order > kWideWarpMaxOrder && p.batch > kWideTail * blocks;
+    return p.max_order > kWideWarpMaxOrder && p.batch > wide_tail(p.max_order) * blocks && order_sort_launches(p.batch) > 1;
 }
 }  // namespace
 
@@ -493,13 +501,12 @@ cudaError_t launch_integrand_wide(const Problem& p, const Scratch& w, int sm_cou
     const int small = std::min(p.max_order, kWideWarpMaxOrder);
     const WideGrid warps = wide_grid(p, w, sm_count, small, kWarp);
     if (p.max_order <= kWideWarpMaxOrder)
-        return launch_wide<kWarp, kWideWarpMaxOrder>(p, w, warps, true, static_cast<uint32_t>(p.batch), stream);
+        return launch_wide<kWarp, kWideWarpMaxOrder>(p, w, warps, true, false, stream);
     const WideGrid g = wide_grid(p, w, sm_count, p.max_order, 4 * kWarp);
     const bool split = wide_splits(p, g.blocks);
-    const uint32_t leave = static_cast<uint32_t>(split ? kWideTail * g.blocks : p.batch);
-    const cudaError_t err = launch_wide<4 * kWarp, kDDMaxOrder>(p, w, g, true, leave, stream);
+    const cudaError_t err = launch_wide<4 * kWarp, kDDMaxOrder>(p, w, g, true, split, stream);
     if (err != cudaSuccess || !split) return err;
-    return launch_wide<kWarp, kWideWarpMaxOrder>(p, w, warps, false, static_cast<uint32_t>(p.batch), stream);
+    return launch_wide<kWarp, kWideWarpMaxOrder>(p, w, warps, false, false, stream);
 }
 
 }  // namespace cdet

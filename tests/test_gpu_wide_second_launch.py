@@ -3,7 +3,8 @@ small configurations run as a warp each behind the four-warp blocks. It is one
 launch more than the same mixture below the line takes, and the values and
 statuses are those of batches of one, with every matrix on the Schur recursion
 and with every matrix on the LU fallback (whose scratch a warp indexes by the
-batch's largest order, while the arena holds orders up to 7)."""
+batch's largest order, while the arena holds orders up to 7). A batch as large
+with few small configurations finds nothing left for that launch."""
 import dataclasses
 import os
 
@@ -43,10 +44,12 @@ def test_second_launch(case, tol_fpm):
     if tol_fpm:
         assert all(want_status[c] & L.CONFIG_FPM_FALLBACK for c in want if o[c] >= 2)
     few = np.concatenate([large, np.resize(small, 600)])
+    eights = np.flatnonzero(o == 8)[:4]
+    mostly_large = np.concatenate([large, np.resize(eights, 6400), np.resize(small, 60)])
     launches = {}
-    for name, part in (("few", few), ("many", idx)):
+    for name, part in (("few", few), ("many", idx), ("mostly large", mostly_large)):
         got, status = gpu.integrand_batch(np.ascontiguousarray(v[part]), o[part])
         launches[name] = gpu.last_launch_count()
         assert bits_equal(got, np.array([want[c] for c in part])), name
         assert np.array_equal(np.asarray(status), np.array([want_status[c] for c in part])), name
-    assert launches["many"] == launches["few"] + 1, launches
+    assert launches["many"] == launches["mostly large"] == launches["few"] + 1, launches
